@@ -2,9 +2,11 @@
 // to the converged, tonemapped image.  Four levels of 32-48-64-96 channels, two 3x3 convolutions
 // + ReLU per level, 2x2 average pooling down, nearest-neighbour upsampling and channel-concatenated
 // skip connections up, a 1x1 output convolution to RGB.  Weights are FP32 masters with BF16 copies;
-// every 3x3 convolution is an implicit-im2col tcgen05 BF16 GEMM with FP32 accumulation (gemm.cu:
-// the GEMM gathers its operand rows from the NHWC activations), and the backward pass and the Adam
-// update are the same GEMMs and hand-written kernels (denoise_ops.cu).
+// every convolution and both of its gradients are tcgen05 BF16 kernels with FP32 accumulation
+// (conv.cu) whose epilogues carry the elementwise work of the layer: bias, ReLU and the pooled copy
+// going forward; the loss at the head; and going back the ReLU mask, the adjoints of pooling,
+// upsampling and concatenation and the bias gradients, so each layer's output gradient is written
+// once, as the BF16 operand that its weight- and input-gradient kernels read.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -16,8 +18,8 @@
 #include <string>
 #include <vector>
 
+#include "conv.h"
 #include "denoise_ops.h"
-#include "gemm.h"
 #include "internal.h"
 #include "kernels.h"
 #include "refrakt.h"
@@ -32,17 +34,18 @@ struct Conv {
     int src_a, src_b;             // activation indices (-1 = network input / none)
     uint32_t K() const { return taps * (ca + cb); }
     uint32_t ldf() const { return (taps * cout + 7) & ~7u; }  // row stride of the flipped transpose
-    // FP32 master weights [cout x K] and bias, gradients, Adam moments
-    float *w = nullptr, *b = nullptr, *gw = nullptr, *gb = nullptr;
-    float *mw = nullptr, *vw = nullptr, *mb = nullptr, *vb = nullptr;
+    size_t offset = 0;            // of the weights [cout x K], then the biases, in the flat parameter arrays
+    float *b = nullptr, *gw = nullptr, *gb = nullptr;
     __nv_bfloat16 *w16 = nullptr, *wf16 = nullptr;
 };
 
 struct Act {  // one activation tensor (the output of conv i or of a pool)
     uint32_t c;
     int level;
+    bool skip = false;           // also read by a decoder layer
     __nv_bfloat16* x = nullptr;  // bf16 [P_level x c]
-    float* dy = nullptr;         // FP32 gradient, same shape
+    __nv_bfloat16* dz = nullptr; // gradient before the ReLU, same shape (the head: 8 channels per pixel)
+    float* dskip = nullptr;      // FP32 gradient from the decoder layer that reads it, same shape
 };
 
 constexpr uint32_t kIn = 8;  // input feature channels (4 used)
@@ -59,13 +62,9 @@ struct rf_denoiser {
     int out_conv = -1;
     uint64_t P0 = 0;                // pixels at level 0 (max)
     uint32_t H = 0, W = 0, N = 0;   // current shape
-    // scratch
-    __nv_bfloat16* colt = nullptr;  // [K x P]
-    __nv_bfloat16* dz = nullptr;    // [P x cout]
-    __nv_bfloat16* dzt = nullptr;   // [cout x P]
-    float* dx = nullptr;            // [P x Ctot]
-    float* z = nullptr;             // [P0 x 3] output head
-    __nv_bfloat16 *dpred = nullptr, *dpred_t = nullptr;
+    // parameters, gradients and Adam moments, flat over the layers (weights, then biases, of each)
+    float *w = nullptr, *g = nullptr, *m = nullptr, *v = nullptr;
+    AdamLayers adam{};
     double* loss = nullptr;
     uint32_t step = 0;
     std::vector<void*> allocs;
@@ -76,11 +75,11 @@ namespace {
 int cuda_fail(cudaError_t e, const char* what) { return fail(RF_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e)); }
 
 template <class T>
-cudaError_t dalloc(rf_denoiser* d, T** p, size_t n) {
+cudaError_t dalloc(rf_denoiser* d, T** p, size_t n, bool zero = false) {
     cudaError_t e = cudaMalloc((void**)p, n * sizeof(T) + 16);
     if (e == cudaSuccess) {
         d->allocs.push_back(*p);
-        e = cudaMemset(*p, 0, n * sizeof(T) + 16);
+        if (zero) e = cudaMemset(*p, 0, n * sizeof(T) + 16);
     }
     return e;
 }
@@ -124,6 +123,7 @@ void build_graph(rf_denoiser* D) {
     int low = skip[3];
     for (int l = 2; l >= 0; l--) {
         int a = conv(kCh[l + 1], kCh[l], kCh[l], l, low, skip[l], 1, 9, 1);
+        D->acts[skip[l]].skip = true;
         int b = conv(kCh[l], 0, kCh[l], l, a, -1, 0, 9, 1);
         low = b;
     }
@@ -141,186 +141,109 @@ void build_graph(rf_denoiser* D) {
 }
 
 // ---- forward ---------------------------------------------------------------------------------
-int forward(rf_denoiser* D, const __nv_bfloat16* input, bool need_out) {
-    const uint32_t n = D->N, h = D->H, w = D->W;
-    cudaStream_t st = D->stream;
-    for (size_t i = 0; i < D->convs.size(); i++) {
-        Conv& c = D->convs[i];
-        const int l = c.level;
-        const uint32_t hl = h >> l, wl = w >> l;
-        const uint64_t P = level_pixels(n, h, w, l);
-        // pooled input of an encoder conv
-        if (c.src_a >= (int)D->convs.size()) {
-            Act& pa = D->acts[c.src_a];
-            const Act& from = D->acts[2 * (l - 1) + 1];  // encoder conv 'b' of the level above
-            cudaError_t e = launch_avgpool(from.x, pa.c, n, h >> (l - 1), w >> (l - 1), pa.x, st);
-            if (e != cudaSuccess) return cuda_fail(e, "avgpool");
-        }
-        const __nv_bfloat16* xa = c.src_a < 0 ? input : D->acts[c.src_a].x;
-        const __nv_bfloat16* xb = c.src_b < 0 ? nullptr : D->acts[c.src_b].x;
-        GemmArgs g{};
-        if (c.taps == 9) {  // implicit convolution: the GEMM gathers its im2col rows from xa, xb
-            g.xa = xa;
-            g.xb = xb;
-            g.ca = c.ca;
-            g.cb = c.cb;
-            g.n = n;
-            g.h = hl;
-            g.w = wl;
-            g.up = c.up;
-        } else {
-            g.A = xa;
-            g.lda = c.ca;
-        }
-        g.B = c.w16;
-        g.M = (uint32_t)P;
-        g.N = c.cout;
-        g.K = c.K();
-        g.ldb = c.K();
-        if ((int)i == D->out_conv) {
-            if (!need_out) continue;
-            g.C = D->z;
-            g.ldc = 3;
-            g.mode = kGemmStoreF32;
-        } else {
-            g.C = D->acts[i].x;
-            g.ldc = c.cout;
-            g.mode = kGemmStoreBF16;
-            g.bias = c.b;
-            g.relu = c.relu;
-        }
-        cudaError_t e = c.taps == 9 ? launch_gemm_conv(g, st) : launch_gemm(g, 1, st);
-        if (e != cudaSuccess) return cuda_fail(e, "conv gemm");
-    }
-    return RF_OK;
+// the input side of layer i's convolution at the current shape
+ConvArgs layer_input(rf_denoiser* D, size_t i, const __nv_bfloat16* input) {
+    const Conv& c = D->convs[i];
+    ConvArgs a{};
+    a.xa = c.src_a < 0 ? input : D->acts[c.src_a].x;
+    a.xb = c.src_b < 0 ? nullptr : D->acts[c.src_b].x;
+    a.ca = c.ca;
+    a.cb = c.cb;
+    a.up = c.up;
+    a.n = D->N;
+    a.h = D->H >> c.level;
+    a.w = D->W >> c.level;
+    a.taps = c.taps;
+    return a;
 }
 
-uint32_t splits_for(uint64_t P) {
-    const uint64_t kb = (P + 63) / 64;
-    uint64_t s = kb / 256;  // >= 256 K blocks per CTA
-    if (s < 1) s = 1;
-    if (s > 64) s = 64;
-    return (uint32_t)s;
+// every layer; the head writes the image to `out`, or with a target the loss and its gradient
+int forward(rf_denoiser* D, const __nv_bfloat16* input, float* out, const float* target) {
+    for (size_t i = 0; i < D->convs.size(); i++) {
+        Conv& c = D->convs[i];
+        ConvArgs a = layer_input(D, i, input);
+        a.B = c.w16;
+        a.ldb = c.K();
+        a.N = c.cout;
+        a.bias = c.b;
+        ConvEpilogue epi = kConvStoreBF16;
+        if ((int)i == D->out_conv) {
+            epi = target ? kConvL1 : kConvHead;
+            a.feats = input;
+            a.target = target;
+            a.out = out;
+            a.dz = D->acts[i].dz;
+            a.loss = D->loss;
+        } else {
+            a.C = D->acts[i].x;
+            a.ldc = c.cout;
+            a.relu = c.relu;
+            // an encoder layer whose output is pooled for the level below
+            const int pooled = i < 6 && i % 2 == 1 ? D->convs[i + 1].src_a : -1;
+            if (pooled >= 0) a.pool = D->acts[pooled].x;
+        }
+        const cudaError_t e = launch_conv(a, epi, D->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "convolution");
+    }
+    return RF_OK;
 }
 
 // ---- backward + Adam -------------------------------------------------------------------------
-int backward(rf_denoiser* D, const __nv_bfloat16* input, const float* target, float lr) {
-    const uint32_t n = D->N, h = D->H, w = D->W;
-    cudaStream_t st = D->stream;
-    cudaError_t e = cudaSuccess;
-    // zero gradients
-    for (auto& a : D->acts)
-        if (e == cudaSuccess) e = cudaMemsetAsync(a.dy, 0, level_pixels(n, h, w, a.level) * a.c * sizeof(float), st);
-    for (auto& c : D->convs) {
-        if (e == cudaSuccess) e = cudaMemsetAsync(c.gw, 0, (size_t)c.cout * c.K() * sizeof(float), st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(c.gb, 0, c.cout * sizeof(float), st);
-    }
-    if (e == cudaSuccess) e = cudaMemsetAsync(D->loss, 0, sizeof(double), st);
-    if (e != cudaSuccess) return cuda_fail(e, "gradient clear");
-    const uint64_t P0 = level_pixels(n, h, w, 0);
+int update(rf_denoiser* D, float lr, uint32_t step) {
+    const cudaError_t e = launch_adam(D->w, D->g, D->m, D->v, D->adam, (uint32_t)D->convs.size(), lr, 0.9f, 0.999f, 1e-8f,
+                                      step, D->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "adam");
+    return RF_OK;
+}
 
+int train(rf_denoiser* D, const __nv_bfloat16* input, const float* target, float lr) {
+    cudaError_t e = cudaMemsetAsync(D->g, 0, rf_denoiser_num_params(D) * sizeof(float), D->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(D->loss, 0, sizeof(double), D->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "gradient clear");
+    if (int rc = forward(D, input, nullptr, target)) return rc;
+    std::vector<WgradTask> tasks;
     for (int i = (int)D->convs.size() - 1; i >= 0; i--) {
         Conv& c = D->convs[i];
-        const int l = c.level;
-        const uint32_t hl = h >> l, wl = w >> l;
-        const uint64_t P = level_pixels(n, h, w, l);
-        const uint32_t ldp = (uint32_t)((P + 7) & ~7ull);  // row stride of the transposed operands
-        const __nv_bfloat16* xa = c.src_a < 0 ? input : D->acts[c.src_a].x;
-        const __nv_bfloat16* xb = c.src_b < 0 ? nullptr : D->acts[c.src_b].x;
-        const __nv_bfloat16* dzp;
-        const __nv_bfloat16* dztp;
-        uint32_t ldz;
-        if (i == D->out_conv) {
-            e = launch_l1_head(D->z, c.b, input, target, P0, D->dpred, D->dpred_t, ldp, c.gb, D->loss, st);
-            if (e != cudaSuccess) return cuda_fail(e, "l1 head");
-            dzp = D->dpred;
-            dztp = D->dpred_t;
-            ldz = 8;
-        } else {
-            e = launch_relu_back(D->acts[i].dy, D->acts[i].x, c.cout, P, c.relu, D->dz, D->dzt, ldp, c.gb, st);
-            if (e != cudaSuccess) return cuda_fail(e, "relu backward");
-            dzp = D->dz;
-            dztp = D->dzt;
-            ldz = c.cout;
-        }
-        // weight gradient: gw[cout x K] += dz^T[cout x P] * col[P x K]
-        GemmArgs gw{};
-        gw.A = dztp;
-        gw.lda = ldp;
-        e = launch_im2col_t(xa, c.ca, c.up, xb, c.cb, c.taps, n, hl, wl, D->colt, ldp, st);
-        if (e != cudaSuccess) return cuda_fail(e, "im2col_t");
-        gw.B = D->colt;
-        gw.ldb = ldp;
-        gw.M = c.cout;
-        gw.N = c.K();
-        gw.K = (uint32_t)P;
-        gw.C = c.gw;
-        gw.ldc = c.K();
-        gw.mode = kGemmAtomicF32;
-        e = launch_gemm(gw, splits_for(P), st);
-        if (e != cudaSuccess) return cuda_fail(e, "weight-gradient gemm");
+        const uint32_t ldz = i == D->out_conv ? 8 : c.cout;  // the head's gradient is padded to 8 channels
+        tasks.push_back(WgradTask{layer_input(D, (size_t)i, input), c.cout, ldz, c.gw});
+        tasks.back().conv.dz = D->acts[i].dz;
         if (c.src_a < 0) continue;  // first layer: no input gradient
-        // input gradient: dX[P x Ctot] = conv(dz, flipped transposed weights)
-        GemmArgs gx{};
-        if (c.taps == 9) {  // implicit convolution of dz
-            gx.xa = dzp;
-            gx.ca = c.cout;
-            gx.n = n;
-            gx.h = hl;
-            gx.w = wl;
-            gx.K = 9 * c.cout;
-        } else {
-            gx.A = dzp;
-            gx.lda = ldz;
-            gx.K = ldz;  // dpred is zero beyond its 3 channels; wf16 rows are zero there too
-        }
+        // input gradient: dX = conv(dz, flipped transposed weights)
+        ConvArgs gx{};
+        gx.xa = D->acts[i].dz;
+        gx.ca = ldz;
+        gx.n = D->N;
+        gx.h = D->H >> c.level;
+        gx.w = D->W >> c.level;
+        gx.taps = c.taps;
         gx.B = c.wf16;
         gx.ldb = c.ldf();
-        gx.M = (uint32_t)P;
         gx.N = c.ca + c.cb;
-        const bool concat = c.cb > 0;
-        const bool pooled = !concat && c.src_a >= (int)D->convs.size();
-        if (!concat && !pooled) {  // straight into the source activation's gradient
-            gx.C = D->acts[c.src_a].dy;
-            gx.ldc = c.ca;
-            gx.mode = kGemmAtomicF32;
-        } else {
-            gx.C = D->dx;
-            gx.ldc = c.ca + c.cb;
-            gx.mode = kGemmStoreF32;
+        ConvEpilogue epi = kConvMask;
+        int into = c.src_a;  // the layer whose output gradient this completes
+        if (c.cb > 0) {
+            epi = kConvConcat;
+            gx.nlow = c.ca;
+            gx.dskip = D->acts[c.src_b].dskip;
+        } else if (c.src_a >= (int)D->convs.size()) {
+            epi = kConvPool;
+            into = 2 * (c.level - 1) + 1;  // the last encoder layer of the level above
+            gx.dskip = D->acts[into].dskip;
         }
-        e = c.taps == 9 ? launch_gemm_conv(gx, st) : launch_gemm(gx, 1, st);
-        if (e != cudaSuccess) return cuda_fail(e, "input-gradient gemm");
-        if (concat) {
-            e = launch_split_concat_grad(D->dx, c.ca, c.cb, n, hl, wl, D->acts[c.src_a].dy, D->acts[c.src_b].dy, st);
-            if (e != cudaSuccess) return cuda_fail(e, "concat gradient");
-        } else if (pooled) {
-            const int from = 2 * (l - 1) + 1;  // encoder conv 'b' of the level above
-            e = launch_avgpool_back(D->dx, c.ca, n, h >> (l - 1), w >> (l - 1), D->acts[from].dy, st);
-            if (e != cudaSuccess) return cuda_fail(e, "pool gradient");
-        }
+        gx.y = D->acts[into].x;
+        gx.dz = D->acts[into].dz;
+        gx.gb = D->convs[into].gb;
+        e = launch_conv(gx, epi, D->stream);
+        if (e != cudaSuccess) return cuda_fail(e, "input gradient");
     }
-    // Adam
-    D->step++;
-    for (auto& c : D->convs) {
-        e = launch_adam(c.w, c.gw, c.mw, c.vw, c.cout * c.K(), lr, 0.9f, 0.999f, 1e-8f, D->step, c.cout, c.K(), c.taps,
-                        c.w16, c.wf16, c.ldf(), st);
-        if (e == cudaSuccess)
-            e = launch_adam(c.b, c.gb, c.mb, c.vb, c.cout, lr, 0.9f, 0.999f, 1e-8f, D->step, c.cout, 1, 1, nullptr,
-                            nullptr, 0, st);
-        if (e != cudaSuccess) return cuda_fail(e, "adam");
-    }
-    return RF_OK;
+    const Conv& head = D->convs[D->out_conv];
+    e = launch_conv_wgrad(tasks.data(), (uint32_t)tasks.size(), D->acts[D->out_conv].dz, level_pixels(D->N, D->H, D->W, 0),
+                          head.gb, D->stream);
+    if (e != cudaSuccess) return cuda_fail(e, "weight gradients");
+    return update(D, lr, ++D->step);
 }
 
-int refresh_bf16(rf_denoiser* D) {
-    for (auto& c : D->convs) {
-        cudaError_t e = launch_adam(c.w, c.gw, c.mw, c.vw, c.cout * c.K(), 0.0f, 0.9f, 0.999f, 1e-8f, 1, c.cout, c.K(),
-                                    c.taps, c.w16, c.wf16, c.ldf(), D->stream);
-        if (e != cudaSuccess) return cuda_fail(e, "weight refresh");
-    }
-    return RF_OK;
-}
+int refresh_bf16(rf_denoiser* D) { return update(D, 0.0f, 1); }
 
 int check_shape(rf_denoiser* D, uint32_t n, uint32_t h, uint32_t w) {
     if (n == 0 || h == 0 || w == 0 || h % 8 || w % 8)
@@ -349,6 +272,9 @@ int rf_denoiser_create(const rf_denoiser_desc* desc, rf_denoiser** out) {
     if (e != cudaSuccess) return bail(cuda_fail(e, "stream"));
     build_graph(D);
     // parameters, He-normal initialisation from a seeded generator
+    const size_t np = rf_denoiser_num_params(D);
+    std::vector<float> hp;
+    hp.reserve(np);
     std::mt19937_64 gen(desc->seed);
     for (auto& c : D->convs) {
         const size_t nw = (size_t)c.cout * c.K();
@@ -360,39 +286,36 @@ int rf_denoiser_create(const rf_denoiser_desc* desc, rf_denoiser** out) {
                 for (uint32_t t = 0; t < 9; t++) hw[(size_t)co * c.K() + t * kIn + kIn - 1] = 0.0f;
         if (c.taps == 1)  // the output layer starts at zero: the first prediction is the plain image
             std::fill(hw.begin(), hw.end(), 0.0f);
-        if (e == cudaSuccess) e = dalloc(D, &c.w, nw);
-        if (e == cudaSuccess) e = dalloc(D, &c.gw, nw);
-        if (e == cudaSuccess) e = dalloc(D, &c.mw, nw);
-        if (e == cudaSuccess) e = dalloc(D, &c.vw, nw);
-        if (e == cudaSuccess) e = dalloc(D, &c.b, c.cout);
-        if (e == cudaSuccess) e = dalloc(D, &c.gb, c.cout);
-        if (e == cudaSuccess) e = dalloc(D, &c.mb, c.cout);
-        if (e == cudaSuccess) e = dalloc(D, &c.vb, c.cout);
+        c.offset = hp.size();
+        hp.insert(hp.end(), hw.begin(), hw.end());
+        hp.insert(hp.end(), c.cout, 0.0f);  // biases
         if (e == cudaSuccess) e = dalloc(D, &c.w16, nw);
-        if (e == cudaSuccess) e = dalloc(D, &c.wf16, (size_t)(c.ca + c.cb) * c.ldf());
-        if (e == cudaSuccess) e = cudaMemcpy(c.w, hw.data(), nw * sizeof(float), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) return bail(cuda_fail(e, "rf_denoiser_create: parameters"));
+        if (e == cudaSuccess) e = dalloc(D, &c.wf16, (size_t)(c.ca + c.cb) * c.ldf(), true);  // padding columns stay zero
     }
-    // activations and scratch at the maximum size
-    size_t colt = 0, dx = 0, dz = 0;
-    for (auto& a : D->acts) {
+    if (e == cudaSuccess) e = dalloc(D, &D->w, np);
+    if (e == cudaSuccess) e = dalloc(D, &D->g, np, true);
+    if (e == cudaSuccess) e = dalloc(D, &D->m, np, true);
+    if (e == cudaSuccess) e = dalloc(D, &D->v, np, true);
+    // (the copy runs behind the clears on the default stream and returns when it is done)
+    if (e == cudaSuccess) e = cudaMemcpy(D->w, hp.data(), np * sizeof(float), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return bail(cuda_fail(e, "rf_denoiser_create: parameters"));
+    for (size_t i = 0; i < D->convs.size(); i++) {
+        Conv& c = D->convs[i];
+        const size_t nw = (size_t)c.cout * c.K();
+        c.b = D->w + c.offset + nw;
+        c.gw = D->g + c.offset;
+        c.gb = c.gw + nw;
+        D->adam.layer[i] = AdamLayer{(uint32_t)c.offset, c.cout, c.K(), c.taps, c.ldf(), c.w16, c.wf16};
+    }
+    // activations and their gradients at the maximum size
+    for (size_t i = 0; i < D->acts.size(); i++) {
+        Act& a = D->acts[i];
         const uint64_t P = D->P0 >> (2 * a.level);
-        if (e == cudaSuccess) e = dalloc(D, &a.x, P * a.c);
-        if (e == cudaSuccess) e = dalloc(D, &a.dy, P * a.c);
+        const bool head = (int)i == D->out_conv;
+        if (e == cudaSuccess && !head) e = dalloc(D, &a.x, P * a.c);
+        if (e == cudaSuccess && i < D->convs.size()) e = dalloc(D, &a.dz, P * (head ? 8 : a.c));
+        if (e == cudaSuccess && a.skip) e = dalloc(D, &a.dskip, P * a.c);
     }
-    for (auto& c : D->convs) {
-        const uint64_t P = ((D->P0 >> (2 * c.level)) + 7) & ~7ull;
-        colt = std::max<size_t>(colt, P * c.K());
-        dx = std::max<size_t>(dx, P * (c.ca + c.cb));
-        dz = std::max<size_t>(dz, P * std::max<uint32_t>(c.cout, 8));
-    }
-    if (e == cudaSuccess) e = dalloc(D, &D->colt, colt);
-    if (e == cudaSuccess) e = dalloc(D, &D->dz, dz);
-    if (e == cudaSuccess) e = dalloc(D, &D->dzt, dz);
-    if (e == cudaSuccess) e = dalloc(D, &D->dx, dx);
-    if (e == cudaSuccess) e = dalloc(D, &D->z, D->P0 * 3);
-    if (e == cudaSuccess) e = dalloc(D, &D->dpred, D->P0 * 8);
-    if (e == cudaSuccess) e = dalloc(D, &D->dpred_t, ((D->P0 + 7) & ~7ull) * 8);
     if (e == cudaSuccess) e = dalloc(D, &D->loss, 1);
     if (e != cudaSuccess) return bail(cuda_fail(e, "rf_denoiser_create: activations"));
     if (int rc = refresh_bf16(D)) return bail(rc);
@@ -459,14 +382,7 @@ int rf_denoiser_get_params(rf_denoiser* D, float* host, size_t cap) {
     if (!D || !host || cap < rf_denoiser_num_params(D)) return fail(RF_ERR_INVALID_ARG, "rf_denoiser_get_params: bad arguments");
     cudaSetDevice(D->device);
     cudaError_t e = cudaStreamSynchronize(D->stream);
-    size_t o = 0;
-    for (auto& c : D->convs) {
-        const size_t nw = (size_t)c.cout * c.K();
-        if (e == cudaSuccess) e = cudaMemcpy(host + o, c.w, nw * sizeof(float), cudaMemcpyDeviceToHost);
-        o += nw;
-        if (e == cudaSuccess) e = cudaMemcpy(host + o, c.b, c.cout * sizeof(float), cudaMemcpyDeviceToHost);
-        o += c.cout;
-    }
+    if (e == cudaSuccess) e = cudaMemcpy(host, D->w, rf_denoiser_num_params(D) * sizeof(float), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(e, "rf_denoiser_get_params");
     return RF_OK;
 }
@@ -475,14 +391,7 @@ int rf_denoiser_set_params(rf_denoiser* D, const float* host, size_t count) {
     if (!D || !host || count != rf_denoiser_num_params(D)) return fail(RF_ERR_INVALID_ARG, "rf_denoiser_set_params: bad arguments");
     cudaSetDevice(D->device);
     cudaError_t e = cudaStreamSynchronize(D->stream);
-    size_t o = 0;
-    for (auto& c : D->convs) {
-        const size_t nw = (size_t)c.cout * c.K();
-        if (e == cudaSuccess) e = cudaMemcpy(c.w, host + o, nw * sizeof(float), cudaMemcpyHostToDevice);
-        o += nw;
-        if (e == cudaSuccess) e = cudaMemcpy(c.b, host + o, c.cout * sizeof(float), cudaMemcpyHostToDevice);
-        o += c.cout;
-    }
+    if (e == cudaSuccess) e = cudaMemcpy(D->w, host, count * sizeof(float), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "rf_denoiser_set_params");
     return refresh_bf16(D);
 }
@@ -509,11 +418,7 @@ int rf_denoiser_infer(rf_denoiser* D, const void* feats, uint32_t n, uint32_t h,
     if (!D || !feats || !out_rgb) return fail(RF_ERR_INVALID_ARG, "rf_denoiser_infer: null argument");
     if (int rc = check_shape(D, n, h, w)) return rc;
     cudaSetDevice(D->device);
-    if (int rc = forward(D, static_cast<const __nv_bfloat16*>(feats), true)) return rc;
-    const Conv& oc = D->convs[D->out_conv];
-    cudaError_t e = launch_head(D->z, oc.b, static_cast<const __nv_bfloat16*>(feats), (uint64_t)n * h * w, out_rgb,
-                                D->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "rf_denoiser_infer");
+    if (int rc = forward(D, static_cast<const __nv_bfloat16*>(feats), out_rgb, nullptr)) return rc;
     return RF_OK;
 }
 
@@ -522,9 +427,10 @@ int rf_denoiser_train_step(rf_denoiser* D, const void* feats, const float* targe
     if (!D || !feats || !target_rgb) return fail(RF_ERR_INVALID_ARG, "rf_denoiser_train_step: null argument");
     if (int rc = check_shape(D, n, h, w)) return rc;
     cudaSetDevice(D->device);
-    const auto* in = static_cast<const __nv_bfloat16*>(feats);
-    if (int rc = forward(D, in, true)) return rc;
-    if (int rc = backward(D, in, target_rgb, lr)) return rc;
+    // the weight-gradient products run over whole blocks of 8 pixels at every level
+    if ((uint64_t)n * (h / 8) * (w / 8) % 8)
+        return fail(RF_ERR_CUDA, "rf_denoiser_train_step: batch x height / 8 x width / 8 must be a multiple of 8");
+    if (int rc = train(D, static_cast<const __nv_bfloat16*>(feats), target_rgb, lr)) return rc;
     if (loss) {
         double l = 0;
         cudaError_t e = cudaMemcpyAsync(&l, D->loss, sizeof(double), cudaMemcpyDeviceToHost, D->stream);
@@ -539,14 +445,7 @@ int rf_denoiser_gradients(rf_denoiser* D, float* host, size_t cap) {
     if (!D || !host || cap < rf_denoiser_num_params(D)) return fail(RF_ERR_INVALID_ARG, "rf_denoiser_gradients: bad arguments");
     cudaSetDevice(D->device);
     cudaError_t e = cudaStreamSynchronize(D->stream);
-    size_t o = 0;
-    for (auto& c : D->convs) {
-        const size_t nw = (size_t)c.cout * c.K();
-        if (e == cudaSuccess) e = cudaMemcpy(host + o, c.gw, nw * sizeof(float), cudaMemcpyDeviceToHost);
-        o += nw;
-        if (e == cudaSuccess) e = cudaMemcpy(host + o, c.gb, c.cout * sizeof(float), cudaMemcpyDeviceToHost);
-        o += c.cout;
-    }
+    if (e == cudaSuccess) e = cudaMemcpy(host, D->g, rf_denoiser_num_params(D) * sizeof(float), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(e, "rf_denoiser_gradients");
     return RF_OK;
 }

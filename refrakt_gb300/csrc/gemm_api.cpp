@@ -4,6 +4,7 @@
 
 #include <string>
 
+#include "conv.h"
 #include "gemm.h"
 #include "internal.h"
 #include "refrakt.h"
@@ -13,10 +14,10 @@ using namespace rfk;
 namespace {
 
 // waits for the launch, then reads the kernels' bounded-wait error word
-int finish(const char* fn, cudaError_t e, cudaStream_t st) {
+int finish(const char* fn, cudaError_t e, cudaStream_t st, cudaError_t (*error)(int*) = gemm_error) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     int werr = 0;
-    if (e == cudaSuccess) e = gemm_error(&werr);
+    if (e == cudaSuccess) e = error(&werr);
     if (e != cudaSuccess) return fail(RF_ERR_CUDA, std::string(fn) + ": " + cudaGetErrorString(e));
     if (werr) return fail(RF_ERR_CUDA, std::string(fn) + ": an mbarrier wait ran out (stage " + std::to_string(werr - 1) + ")");
     return RF_OK;
@@ -63,6 +64,30 @@ extern "C" int rf_conv3x3_bf16(const void* xa, uint32_t ca, int up, const void* 
     if ((((uintptr_t)xa) | ((uintptr_t)xb) | ((uintptr_t)B)) & 15)
         return fail(RF_ERR_INVALID_ARG, "rf_conv3x3_bf16: operands must be 16-byte aligned");
     if (mode < RF_GEMM_STORE_F32 || mode > RF_GEMM_ATOMIC_F32) return fail(RF_ERR_INVALID_ARG, "rf_conv3x3_bf16: bad mode");
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // channels in whole K steps and a tile's operands within shared memory: the staged-tile kernel
+    // (conv.cu); other channel counts gather im2col rows (gemm.cu)
+    if (conv_supported(ca + cb, N, 9)) {
+        ConvArgs a{};
+        a.xa = static_cast<const __nv_bfloat16*>(xa);
+        a.xb = static_cast<const __nv_bfloat16*>(xb);
+        a.ca = ca;
+        a.cb = cb;
+        a.up = up;
+        a.n = n;
+        a.h = h;
+        a.w = w;
+        a.taps = 9;
+        a.B = static_cast<const __nv_bfloat16*>(B);
+        a.N = N;
+        a.ldb = ldb;
+        a.C = C;
+        a.ldc = ldc;
+        a.bias = bias;
+        a.relu = relu;
+        const ConvEpilogue epi = mode == RF_GEMM_STORE_F32 ? kConvStoreF32 : mode == RF_GEMM_ATOMIC_F32 ? kConvAtomicF32 : kConvStoreBF16;
+        return finish("rf_conv3x3_bf16", launch_conv(a, epi, st), st, conv_error);
+    }
     GemmArgs g{};
     g.xa = static_cast<const __nv_bfloat16*>(xa);
     g.xb = static_cast<const __nv_bfloat16*>(xb);
@@ -82,6 +107,5 @@ extern "C" int rf_conv3x3_bf16(const void* xa, uint32_t ca, int up, const void* 
     g.mode = mode;
     g.bias = bias;
     g.relu = relu;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
     return finish("rf_conv3x3_bf16", launch_gemm_conv(g, st), st);
 }

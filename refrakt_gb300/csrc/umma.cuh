@@ -49,9 +49,22 @@ __host__ __device__ constexpr uint64_t smem_desc_sw128(uint32_t saddr) {
 __host__ __device__ constexpr uint32_t idesc_bf16_f32(uint32_t m, uint32_t n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);
 }
+// bits 15 and 16: A, B stored MN-major.  Without swizzle a core matrix is then 8 K rows of 16 bytes (8
+// consecutive M or N elements) in 128 contiguous bytes; the descriptor's leading-dimension offset is
+// the distance of core matrices along K, the stride offset that along M or N.
+constexpr uint32_t kTransposeA = 1u << 15, kTransposeB = 1u << 16;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
+}
+
+// One lane of a converged warp (elect.sync).  Code under it is known to run in one thread, so the
+// descriptors of a sequence of MMAs stay in uniform registers; under a lane == 0 test every MMA
+// first moves them there (about 60 cycles each, conv.cu).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
 }
 
 // ---- mbarrier ------------------------------------------------------------------------------
@@ -110,6 +123,16 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
         "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
         " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// the same with each descriptor as two words: within one operand only the low word (start address)
+// changes from step to step
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint32_t alo, uint32_t ahi, uint32_t blo, uint32_t bhi,
+                                         uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n .reg .b64 a, b;\n mov.b64 a, {%1, %2};\n mov.b64 b, {%3, %4};\n setp.ne.b32 p, %6, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %5, p;\n}\n" ::"r"(d_tmem),
+        "r"(alo), "r"(ahi), "r"(blo), "r"(bhi), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 // arrives once on `bar` when every MMA this thread issued before has completed
