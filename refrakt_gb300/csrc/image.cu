@@ -4,16 +4,17 @@
 // The reference does density estimation as a GL point-sprite raster pass with additive
 // blending (src/main.cpp:490-515, shaders/density_vert.glsl:26-63, density_frag.glsl:9-18):
 // every non-empty bin becomes a sprite of radius r = max(min, min(R, int(R / a^curve))) whose
-// fragments add color * (1 - d^2) * (2/pi) / r^2.  Here each CTA owns an output tile and gathers
-// it from the tile and its halo staged in shared memory, walking either the whole box of the
-// tile's largest radius or only its large discs, whichever is less work for that tile (radii
-// above 12 gather from global memory).  The disc is the symmetric restatement
+// fragments add color * (1 - d^2) * (2/pi) / r^2.  Here each warp owns an output tile and gathers it
+// from the tile and its halo staged in shared memory, sweeping the sources that reach it (radii above
+// kDeMaxSweepR gather from global memory).  The disc is the symmetric restatement
 // 4 (dx^2 + dy^2) <= (2r + 1)^2 with
 // d^2 = (dx^2 + dy^2) / (r + 0.5)^2 (the GL sprite's sub-pixel centring depends on point
-// rasterisation rules).  Radii come from thresholds on a, computed on the host in FP64, and
-// the kernel weights from a per-radius table, so every radius and weight is exactly defined.
+// rasterisation rules).  Radii come from thresholds on a, computed on the host in FP64, and the
+// kernel weights are those of a per-radius FP64 table rounded to FP32, so every radius and weight is
+// exactly defined.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <vector>
 
@@ -21,7 +22,8 @@
 
 namespace rfk {
 
-constexpr int kDeMaxSmemR = 12;  // radius handled through shared-memory tiles
+constexpr int kDeMaxSmemR = 12;   // radius of the fused path: a tile and its whole halo in shared memory
+constexpr int kDeMaxSweepR = 56;  // radius up to which de_weight_params reproduces the weight table
 
 struct DeTables {
     float thr[101];      // thr[k-1]: bin radius >= k  <=>  a <= thr (curve > 0) or a >= thr (curve < 0)
@@ -149,7 +151,10 @@ __device__ __forceinline__ float4 tonemap_finish(float r, float g, float b, floa
     const float rgb[3] = {r, g, b};
     float res[3];
     for (int q = 0; q < 3; q++) {
-        const float v = powf(rgb[q], ig) * (1.0f - vibrancy) + gf * rgb[q] * vibrancy;
+        // at vibrancy 1 the first term is zero for every finite colour (a negative one's NaN clamps to 0, as
+        // its second term does): three of a pixel's four powers are not needed
+        const bool plain = vibrancy == 1.0f && fabsf(rgb[q]) < INFINITY;
+        const float v = (plain ? 0.0f : powf(rgb[q], ig) * (1.0f - vibrancy)) + gf * rgb[q] * vibrancy;
         res[q] = fminf(fmaxf(v, 0.0f), 1.0f);
     }
     return make_float4(res[0], res[1], res[2], 1.0f);
@@ -189,7 +194,43 @@ __device__ __forceinline__ uchar4 to_rgba8(float4 o) {
                        (unsigned char)lrintf(o.z * 255.0f), 255);
 }
 
-// the tonemap a DE tile kernel applies to its own output (TM = true)
+// ---- pass 2: the sweep --------------------------------------------------------------------------
+//
+// A warp owns 32 x ROWS outputs (8, 4 or 2 rows), one column of ROWS outputs per lane, and takes the
+// staged source rows one after another, each in the cheaper of two ways (de_row):
+//   by offset  every lane takes the source dx columns from its own, for dx up to the row's largest
+//              reach; a step without a disc that reaches is dropped (a warp-wide maximum of the radii);
+//   by source  the row's non-empty sources, fewer than those offsets, one after another for all lanes.
+// Either way a source's colour and weight parameters are read once for up to ROWS outputs, only the output
+// rows within the largest disc at hand are touched, and every output adds its sources in ascending
+// column order.
+//
+// The order of every output's sum is fixed: row-major over the discs that cover it, or, in 32 x 8 tiles
+// with few discs of radius >= 2 (9 + their number < (2 rmax + 1)^2), first those of radius 0 and 1 and then
+// the larger ones, row-major each.
+//
+// Weights.  w(d2) = (1 - d2 / (r + 1/2)^2) (2/pi) / r^2 as the FP64 table rounds it, without the table:
+// with both coefficients split into a multiple of g = 2^-24 times the leading one's binade and a
+// remainder, (hi - d2 * step) is exact in FP32, the remainders' part is below 2^-10 of it, and one
+// addition rounds their sum: equal to the table for every radius up to 56 and every offset
+// (de_weight_params, checked on the host).  Outside the disc the same expression is negative, so its
+// maximum with zero is the coverage test.  Two outputs at a time in packed FP32 arithmetic.
+//
+// Bound: instruction issue (62 % of the slots at 24 warps per SM; about 70 instructions per source and
+// 8 outputs).  Density estimation of 3840 x 2160 bins at 1000 points per bin: 990 us as one output per
+// thread over the box of the tile's largest radius, 642 here; 960 x 540 at radius 20 1,090 us as a gather
+// from global memory, 344 here.
+constexpr int kTileW = 32, kTileH = 8;     // the tile whose discs set the order of its sums
+constexpr int kDeThreads = 256;
+constexpr int kCtaW = 2 * kTileW;          // a CTA: 8 warps, two side by side, each 32 x ROWS outputs
+constexpr int kBandRows = 24;              // staged source rows at a time where the halo is not staged whole
+
+// per radius: hi, step (exact part), and the remainders' coefficients; all zero for an empty bin
+struct DeParams {
+    float4 r[kDeMaxSweepR + 1];
+};
+
+// the tonemap a DE kernel applies to its own output (TM = true)
 struct TmArgs {
     uint32_t ss;
     float gamma, brightness, vibrancy, k2;
@@ -198,160 +239,244 @@ struct TmArgs {
     uchar4* out8;         // may be null
 };
 
-// pass 2: a CTA owns a 32 x 8 output tile.  It stages the colours and radii of the tile and
-// its R halo in shared memory and forms each output bin as a gather in one of two ways, chosen
-// per tile by their work:
-//   box  — sum the bins within the tile's largest radius rmax whose disc covers the output:
-//          up to (2 rmax + 1)^2 taps per output, rows whose largest disc cannot reach the output
-//          skipped and each row's span cut to its largest radius;
-//   list — the discs of radius 0 and 1 from the 3 x 3 neighbourhood, plus a compact list of the
-//          tile's larger discs (those reaching the tile), which every thread walks in the same
-//          order (shared-memory broadcasts): 9 + list-length taps per output.
-// Dense regions (radius 0 and 1 at converged sample counts, a few sparse bins) take the list;
-// sparse fringes full of large discs take the box.  The sum is deterministic either way.
-constexpr int kDsX = 32, kDsY = 8, kDsThreads = 256;
-
-// With TM the tile's output stays in shared memory and the CTA tonemaps its (32/ss) x (8/ss)
-// output pixels from it (ss dividing 8): the estimator's output never goes through DRAM.
-// Shared memory of a tile CTA: NS staged colours (float4), NS list entries, NS packed source
-// records, the weight table of radii up to R, per-warp counts and the rmax slot, per staged row
-// its largest radius; with TM the tile's NO outputs.
-template <int R>
-__host__ __device__ constexpr int de_weight_count() { return (R + 1) * (R + 2) * (2 * R + 3) / 6; }  // sum (r+1)^2
-
-template <int R, bool TM = false>
-__host__ __device__ constexpr size_t de_tile_smem() {
-    return (((size_t)(kDsX + 2 * R) * (kDsY + 2 * R) * (16 + 4 + 4) + 4 * (size_t)de_weight_count<R>() + 16 * 4 +
-             4 * (kDsY + 2 * R) + 15) & ~(size_t)15) +
-           (TM ? (size_t)kDsX * kDsY * 16 : 0);
+typedef unsigned long long f32x2;  // two packed FP32 values
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
 }
 
-// A staged source bin as one word: the disc's squared-distance limit r^2 + r (bits 0-8: a tap at
-// squared distance d2 is inside the disc exactly when d2 <= limit, the symmetric restatement of
-// 4 d2 <= (2r + 1)^2), the offset of radius r's weights in the table (bits 9-18) and the table's
-// row length r + 1 (bits 19-23).  An empty bin is a radius-0 disc of colour zero: it adds zero.
-__device__ __forceinline__ uint32_t de_pack(int r) {
-    return (uint32_t)(r * r + r) | ((uint32_t)(r * (r + 1) * (2 * r + 1) / 6) << 9) | ((uint32_t)(r + 1) << 19);
-}
-
-// one tap: source record p at offset (ax, ay) (squared distance d2) into the accumulator
-__device__ __forceinline__ void de_tap(float4& a4, uint32_t p, int ax, int ay, int d2, const float* s_wt,
-                                       const float4& v) {
-    const bool in = d2 <= (int)(p & 0x1ffu);
-    const float wt = in ? s_wt[((p >> 9) & 0x3ffu) + ay * (int)(p >> 19) + ax] : 0.0f;
-    a4.x = fmaf(v.x, wt, a4.x);
-    a4.y = fmaf(v.y, wt, a4.y);
-    a4.z = fmaf(v.z, wt, a4.z);
-    a4.w = fmaf(v.w, wt, a4.w);
-}
-
-template <int R, bool TM = false>
-__global__ void __launch_bounds__(kDsThreads) de_tile_kernel(
-    const float4* __restrict__ in, const uint8_t* __restrict__ rad, uint32_t w, uint32_t h,
-    const float* __restrict__ weights, const DeTables T, float4* __restrict__ out, const TmArgs tm) {
-    constexpr int SW = kDsX + 2 * R, SH = kDsY + 2 * R, NS = SW * SH, NO = kDsX * kDsY, NW = de_weight_count<R>();
-    extern __shared__ __align__(16) unsigned char smem[];
-    float4* s_c = reinterpret_cast<float4*>(smem);                  // NS colours (zero where empty)
-    int* s_list = reinterpret_cast<int*>(s_c + NS);                 // indices of discs of radius >= 2
-    uint32_t* s_pk = reinterpret_cast<uint32_t*>(s_list + NS);      // NS packed source records
-    float* s_wt = reinterpret_cast<float*>(s_pk + NS);              // weights of radii 0..R
-    int* s_stat = reinterpret_cast<int*>(s_wt + NW);                // [0] rmax, [1..8] per-warp counts
-    int* s_rowmax = s_stat + 16;                                     // SH: largest radius per staged row
-    float4* s_out = reinterpret_cast<float4*>(smem + ((de_tile_smem<R, false>() + 15) & ~(size_t)15));  // TM: NO outputs
-    const int tx0 = blockIdx.x * kDsX, ty0 = blockIdx.y * kDsY;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_stat[0] = 0;
-    for (int i = threadIdx.x; i < SH; i += kDsThreads) s_rowmax[i] = -1;
-    {  // the weight table holds radii up to this launch's largest (<= R); the rest stays zero
-        const int rl = T.R > T.min_r ? T.R : T.min_r;
-        const int nw = (rl + 1) * (rl + 2) * (2 * rl + 3) / 6;
-        for (int i = threadIdx.x; i < NW; i += kDsThreads) s_wt[i] = i < nw ? weights[i] : 0.0f;
+// the lane's outputs: channel c of outputs 2q and 2q + 1 in v[q][c]
+template <int ROWS>
+struct DeAcc {
+    f32x2 v[ROWS / 2][4];
+};
+// the rows of a warp seen from one source row: their squared distances, negated, and each pair's nearer one
+template <int ROWS>
+struct DeRows {
+    f32x2 ndy2[ROWS / 2];
+    int near2[ROWS / 2];
+};
+// one source (or each lane's own) at -dx^2 into the outputs: colour, parameters p[0], p[1], and the
+// largest squared row distance that matters
+template <int ROWS>
+__device__ __forceinline__ void de_add(DeAcc<ROWS>& acc, const float4& c, const float4* p, float ndx2, const DeRows<ROWS>& rows,
+                                       int left) {
+    const float4 pa = p[0], pb = p[1];
+    const f32x2 nd = pack2(ndx2, ndx2), step = pack2(pa.z, pa.w), lstep = pack2(pb.z, pb.w);
+    const f32x2 t0 = fma2(nd, step, pack2(pa.x, pa.y)), l0 = fma2(nd, lstep, pack2(pb.x, pb.y));
+    const f32x2 cr = pack2(c.x, c.x), cg = pack2(c.y, c.y), cb = pack2(c.z, c.z), ca = pack2(c.w, c.w);
+#pragma unroll
+    for (int q = 0; q < ROWS / 2; q++) {
+        if (rows.near2[q] > left) continue;
+        const float2 w = unpack2(add2(fma2(rows.ndy2[q], step, t0), fma2(rows.ndy2[q], lstep, l0)));
+        const f32x2 wt = pack2(fmaxf(w.x, 0.0f), fmaxf(w.y, 0.0f));
+        acc.v[q][0] = fma2(cr, wt, acc.v[q][0]);
+        acc.v[q][1] = fma2(cg, wt, acc.v[q][1]);
+        acc.v[q][2] = fma2(cb, wt, acc.v[q][2]);
+        acc.v[q][3] = fma2(ca, wt, acc.v[q][3]);
     }
-    __syncthreads();
-    int rmax = 0, nl = 0;
-    // stage the tile + halo; list the large discs that reach the tile in source order (a
-    // ballot-and-prefix compaction, so the list and the sums are the same on every run)
-    for (int i0 = 0; i0 < NS; i0 += kDsThreads) {
-        const int i = i0 + (int)threadIdx.x;
-        bool big = false;
-        if (i < NS) {
-            const int gx = tx0 - R + i % SW, gy = ty0 - R + i / SW;
+}
+
+// One staged source row into the warp's outputs: s_c, s_r (radius + 1, 0 = empty) point at the row's first
+// column of the warp's window (R columns left of its outputs), dy = the row's offset from the warp's
+// first output row.  WHICH: kAll radii, kSmall (0 and 1) or kLarge (the others).  s_p: the parameters,
+// each value twice.
+enum DeWhich { kAll, kSmall, kLarge };
+template <DeWhich WHICH>
+__device__ __forceinline__ int de_pick(int r) {
+    if (WHICH == kSmall) return r > 1 ? -1 : r;
+    if (WHICH == kLarge) return r < 2 ? -1 : r;
+    return r;
+}
+template <int ROWS, int CHUNKS, DeWhich WHICH>
+__device__ __forceinline__ void de_row(DeAcc<ROWS>& acc, const float4* s_c, const uint8_t* s_r, const float4* s_p, int R, int dy) {
+    const int lane = threadIdx.x & 31;
+    const int md = dy < 0 ? -dy : (dy > ROWS - 1 ? dy - (ROWS - 1) : 0);  // to the warp's nearest row
+    // the discs of the row that reach the warp's rows, 32 columns at a time
+    unsigned b[CHUNKS];
+    int r[CHUNKS], rr = -1, n = 0;
+#pragma unroll
+    for (int k = 0; k < CHUNKS; k++) {
+        const int x = 32 * k + lane;
+        r[k] = x < kTileW + 2 * R ? de_pick<WHICH>((int)s_r[x] - 1) : -1;
+        if (r[k] < md) r[k] = -1;
+        b[k] = __ballot_sync(0xffffffffu, r[k] >= 0);
+        n += __popc(b[k]);
+        rr = max(rr, r[k]);
+    }
+    if (n == 0) return;
+    rr = __reduce_max_sync(0xffffffffu, rr);
+    const int span = min(rr, (int)sqrtf((float)(rr * rr + rr - md * md)));
+    DeRows<ROWS> rows;
+#pragma unroll
+    for (int q = 0; q < ROWS / 2; q++) {
+        const int e0 = dy - 2 * q, e1 = e0 - 1;
+        rows.ndy2[q] = pack2(-(float)(e0 * e0), -(float)(e1 * e1));
+        rows.near2[q] = min(e0 * e0, e1 * e1);
+    }
+    if (n <= 2 * span + 1) {
+#pragma unroll
+        for (int k = 0; k < CHUNKS; k++)
+            while (b[k]) {
+                const int col = __ffs(b[k]) - 1, x = 32 * k + col;
+                b[k] &= b[k] - 1;
+                const int rs = __shfl_sync(0xffffffffu, r[k], col);
+                const float dx = (float)(lane + R - x);
+                de_add(acc, s_c[x], s_p + 2 * (rs + 1), -dx * dx, rows, rs * rs + rs);
+            }
+        return;
+    }
+    const int reach = md * md;
+    for (int dx = -span; dx <= span; dx++) {
+        const int q = de_pick<WHICH>((int)s_r[R + lane + dx] - 1);
+        const int m = __reduce_max_sync(0xffffffffu, q);
+        const int left = m * m + m - dx * dx;
+        if (m < 0 || left < reach) continue;
+        de_add(acc, s_c[R + lane + dx], s_p + 2 * (q + 1), -(float)(dx * dx), rows, left);
+    }
+}
+
+// staged rows [row0, row0 + rows) of the CTA's window, whose origin is (gx0, gy0), to the staging's start
+__device__ __forceinline__ void de_stage(const float4* __restrict__ in, const uint8_t* __restrict__ rad, int w, int h, int gx0,
+                                         int gy0, int pitch, int row0, int rows, float4* s_c, uint8_t* s_r) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+    for (int i = warp; i < rows; i += warps) {
+        const int gy = gy0 + row0 + i;
+        const bool row = gy >= 0 && gy < h;
+        for (int x = lane; x < pitch; x += 32) {
+            const int gx = gx0 + x;
             int r = 255;
             float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (gx >= 0 && gy >= 0 && gx < (int)w && gy < (int)h) {
+            if (row && gx >= 0 && gx < w) {
                 const size_t gi = (size_t)gy * w + gx;
                 r = rad[gi];
                 if (r != 255) v = in[gi];
             }
-            s_pk[i] = de_pack(r == 255 ? 0 : r);
-            s_c[i] = v;
-            if (r != 255) atomicMax(&s_rowmax[i / SW], r);
-            if (r != 255 && gx - r <= tx0 + kDsX - 1 && gx + r >= tx0 && gy - r <= ty0 + kDsY - 1 && gy + r >= ty0) {
+            s_c[i * pitch + x] = v;
+            s_r[i * pitch + x] = (uint8_t)(r + 1);  // 255 -> 0
+        }
+    }
+}
+
+__host__ __device__ constexpr size_t de_smem_bytes(int rows, int R, bool whole) {
+    const size_t n = (size_t)(whole ? 4 * rows + 2 * R : kBandRows) * (kCtaW + 2 * R);
+    return (size_t)(R + 2) * 32 + n * 16 + ((n + 15) & ~(size_t)15);
+}
+
+// WHOLE: the halo staged whole (R <= kDeMaxSmemR), each tile's order chosen as above; else the source
+// rows pass through shared memory in bands, every tile row-major.  TM: the outputs stay in shared
+// memory (over the staging) and are tonemapped there.
+template <bool WHOLE, bool TM, int ROWS>
+__global__ void __launch_bounds__(kDeThreads, 3) de_sweep_kernel(const float4* __restrict__ in, const uint8_t* __restrict__ rad,
+                                                                 uint32_t w, uint32_t h, int R, const __grid_constant__ DeParams P,
+                                                                 float4* __restrict__ out, const TmArgs tm) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int cta_rows = 4 * ROWS;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int pitch = kCtaW + 2 * R, all = cta_rows + 2 * R;
+    const int held = WHOLE ? all : kBandRows;
+    float4* s_p = reinterpret_cast<float4*>(smem);                  // (R + 2) x {hi, hi, step, step}, {lo, lo, lstep, lstep}
+    float4* s_c = s_p + 2 * (R + 2);
+    uint8_t* s_r = reinterpret_cast<uint8_t*>(s_c + (size_t)held * pitch);
+    const int tx0 = blockIdx.x * kCtaW, ty0 = blockIdx.y * cta_rows;
+    for (int r = threadIdx.x; r <= R + 1; r += kDeThreads) {  // entry 0: the empty bin
+        const float4 p = r ? P.r[r - 1] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        s_p[2 * r] = make_float4(p.x, p.x, p.y, p.y);
+        s_p[2 * r + 1] = make_float4(p.z, p.z, p.w, p.w);
+    }
+    const int x0 = (warp & 1) * kTileW, y0 = (warp >> 1) * ROWS;  // the warp's outputs in the CTA's
+    DeAcc<ROWS> acc;
+#pragma unroll
+    for (int q = 0; q < ROWS / 2; q++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) acc.v[q][c] = 0;
+    if constexpr (WHOLE) {
+        de_stage(in, rad, (int)w, (int)h, tx0 - R, ty0 - R, pitch, 0, all, s_c, s_r);
+        __syncthreads();
+        // of the discs that reach the warp's 32 x 8 tile: the largest radius, and the number of those of
+        // radius >= 2
+        int rmax = 0, big = 0;
+        const uint8_t* tr = s_r + (y0 & ~(kTileH - 1)) * pitch + x0;
+        for (int i = 0; i < kTileH + 2 * R; i++) {
+            const int dy = i - R, md = dy < 0 ? -dy : (dy > kTileH - 1 ? dy - (kTileH - 1) : 0);
+            for (int x = lane; x < kTileW + 2 * R; x += 32) {
+                const int r = (int)tr[i * pitch + x] - 1, dx = x - R;
+                if (r < 0 || r < md || dx + r < 0 || dx - r > kTileW - 1) continue;
                 rmax = max(rmax, r);
-                big = r >= 2;
+                big += r >= 2;
             }
         }
-        const unsigned m = __ballot_sync(0xffffffffu, big);
-        if (lane == 0) s_stat[1 + warp] = __popc(m);
-        __syncthreads();
-        int off = nl, tot = 0;
-        for (int q = 0; q < kDsThreads / 32; q++) {
-            const int c = s_stat[1 + q];
-            if (q < warp) off += c;
-            tot += c;
-        }
-        if (big) s_list[off + __popc(m & ((1u << lane) - 1u))] = i;
-        nl += tot;
-        __syncthreads();
-    }
-    atomicMax(&s_stat[0], rmax);
-    __syncthreads();
-    const int rm = s_stat[0];
-    const bool use_list = 9 + nl < (2 * rm + 1) * (2 * rm + 1);
-    for (int o = threadIdx.x; o < NO; o += kDsThreads) {
-        const int ox = o % kDsX, oy = o / kDsX;
-        float4 a4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (use_list) {
-            // discs of radius 0 and 1 from the 3 x 3 neighbourhood, then the listed larger discs
-            for (int dy = -1; dy <= 1; dy++)
-                for (int dx = -1; dx <= 1; dx++) {
-                    const int si = (oy + R + dy) * SW + ox + R + dx;
-                    const uint32_t p = s_pk[si];
-                    if ((p & 0x1ffu) > 2u) continue;  // radius >= 2: in the list
-                    de_tap(a4, p, dx * dx, dy * dy, dx * dx + dy * dy, s_wt, s_c[si]);
-                }
-            for (int k = 0; k < nl; k++) {
-                const int si = s_list[k];
-                const int ax = abs(ox + R - si % SW), ay = abs(oy + R - si / SW);
-                if (ax > R || ay > R) continue;
-                de_tap(a4, s_pk[si], ax, ay, ax * ax + ay * ay, s_wt, s_c[si]);
-            }
+        rmax = __reduce_max_sync(0xffffffffu, rmax);
+        big = __reduce_add_sync(0xffffffffu, big);
+        const float4* wc = s_c + y0 * pitch + x0;  // the warp's window
+        const uint8_t* wr = s_r + y0 * pitch + x0;
+        const bool small_first = 9 + big < (2 * rmax + 1) * (2 * rmax + 1);
+        if (small_first) {
+            for (int i = max(0, R - 1); i < min(ROWS + R + 1, ROWS + 2 * R); i++)
+                de_row<ROWS, 2, kSmall>(acc, wc + i * pitch, wr + i * pitch, s_p, R, i - R);
+            if (big)
+                for (int i = 0; i < ROWS + 2 * R; i++) de_row<ROWS, 2, kLarge>(acc, wc + i * pitch, wr + i * pitch, s_p, R, i - R);
         } else {
-            for (int dy = -rm; dy <= rm; dy++) {
-                const int ay = dy < 0 ? -dy : dy;
-                const int rr = min(rm, s_rowmax[oy + R + dy]);  // no disc of this row reaches |dy| rows
-                if (rr < ay) continue;
-                const int row = (oy + R + dy) * SW + ox + R;
-                for (int dx = -rr; dx <= rr; dx++) {
-                    const int ax = dx < 0 ? -dx : dx;
-                    de_tap(a4, s_pk[row + dx], ax, ay, ax * ax + ay * ay, s_wt, s_c[row + dx]);
-                }
+            for (int i = 0; i < ROWS + 2 * R; i++) de_row<ROWS, 2, kAll>(acc, wc + i * pitch, wr + i * pitch, s_p, R, i - R);
+        }
+        __syncthreads();
+    } else {
+        for (int b = 0; b < all; b += kBandRows) {
+            const int rows = min(kBandRows, all - b);
+            __syncthreads();
+            de_stage(in, rad, (int)w, (int)h, tx0 - R, ty0 - R, pitch, b, rows, s_c, s_r);
+            __syncthreads();
+            // this band's rows within reach of the warp's
+            const int first = max(0, y0 - b), last = min(rows, y0 + ROWS + 2 * R - b);
+            for (int i = first; i < last; i++) {
+                const float4* rc = s_c + i * pitch + x0;
+                const uint8_t* rr = s_r + i * pitch + x0;
+                const int dy = b + i - y0 - R;
+                if (R <= 16) de_row<ROWS, 2, kAll>(acc, rc, rr, s_p, R, dy);
+                else if (R <= 32) de_row<ROWS, 3, kAll>(acc, rc, rr, s_p, R, dy);
+                else de_row<ROWS, 5, kAll>(acc, rc, rr, s_p, R, dy);
             }
         }
-        const int gx = tx0 + ox, gy = ty0 + oy;
-        if (out && gx < (int)w && gy < (int)h) out[(size_t)gy * w + gx] = a4;
-        if (TM) s_out[o] = a4;
     }
-    if (TM) {
+    float4* s_out = s_c;  // TM: the CTA's outputs, over the staging (every warp is past it)
+#pragma unroll
+    for (int q = 0; q < ROWS / 2; q++) {
+        const float2 r = unpack2(acc.v[q][0]), g = unpack2(acc.v[q][1]), b = unpack2(acc.v[q][2]), a = unpack2(acc.v[q][3]);
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            const float4 o = k ? make_float4(r.y, g.y, b.y, a.y) : make_float4(r.x, g.x, b.x, a.x);
+            const int oy = y0 + 2 * q + k, ox = x0 + lane;
+            const int gx = tx0 + ox, gy = ty0 + oy;
+            if (TM) s_out[oy * kCtaW + ox] = o;
+            else if (gx < (int)w && gy < (int)h) out[(size_t)gy * w + gx] = o;
+        }
+    }
+    if constexpr (TM) {
         __syncthreads();
-        const uint32_t ss = tm.ss, pw = kDsX / ss, ph = kDsY / ss, ow = w / ss, oh = h / ss;
+        const uint32_t ss = tm.ss, pw = kCtaW / ss, ph = cta_rows / ss, ow = w / ss, oh = h / ss;
         const float k = tonemap_scale(tm.k2, tm.stats, w, h);
-        for (uint32_t p = threadIdx.x; p < pw * ph; p += kDsThreads) {
+        for (uint32_t p = threadIdx.x; p < pw * ph; p += kDeThreads) {
             const uint32_t px = p % pw, py = p / pw;
             const uint32_t gx = tx0 / ss + px, gy = ty0 / ss + py;
             if (gx >= ow || gy >= oh) continue;
-            const float4 o = tonemap_block(s_out + (size_t)py * ss * kDsX + px * ss, kDsX, ss, k, tm.gamma,
-                                           tm.brightness, tm.vibrancy);
+            const float4 o = tonemap_block(s_out + (size_t)py * ss * kCtaW + px * ss, kCtaW, ss, k, tm.gamma, tm.brightness,
+                                           tm.vibrancy);
             const size_t oi = (size_t)gy * ow + gx;
             if (tm.out_f32) tm.out_f32[oi] = o;
             if (tm.out8) tm.out8[oi] = to_rgba8(o);
@@ -359,13 +484,17 @@ __global__ void __launch_bounds__(kDsThreads) de_tile_kernel(
     }
 }
 
-template <int R>
-static cudaError_t set_de_tile_smem() {
-    cudaError_t e = cudaFuncSetAttribute(de_tile_kernel<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)de_tile_smem<R, false>());
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(de_tile_kernel<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)de_tile_smem<R, true>());
+constexpr size_t kDeMaxSmem = 112 * 1024;  // two CTAs per SM
+
+template <int ROWS>
+static cudaError_t set_de_smem() {
+    const void* k[3] = {(const void*)de_sweep_kernel<true, false, ROWS>, (const void*)de_sweep_kernel<true, true, ROWS>,
+                        (const void*)de_sweep_kernel<false, false, ROWS>};
+    for (const void* f : k) {
+        const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDeMaxSmem);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 // the DE kernels' shared-memory limits, set once per device before any launch (also before a
@@ -376,25 +505,52 @@ cudaError_t density_prepare() {
     if (e != cudaSuccess) return e;
     static bool done[64] = {};
     if (dev >= 0 && dev < 64 && done[dev]) return cudaSuccess;
-    e = set_de_tile_smem<3>();
-    if (e == cudaSuccess) e = set_de_tile_smem<6>();
-    if (e == cudaSuccess) e = set_de_tile_smem<9>();
-    if (e == cudaSuccess) e = set_de_tile_smem<kDeMaxSmemR>();
+    e = set_de_smem<8>();
+    if (e == cudaSuccess) e = set_de_smem<4>();
+    if (e == cudaSuccess) e = set_de_smem<2>();
     if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev] = true;
     return e;
 }
 
-template <int R>
-static cudaError_t launch_de_tile(const float4* in, const uint8_t* rad, uint32_t w, uint32_t h, const float* dw,
-                                  const DeTables& T, float4* out, cudaStream_t st, const TmArgs* tm = nullptr) {
+// The weight parameters of every radius up to R (the sweep's comment).  The leading coefficient's
+// binade sets the grid of the exact part; the remainders are rounded to FP32.
+static void de_weight_params(int R, DeParams& P) {
+    P.r[0] = make_float4(1.0f, 4.0f, 0.0f, 0.0f);  // radius 0: weight 1 at the centre
+    for (int r = 1; r <= R; r++) {
+        const double lead = 0.63661977236 / (double)(r * r), slope = lead / ((r + 0.5) * (r + 0.5));
+        int e = 0;
+        std::frexp(lead, &e);
+        const double g = std::ldexp(1.0, e - 24), hi = std::rint(lead / g) * g, step = std::rint(slope / g) * g;
+        P.r[r] = make_float4((float)hi, (float)step, (float)(lead - hi), (float)(slope - step));
+    }
+}
+
+template <int ROWS>
+static cudaError_t launch_de_rows(int R, const DeParams& P, const float4* in, const uint8_t* rad, uint32_t w, uint32_t h,
+                                  float4* out, cudaStream_t st, const TmArgs* tm) {
+    const bool whole = R <= kDeMaxSmemR;
+    const dim3 grid((w + kCtaW - 1) / kCtaW, (h + 4 * ROWS - 1) / (4 * ROWS));
+    const size_t smem = de_smem_bytes(ROWS, R, whole);  // (a fused CTA's outputs fit in its staging)
+    if (tm) de_sweep_kernel<true, true, ROWS><<<grid, kDeThreads, smem, st>>>(in, rad, w, h, R, P, out, *tm);
+    else if (whole) de_sweep_kernel<true, false, ROWS><<<grid, kDeThreads, smem, st>>>(in, rad, w, h, R, P, out, TmArgs{});
+    else de_sweep_kernel<false, false, ROWS><<<grid, kDeThreads, smem, st>>>(in, rad, w, h, R, P, out, TmArgs{});
+    return cudaGetLastError();
+}
+
+// R: the launch's largest radius.  More rows per warp read a source once for more outputs, fewer leave
+// more warps to hide latency.  Measured, radius 9 (density estimation alone, 8 / 4 / 2 rows): 3840 x 2160
+// 642 / 737 / 872 us, 1920 x 1080 242 / 236 / 274, 960 x 540 116 / 96 / 107, 512 x 512 95 / 73 / 82, 640 x 360
+// 93 / 70 / 64, 320 x 180 88 / 58 / 47: 8 rows from 12 CTAs for each of the 152 SMs, 4 from about 1.6.
+static cudaError_t launch_de_sweep(int R, const float4* in, const uint8_t* rad, uint32_t w, uint32_t h, float4* out,
+                                   cudaStream_t st, const TmArgs* tm = nullptr) {
     cudaError_t e = density_prepare();
     if (e != cudaSuccess) return e;
-    const dim3 grid((w + kDsX - 1) / kDsX, (h + kDsY - 1) / kDsY);
-    if (tm)
-        de_tile_kernel<R, true><<<grid, kDsThreads, de_tile_smem<R, true>(), st>>>(in, rad, w, h, dw, T, out, *tm);
-    else
-        de_tile_kernel<R, false><<<grid, kDsThreads, de_tile_smem<R, false>(), st>>>(in, rad, w, h, dw, T, out, TmArgs{});
-    return cudaGetLastError();
+    DeParams P;
+    de_weight_params(R, P);
+    const auto ctas = [&](uint32_t rows) { return (uint64_t)((w + kCtaW - 1) / kCtaW) * ((h + 4 * rows - 1) / (4 * rows)); };
+    if (ctas(8) >= 12 * 152) return launch_de_rows<8>(R, P, in, rad, w, h, out, st, tm);
+    if (ctas(4) >= 240) return launch_de_rows<4>(R, P, in, rad, w, h, out, st, tm);
+    return launch_de_rows<2>(R, P, in, rad, w, h, out, st, tm);
 }
 
 // large radii: the gather straight from global memory
@@ -611,7 +767,8 @@ cudaError_t launch_tonemap_filter(const float4* in, uint32_t w, uint32_t h, uint
 }
 
 // ---------------------------------------------------------------------------------------------
-static void de_tables(int R, int min_r, float curve, DeTables& T, std::vector<float>& wts) {
+// the radius thresholds alone
+static void de_thresholds(int R, int min_r, float curve, DeTables& T) {
     T = DeTables{};
     T.R = R;
     T.min_r = min_r;
@@ -624,6 +781,10 @@ static void de_tables(int R, int min_r, float curve, DeTables& T, std::vector<fl
         if (T.mode == 1 && (double)f < t) f = std::nextafter(f, INFINITY);   // a >= f  <=>  a >= t
         T.thr[k - 1] = f;
     }
+}
+
+static void de_tables(int R, int min_r, float curve, DeTables& T, std::vector<float>& wts) {
+    de_thresholds(R, min_r, curve, T);
     wts.clear();
     const int rmax = R > min_r ? R : min_r;
     for (int r = 0; r <= rmax && r <= 100; r++) {
@@ -655,18 +816,21 @@ cudaError_t launch_density(const float4* in, uint32_t w, uint32_t h, int R, int 
                            cudaStream_t st) {
     DeTables T;
     std::vector<float> wts;
-    de_tables(R, min_r, curve, T, wts);
-    const size_t n = (size_t)w * h;
+    const bool sweep = std::max(R, min_r) <= kDeMaxSweepR;  // else the gather, which reads the weight table
+    if (sweep) de_thresholds(R, min_r, curve, T);
+    else de_tables(R, min_r, curve, T, wts);
     uint8_t* rad = nullptr;
     float* dw = nullptr;
-    cudaError_t e = cudaMallocAsync(&rad, n, st);
+    cudaError_t e = cudaMallocAsync(&rad, (size_t)w * h, st);
     if (e != cudaSuccess) return e;
-    e = cudaMallocAsync(&dw, wts.size() * sizeof(float), st);
-    if (e != cudaSuccess) { cudaFreeAsync(rad, st); return e; }
-    cudaMemcpyAsync(dw, wts.data(), wts.size() * sizeof(float), cudaMemcpyHostToDevice, st);
+    if (!sweep) {
+        e = cudaMallocAsync(&dw, wts.size() * sizeof(float), st);
+        if (e != cudaSuccess) { cudaFreeAsync(rad, st); return e; }
+        cudaMemcpyAsync(dw, wts.data(), wts.size() * sizeof(float), cudaMemcpyHostToDevice, st);
+    }
     e = launch_density_passes(in, w, h, T, out, rad, dw, st);
     cudaFreeAsync(rad, st);
-    cudaFreeAsync(dw, st);
+    if (dw) cudaFreeAsync(dw, st);
     return e;
 }
 
@@ -677,29 +841,19 @@ size_t density_weight_count(int R, int min_r) {
     return n;
 }
 
-// the tile kernel for the largest radius (rmax <= kDeMaxSmemR)
-static cudaError_t launch_tile_for(int rmax, const float4* in, const uint8_t* rad, uint32_t w, uint32_t h,
-                                   const float* dw, const DeTables& T, float4* out, cudaStream_t st,
-                                   const TmArgs* tm) {
-    if (rmax <= 3) return launch_de_tile<3>(in, rad, w, h, dw, T, out, st, tm);
-    if (rmax <= 6) return launch_de_tile<6>(in, rad, w, h, dw, T, out, st, tm);
-    if (rmax <= 9) return launch_de_tile<9>(in, rad, w, h, dw, T, out, st, tm);
-    return launch_de_tile<kDeMaxSmemR>(in, rad, w, h, dw, T, out, st, tm);
-}
-
 static cudaError_t launch_density_passes(const float4* in, uint32_t w, uint32_t h, const DeTables& T, float4* out,
                                          uint8_t* rad, const float* dw, cudaStream_t st) {
     const size_t n = (size_t)w * h;
     de_radius_kernel<<<1024, 256, 0, st>>>(in, n, T, rad);
     const int rmax = T.R > T.min_r ? T.R : T.min_r;
-    if (rmax <= kDeMaxSmemR) return launch_tile_for(rmax, in, rad, w, h, dw, T, out, st, nullptr);
+    if (rmax <= kDeMaxSweepR) return launch_de_sweep(rmax, in, rad, w, h, out, st);
     de_gather_global_kernel<<<dim3((w + 127) / 128, h), 128, 0, st>>>(in, rad, w, h, dw, T, out);
     return cudaGetLastError();
 }
 
 bool density_tonemap_fused(int R, int min_r, uint32_t ss) {
     const int rmax = R > min_r ? R : min_r;
-    return rmax <= kDeMaxSmemR && ss >= 1 && kDsX % ss == 0 && kDsY % ss == 0;
+    return rmax <= kDeMaxSmemR && ss >= 1 && kTileW % ss == 0 && kTileH % ss == 0;
 }
 
 // The image tail of a frame (main.cpp:490-535: the density-estimation raster pass, then the
@@ -736,7 +890,7 @@ cudaError_t launch_density_tonemap(const float4* in, uint32_t w, uint32_t h, int
         de_radius_kernel<<<1024, 256, 0, st>>>(in, (size_t)w * h, T, rad);
     }
     const TmArgs tm{ss, gamma, brightness, vibrancy, k2, need_sum ? stats : nullptr, out_f32, out8};
-    return launch_tile_for(R > min_r ? R : min_r, in, rad, w, h, dw, T, nullptr, st, &tm);
+    return launch_de_sweep(R > min_r ? R : min_r, in, rad, w, h, nullptr, st, &tm);
 }
 
 void density_weights(int R, int min_r, std::vector<float>& wts) {
