@@ -267,8 +267,10 @@ RF_API int  rf_set_bad_value_reset(rf_sim* s, int on);
    tile or walker reset) the first two drawing launches of >= 32 passes and equal length run one
    form each, timed with CUDA events, and the faster runs from then on (decided without a host
    wait, once the second launch has finished; not during stream capture, where the pipelined form
-   runs).  All forms give
-   identical results.  A pipelined wait that runs out (bounded) makes the next synchronising call
+   runs).  Where cta_threads is 0 and the mixing domains are fewer than the SMs, AUTO spreads each
+   domain over a cluster of 2 to 8 CTAs with a cluster barrier per pass (reported as barrier), in
+   place of the barrier form where a CTA keeps two slots per thread and without timing where it
+   keeps one.  All forms give identical results.  A pipelined wait that runs out (bounded) makes the next synchronising call
    (rf_draw_to_bins with `drawn`, rf_sim_counters, rf_render) return RF_ERR_TIMEOUT. */
 enum rf_exchange { RF_EXCHANGE_BARRIER = 0, RF_EXCHANGE_PIPELINED = 1, RF_EXCHANGE_AUTO = 2 };
 RF_API int  rf_set_exchange(rf_sim* s, int mode);

@@ -78,6 +78,16 @@ bool use_pipe(const rf_sim* s, uint32_t tile_bins) {
     return s->table_phases >= 3 && chaos_smem(s->slots, s->prog_words, s->L, tile_bins, 1) <= kMaxCtaSmem;
 }
 
+// RF_EXCHANGE_AUTO with the CTA shape left to the library: domains fewer than the SMs spread over
+// clusters (chaos_cluster).  With a slot per thread that is the faster form (1.1 to 2.1 times on five
+// genomes); with two (a 4096-slot domain on two CTAs) it stands in for the barrier form in the timing
+// against the pipelined exchange (1.25 times its speed on the 1080p genome, 1.0 on a 5-xform one).
+// `barrier`: the timing's choice.
+int cluster_for_launch(const rf_sim* s, bool barrier) {
+    if (!s->spec || s->exchange != RF_EXCHANGE_AUTO || s->d.cta_threads != 0 || s->cluster == 1) return 1;
+    return s->slots / s->cluster <= 1024 || barrier ? s->cluster : 1;
+}
+
 void reset_exchange_tuning(rf_sim* s);
 
 bool capturing(cudaStream_t st) {
@@ -177,7 +187,8 @@ int exchange_for_launch(rf_sim* s, bool draw, uint32_t steps, bool may_measure, 
             float tb = 0.0f, tp = 0.0f;
             if (cudaEventElapsedTime(&tb, s->tune_ev[0], s->tune_ev[1]) == cudaSuccess &&
                 cudaEventElapsedTime(&tp, s->tune_ev[2], s->tune_ev[3]) == cudaSuccess)
-                s->tune_pipe = tp <= tb ? 1 : 0;
+                // (a cluster that stands in for the barrier form takes twice the SMs: only for a clear gain)
+                s->tune_pipe = tp <= (cluster_for_launch(s, true) > 1 ? 1.05f * tb : tb) ? 1 : 0;
             s->tune_step = 3;
         } else if (q == cudaErrorNotReady) {
             if (cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError();  // clear only this status
@@ -260,23 +271,28 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
         a.trace = s->trace;
         a.trace_passes = s->trace_passes;
         a.n_groups = (uint32_t)(s->N / kGroup);
-        const uint32_t grid = (uint32_t)(s->N / s->slots);
         const uint32_t tile_bins = a.splat == 3 && a.draw ? a.tile_w * a.tile_h : 0u;
         int measure = -1;
         // (RF_SPLAT_AUTO's tile is timed first, in the pipelined form; the exchange after it)
         const bool tile_busy = tile_warmup || tile_timed >= 0 || (s->splat == RF_SPLAT_AUTO && s->auto_tile_state >= 2);
-        const int want = s->spec ? exchange_for_launch(s, a.draw, steps, !tile_busy, &measure) : 0;
+        const bool timed = s->spec && cluster_for_launch(s, false) == 1;  // else the cluster form, untimed
+        const int want = timed ? exchange_for_launch(s, a.draw, steps, !tile_busy, &measure) : 0;
         const int pipe = want && s->spec && use_pipe(s, tile_bins) ? 1 : 0;
-        if (s->spec && (s->spec_splat != a.splat || s->spec_reset != a.reset || s->spec_pipe != pipe)) {
+        // one CTA per mixing domain, or a cluster of `cl`
+        const int cl = cluster_for_launch(s, !want);
+        const uint32_t local = s->slots / cl, threads = cl > 1 ? std::min(1024u, local) : s->threads;
+        const uint32_t grid = (uint32_t)(s->N / s->slots) * cl;
+        if (s->spec && (s->spec_splat != a.splat || s->spec_reset != a.reset || s->spec_pipe != pipe || s->spec_cluster != cl)) {
             // the splat strategy, the reset or the exchange changed since warmup: the kernel compiled for them
             const void* k = nullptr;
-            if (int rc = spec_kernel(s->spec_prog, (int)s->threads, (int)s->slots, s->device, &k, SpecKind::Chaos,
-                                     a.splat, a.reset, pipe))
+            if (int rc = spec_kernel(s->spec_prog, (int)threads, (int)local, s->device, &k, SpecKind::Chaos, a.splat,
+                                     a.reset, pipe, cl))
                 return rc;
             s->spec = k;
             s->spec_splat = a.splat;
             s->spec_reset = a.reset;
             s->spec_pipe = pipe;
+            s->spec_cluster = cl;
         }
         if (chaos_smem(s->slots, a.prog_words, a.steps, tile_bins) > kMaxCtaSmem)
             return fail(RF_ERR_CAPACITY, "splat tile of " + std::to_string(tile_bins) +
@@ -284,8 +300,8 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
                                          " walker slots");
         if (measure >= 0 && cudaEventRecord(s->tune_ev[2 * measure], s->stream) != cudaSuccess) measure = -1;
         if (tile_timed >= 0 && cudaEventRecord(s->tile_ev[2 * tile_timed], s->stream) != cudaSuccess) tile_timed = -1;
-        cudaError_t e = s->spec ? launch_spec(s->spec, (int)s->threads, (int)s->slots, a, grid,
-                                              chaos_smem(s->slots, a.prog_words, a.steps, tile_bins, pipe), s->stream)
+        cudaError_t e = s->spec ? launch_spec(s->spec, (int)threads, (int)local, a, grid,
+                                              chaos_smem(local, a.prog_words, a.steps, tile_bins, pipe), s->stream)
                                 : launch_chaos((int)s->threads, (int)s->slots, a, grid, s->stream);
         if (e != cudaSuccess) return cuda_fail(e, "chaos kernel launch");
         if (measure >= 0 && cudaEventRecord(s->tune_ev[2 * measure + 1], s->stream) == cudaSuccess)
@@ -725,14 +741,18 @@ int rf_warmup(rf_sim* s, rf_flame* f, uint32_t num_passes, float tss_width) {
     }
     if (s->d.specialize >= 0) {
         const void* k = nullptr;
-        const int pipe = s->exchange != RF_EXCHANGE_BARRIER && use_pipe(s, 0) ? 1 : 0;
-        const int rc = spec_kernel(prog, (int)s->threads, (int)s->slots, s->device, &k, SpecKind::Chaos,
-                                   splat_code(s->splat), s->reset, pipe);
+        s->cluster = s->d.cta_threads == 0 ? chaos_cluster((int)s->slots, s->N / s->slots, s->prog_words, s->L) : 1;
+        const int cl = s->exchange == RF_EXCHANGE_AUTO && s->slots / s->cluster <= 1024 ? s->cluster : 1;
+        const int local = (int)s->slots / cl, threads = cl > 1 ? local : (int)s->threads;
+        const int pipe = cl == 1 && s->exchange != RF_EXCHANGE_BARRIER && use_pipe(s, 0) ? 1 : 0;
+        const int rc = spec_kernel(prog, threads, local, s->device, &k, SpecKind::Chaos, splat_code(s->splat), s->reset, pipe,
+                                   cl);
         if (rc == RF_OK) {
             s->spec = k;
             s->spec_splat = splat_code(s->splat);
             s->spec_reset = s->reset;
             s->spec_pipe = pipe;
+            s->spec_cluster = cl;
             s->spec_prog = prog;
         } else if (s->d.specialize > 0) {
             return rc;  // required
@@ -839,6 +859,7 @@ int rf_sim_exchange(const rf_sim* s) {
                                : s->splat == RF_SPLAT_AUTO && s->auto_tile_state == 1 ? s->auto_tile[2] * s->auto_tile[3]
                                                                                       : 0u;
     if (!s->spec || !use_pipe(s, tile_bins)) return 0;
+    if (cluster_for_launch(s, false) > 1) return 0;  // a barrier per pass, of a cluster
     if (s->exchange != RF_EXCHANGE_AUTO) return s->exchange == RF_EXCHANGE_PIPELINED ? 1 : 0;
     return s->tune_pipe;
 }

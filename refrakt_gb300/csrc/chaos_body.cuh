@@ -91,6 +91,22 @@ __device__ __forceinline__ bool xbar_wait(uint64_t* b, uint32_t parity) {
     return false;
 }
 
+// The cluster exchange: a mixing domain spread over the CTAs of a thread-block cluster, each with its
+// share of the slots in its own shared memory.  A pass's walkers are read from the CTA that holds them
+// (distributed shared memory); one cluster barrier per pass replaces the CTA's.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ float4 cluster_load(const float4* local, uint32_t rank) {
+    uint32_t a = (uint32_t)__cvta_generic_to_shared(local);
+    float4 v;
+    asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(a) : "r"(rank));
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(a)
+                 : "memory");
+    return v;
+}
+
 // One CTA of THREADS threads owns SLOTS = THREADS * SPT walker slots — the walker shuffle's mixing
 // domain — for the launch's passes.  Every slot's walker and JSF32 state live in shared memory;
 // each thread serves SPT slots per pass (phase_slot(k, tid), in SPT different 256-slot groups, so
@@ -109,10 +125,20 @@ __device__ __forceinline__ bool xbar_wait(uint64_t* b, uint32_t parity) {
 // phase: the slowest warps' last phase overlaps the others' next pass, with the walkers still
 // double-buffered.  A group's xform for pass s + 1 is drawn right after its first slot's pass-s
 // evaluation (the same point of that slot's RNG stream) into the other xform-id buffer.
-template <int THREADS, int SPT, class Eval, int SPLAT = -1, int RESET = -1, int PIPE = 0>
+//
+// CLUSTER = K > 1 spreads a mixing domain over the K CTAs of a cluster (SLOTS = its slots / K), for
+// simulations whose domains are fewer than the SMs: with one CTA per domain the others idle.  The
+// arrival on the pass's cluster barrier comes right after the walker's store, the wait before the next
+// pass's first read, so the splat and the group's xform draw (as PIPE draws it) pass under it.  What is
+// left is one warp's chain per pass: 65,536 walkers of the three-xform genome in 2048-slot domains take
+// 3.9 us per pass on 32 CTAs and 2.7 us on 128 (16.6 -> 24.0 Gpoints/s), in 4096-slot ones 6.3 us on 16
+// and 4.4 us on 128.
+template <int THREADS, int SPT, class Eval, int SPLAT = -1, int RESET = -1, int PIPE = 0, int CLUSTER = 1>
 __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
     static_assert(!PIPE || SPT >= 3, "the pipelined exchange needs three phases");
-    constexpr uint32_t SLOTS = (uint32_t)THREADS * SPT;
+    static_assert(!PIPE || CLUSTER == 1, "one exchange or the other");
+    constexpr uint32_t SLOTS = (uint32_t)THREADS * SPT;       // of this CTA
+    constexpr uint32_t DOMAIN_SLOTS = SLOTS * CLUSTER;        // of the mixing domain
     constexpr int G = SLOTS / kGroup;
     extern __shared__ __align__(16) unsigned char smem[];
     uint32_t* s_prog = reinterpret_cast<uint32_t*>(smem);
@@ -137,9 +163,11 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
         tt.rgba[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         tt.count[i] = 0u;
     }
-    const uint32_t chunk = blockIdx.x;  // mixing domain
+    const uint32_t chunk = blockIdx.x / CLUSTER;  // mixing domain
+    const uint32_t rank = blockIdx.x % CLUSTER;   // of this CTA in it
     const uint32_t ts = chunk / A.chunks_per_ts;
-    const uint32_t gid0 = (chunk - ts * A.chunks_per_ts) * SLOTS;  // first slot within the temporal sample
+    const uint32_t slot0 = rank * SLOTS;          // first slot within the mixing domain
+    const uint32_t gid0 = (chunk - ts * A.chunks_per_ts) * DOMAIN_SLOTS + slot0;  // and within the temporal sample
     const size_t ts_base = (size_t)ts * A.ppts;
 
     if (PIPE && tid == 0) {
@@ -178,14 +206,14 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
     const bool reset = RESET >= 0 ? RESET != 0 : A.reset != 0;
     uint32_t drawn = 0, emitted = 0;
     // flame.glsl:51-53: the first slot of each 256-slot group draws the group's xform for pass s
-    // from its own RNG stream (the pipelined exchange draws inside the pass loop instead)
+    // from its own RNG stream (the pipelined and cluster exchanges draw inside the pass loop instead)
     auto draw_group_xform = [&](uint32_t s, uint32_t ls, Jsf& rng) {
         const int xi = select_xform(s_prog, randf(rng));
         s_xid[(s & 1) * G + ls / kGroup] = xi;
         if (A.trace && A.pass0 + s < A.trace_passes)
             A.trace[(size_t)(A.pass0 + s) * A.n_groups + (ts_base + gid0 + ls) / kGroup] = (uint8_t)xi;
     };
-    if (PIPE && dphase >= 0) {
+    if ((PIPE || CLUSTER > 1) && dphase >= 0) {
         const uint32_t ls = phase_slot<THREADS>(dphase, tid);
         const uint4 r4 = s_rng[ls];
         Jsf rng{r4.x, r4.y, r4.z, r4.w};
@@ -193,18 +221,32 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
         s_rng[ls] = make_uint4(rng.a, rng.b, rng.c, rng.d);
     }
     __syncthreads();
+    if (CLUSTER > 1) cluster_arrive();
     // PIPE: false after a wait ran out — the thread counts it (the host reports RF_ERR_TIMEOUT)
     // and waits no more, so the launch still ends
     bool synced = true;
+    constexpr bool kAhead = CLUSTER > 1 && SPT == 1;
+    uint32_t ahead[SPT];  // this pass's sources
+    if (kAhead)
+        for (int k = 0; k < SPT; k++) ahead[k] = slot0 + phase_slot<THREADS>(k, tid);
 
     for (uint32_t s = 0; s < A.steps; s++) {
         const int buf = s & 1;
         // this pass's sources in the exchange buffer (identity on the gather pass)
         uint32_t src[SPT];
 #pragma unroll
-        for (int k = 0; k < SPT; k++)
-            src[k] = (s == 0) ? phase_slot<THREADS>(k, tid) : (uint32_t)A.table[(size_t)s_perm[s] * SLOTS + phase_slot<THREADS>(k, tid)];
-        if (!PIPE) {
+        for (int k = 0; k < SPT; k++) {
+            if (kAhead) src[k] = ahead[k];
+            else src[k] = (s == 0) ? slot0 + phase_slot<THREADS>(k, tid)
+                                   : (uint32_t)A.table[(size_t)s_perm[s] * DOMAIN_SLOTS + slot0 + phase_slot<THREADS>(k, tid)];
+        }
+        if (CLUSTER > 1) {
+            cluster_wait();
+            // the next pass's sources, a pass ahead: with a few warps per SM their L2 latency is not hidden
+#pragma unroll
+            for (int k = 0; k < SPT; k++)
+                if (kAhead && s + 1 < A.steps) ahead[k] = A.table[(size_t)s_perm[s + 1] * DOMAIN_SLOTS + slot0 + phase_slot<THREADS>(k, tid)];
+        } else if (!PIPE) {
             if (dphase >= 0) {
                 const uint32_t ls = phase_slot<THREADS>(dphase, tid);
                 const uint4 r4 = s_rng[ls];
@@ -227,7 +269,7 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
                 synced = false;
                 atomicAdd(A.counters + 3, 1ull);
             }
-            const float4 v = s_w[buf * SLOTS + j];
+            const float4 v = CLUSTER > 1 ? cluster_load(s_w + buf * SLOTS + j % SLOTS, j / SLOTS) : s_w[buf * SLOTS + j];
             float x = v.x, y = v.y, c = v.z;
             const uint4 r4 = s_rng[ls];
             Jsf rng{r4.x, r4.y, r4.z, r4.w};
@@ -260,9 +302,10 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
             s_w[(buf ^ 1) * SLOTS + ls] = make_float4(x, y, c, 0.0f);
             // the group's xform for the next pass, at the point of the slot's stream where the
             // pass-barrier form draws it
-            if (PIPE && k == dphase && s + 1 < A.steps) draw_group_xform(s + 1, ls, rng);
+            if ((PIPE || CLUSTER > 1) && k == dphase && s + 1 < A.steps) draw_group_xform(s + 1, ls, rng);
             s_rng[ls] = make_uint4(rng.a, rng.b, rng.c, rng.d);
             if (PIPE && k >= SPT - 2) xbar_arrive(s_bar + (k - (SPT - 2)));
+            if (CLUSTER > 1 && k == SPT - 1) cluster_arrive();
             if (A.draw) {
                 if (op > 0.0f) emitted++;
                 const float px = fmaf(A.ss[0], ex, fmaf(A.ss[2], ey, A.ss[4]));
@@ -297,6 +340,7 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
             }
         }
     }
+    if (CLUSTER > 1) cluster_wait();  // no CTA leaves while another reads its walkers
     // the tile's non-empty bins into the histogram, once per launch
     if (tile_bins) {
         __syncthreads();

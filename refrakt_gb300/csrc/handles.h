@@ -54,6 +54,8 @@ struct rf_sim {
     cudaEvent_t tile_ev[4] = {nullptr, nullptr, nullptr, nullptr};
     int spec_reset = -1;              // the reset setting compiled into the specialised kernel
     int spec_pipe = 0;                // 1: the specialised kernel has the pipelined walker exchange
+    int spec_cluster = 1;             // CTAs per mixing domain compiled into it
+    int cluster = 1;                  // CTAs per mixing domain of the warmed flame's launches (RF_EXCHANGE_AUTO)
     uint32_t table_phases = 0;        // phases per pass the shuffle table is pipelined for (0: uniform)
     int exchange = RF_EXCHANGE_AUTO;  // rf_set_exchange
     // RF_EXCHANGE_AUTO: 0/1 — the next full drawing launch is timed as the barrier / pipelined form;

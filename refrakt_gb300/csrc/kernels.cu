@@ -185,6 +185,42 @@ cudaError_t launch_chaos(int threads, int slots, const ChaosArgs& a, uint32_t gr
     }
 }
 
+// the chaos kernel with a cluster CTA's slots (the same shared memory as a specialised one)
+static const void* cluster_probe(int local) {
+    return local == 256    ? (const void*)chaos_kernel<256, 1>
+           : local == 512  ? (const void*)chaos_kernel<512, 1>
+           : local == 1024 ? (const void*)chaos_kernel<1024, 1>
+                           : (const void*)chaos_kernel<1024, 2>;
+}
+
+int chaos_cluster(int slots, uint64_t domains, uint32_t prog_words, uint32_t steps) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 1;
+    for (int k = 8; k >= 2; k /= 2) {
+        const int local = slots / k;  // slots of a CTA, on up to 1024 threads
+        if (local < kGroup || domains * (uint64_t)k > (uint64_t)sms) continue;
+        const size_t smem = chaos_smem_bytes(local, prog_words, steps);
+        const void* f = cluster_probe(local);
+        cudaLaunchConfig_t c{};
+        c.gridDim = dim3((unsigned)(domains * k));
+        c.blockDim = dim3(local < 1024 ? local : 1024);
+        c.dynamicSmemBytes = smem;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeClusterDimension;
+        at.val.clusterDim.x = k;
+        at.val.clusterDim.y = at.val.clusterDim.z = 1;
+        c.attrs = &at;
+        c.numAttrs = 1;
+        int n = 0;
+        if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+            cudaOccupancyMaxActiveClusters(&n, f, &c) == cudaSuccess && (uint64_t)n >= domains)
+            return k;
+        cudaGetLastError();
+    }
+    return 1;
+}
+
 cudaError_t launch_init_rng(uint4* rng, uint64_t n, uint64_t seed, cudaStream_t st) {
     const uint32_t b = 256;
     init_rng_kernel<<<(unsigned)((n + b - 1) / b), b, 0, st>>>(rng, n, seed);

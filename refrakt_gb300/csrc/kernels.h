@@ -16,6 +16,10 @@ namespace rfk {
 
 size_t chaos_smem(int slots, uint32_t prog_words, uint32_t steps, uint32_t tile_bins = 0, int pipe = 0);
 constexpr size_t kMaxCtaSmem = 232448;  // dynamic shared memory a CTA may opt into (227 KB)
+// CTAs per mixing domain that a simulation of `domains` domains of `slots` should spread over (the
+// cluster exchange, chaos_body.cuh), 1 for none: the most (8, 4, 2) that leave each CTA a 256-slot
+// group, no more CTAs than SMs and every cluster resident at once
+int chaos_cluster(int slots, uint64_t domains, uint32_t prog_words, uint32_t steps);
 bool chaos_shape_supported(int threads, int slots);
 cudaError_t launch_chaos(int threads, int slots, const ChaosArgs& a, uint32_t grid, cudaStream_t st);
 cudaError_t launch_merge_records(float4* rec, size_t n, float4* bins, uint32_t* hits, cudaStream_t st);

@@ -147,7 +147,7 @@ static std::string gen_eval(const std::vector<uint32_t>& prog) {
 }
 
 std::string spec_source(const std::vector<uint32_t>& prog, int threads, int spt, SpecKind kind, int splat, int reset,
-                        int pipe) {
+                        int pipe, int cluster) {
     std::ostringstream o;
     o << "// generated: genome-specialised " << (kind == SpecKind::Batch ? "batch" : "chaos") << " kernel\n"
       << (kind == SpecKind::Batch ? "#include \"batch_body.cuh\"\n" : "#include \"chaos_body.cuh\"\n")
@@ -157,10 +157,12 @@ std::string spec_source(const std::vector<uint32_t>& prog, int threads, int spt,
           << ") rfk_batch_spec(const rfk::BatchArgs A) {\n  rfk::batch_body<" << threads << ", " << spt
           << ", rfk::GenEval>(A);\n}\n";
     else
-        o << "extern \"C\" __global__ void __launch_bounds__(" << threads << ", " << 1024 / threads
+        o << "extern \"C\" __global__ void "
+          << (cluster > 1 ? "__cluster_dims__(" + std::to_string(cluster) + ", 1, 1) " : std::string())
+          << "__launch_bounds__(" << threads << ", " << (cluster > 1 ? 1 : 1024 / threads)
           << ") rfk_chaos_spec(const rfk::ChaosArgs A) {\n  rfk::chaos_body<" << threads << ", " << spt
           << ", rfk::GenEval, " << (splat >= 0 ? splat : -1) << ", " << (reset >= 0 ? reset : -1) << ", "
-          << (pipe ? 1 : 0) << ">(A);\n}\n";
+          << (pipe ? 1 : 0) << (cluster > 1 ? ", " + std::to_string(cluster) : std::string()) << ">(A);\n}\n";
     return o.str();
 }
 
@@ -197,11 +199,11 @@ int spec_compile(const std::string& src, std::vector<char>& cubin) {
 }
 
 int spec_kernel(const std::vector<uint32_t>& prog, int threads, int slots, int device, const void** out,
-                SpecKind kind, int splat, int reset, int pipe) {
+                SpecKind kind, int splat, int reset, int pipe, int cluster) {
     *out = nullptr;
     if (prog.size() < (size_t)H_XOFF || prog[H_MAGIC] != kProgMagic)
         return fail(RF_ERR_INVALID_ARG, "spec_kernel: not a compiled genome");
-    const std::string src = spec_source(prog, threads, slots / threads, kind, splat, reset, pipe);
+    const std::string src = spec_source(prog, threads, slots / threads, kind, splat, reset, pipe, cluster);
     const std::string key = std::to_string(device) + "\n" + src;
     {
         std::lock_guard<std::mutex> lk(g_mu);
