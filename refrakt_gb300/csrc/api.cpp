@@ -15,6 +15,7 @@
 
 #include "internal.h"
 #include "kernels.h"
+#include "scratch.h"
 
 namespace rfk {
 
@@ -690,6 +691,7 @@ int rf_sim_destroy(rf_sim* s) {
         if (ev) cudaEventDestroy(ev);
     for (auto ev : s->tile_ev)
         if (ev) cudaEventDestroy(ev);
+    scratch_trim();
     delete s;
     return RF_OK;
 }
@@ -929,7 +931,7 @@ int rf_tonemap_filter(const float* rgba, uint32_t w, uint32_t h, uint32_t ss, fl
     cudaStream_t st = (cudaStream_t)stream;
     double* stats = nullptr;
     if (!(k2 > 0.0f)) {
-        RF_CUDA(cudaMallocAsync((void**)&stats, 3 * sizeof(double), st));
+        RF_CUDA(scratch_alloc(&stats, 3, st));
         cudaError_t e = launch_stats((const float4*)rgba, w, h, stats, st);
         if (e != cudaSuccess) { cudaFreeAsync(stats, st); return cuda_fail(e, "stats"); }
     }
@@ -951,17 +953,17 @@ int rf_density_tonemap(const float* in, uint32_t w, uint32_t h, int radius, int 
     cudaStream_t st = (cudaStream_t)stream;
     const size_t n = (size_t)w * h;
     std::vector<float> wts;
-    density_weights(radius, min_radius, wts);
+    if (density_reads_weights(radius, min_radius)) density_weights(radius, min_radius, wts);
     const bool fused = density_tonemap_fused(radius, min_radius, ss);
     uint8_t* rad = nullptr;
     float* dw = nullptr;
     double* stats = nullptr;
     float4* de = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&rad, n, st);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&dw, wts.size() * sizeof(float), st);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&stats, 3 * sizeof(double), st);
-    if (e == cudaSuccess && !fused) e = cudaMallocAsync((void**)&de, n * sizeof(float4), st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dw, wts.data(), wts.size() * sizeof(float), cudaMemcpyHostToDevice, st);
+    cudaError_t e = scratch_alloc(&rad, n, st);
+    if (e == cudaSuccess && !wts.empty()) e = scratch_alloc(&dw, wts.size(), st);
+    if (e == cudaSuccess) e = scratch_alloc(&stats, 3, st);
+    if (e == cudaSuccess && !fused) e = scratch_alloc(&de, n, st);
+    if (e == cudaSuccess && dw) e = cudaMemcpyAsync(dw, wts.data(), wts.size() * sizeof(float), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess)
         e = launch_density_tonemap((const float4*)in, w, h, radius, min_radius, curve, ss, gamma, brightness, vibrancy,
                                    k2, (float4*)out_f32, (uchar4*)out8, rad, dw, stats, de, st);
@@ -975,7 +977,7 @@ int rf_hist_stats(const float* rgba, uint32_t w, uint32_t h, double* out3, void*
     if (!rgba || !out3) return fail(RF_ERR_INVALID_ARG, "rf_hist_stats: null argument");
     cudaStream_t st = (cudaStream_t)stream;
     double* d = nullptr;
-    RF_CUDA(cudaMallocAsync((void**)&d, 3 * sizeof(double), st));
+    RF_CUDA(scratch_alloc(&d, 3, st));
     cudaError_t e = launch_stats((const float4*)rgba, w, h, d, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out3, d, 3 * sizeof(double), cudaMemcpyDeviceToHost, st);
     cudaFreeAsync(d, st);
@@ -994,7 +996,7 @@ int rf_tonemap(const float* rgba, uint32_t w, uint32_t h, uint32_t ss, float gam
     cudaStream_t st = (cudaStream_t)stream;
     double* stats = nullptr;
     if (!(k2 > 0.0f)) {
-        RF_CUDA(cudaMallocAsync((void**)&stats, 3 * sizeof(double), st));
+        RF_CUDA(scratch_alloc(&stats, 3, st));
         cudaError_t e = launch_stats((const float4*)rgba, w, h, stats, st);
         if (e != cudaSuccess) { cudaFreeAsync(stats, st); return cuda_fail(e, "stats"); }
     }
@@ -1020,7 +1022,7 @@ int rf_probe_xform(rf_flame* f, int xform, uint32_t n, const float* in, uint32_t
     if (int rc = genome_program(f->g, *f->reg, prog)) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     uint32_t* d = nullptr;
-    RF_CUDA(cudaMallocAsync((void**)&d, prog.size() * 4, st));
+    RF_CUDA(scratch_alloc(&d, prog.size(), st));
     cudaError_t e = cudaMemcpyAsync(d, prog.data(), prog.size() * 4, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess && n) e = launch_probe(d, xform, n, in, rng, first_run, out, st);
     cudaFreeAsync(d, st);
@@ -1119,7 +1121,7 @@ int rf_render(rf_sim* s, rf_flame* f, const rf_render_desc* d, uint8_t* out, dou
             if (e != cudaSuccess) return done(cuda_fail(e, "cudaMalloc"));
             s->r_rad_n = nb;
         }
-        if (!s->r_dw) {  // every radius up to 100: the table is a prefix of itself for any R
+        if (!s->r_dw && density_reads_weights(R, mn)) {  // every radius up to 100: the table is a prefix of itself for any R
             std::vector<float> wts;
             density_weights(100, 0, wts);
             e = cudaMalloc((void**)&s->r_dw, wts.size() * sizeof(float));

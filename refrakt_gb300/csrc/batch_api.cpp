@@ -25,6 +25,7 @@
 #include "denoise_ops.h"
 #include "handles.h"
 #include "kernels.h"
+#include "scratch.h"
 
 using namespace rfk;
 
@@ -114,6 +115,7 @@ void destroy_batch(rf_batch* b) {
     if (b->graph) cudaGraphDestroy(b->graph);
     void* ptrs[] = {b->pool, b->table, b->dinst, b->dunits, b->queue, b->counters, b->stats};
     for (void* p : ptrs) if (p) cudaFree(p);
+    scratch_trim();
     if (b->ev0) cudaEventDestroy(b->ev0);
     if (b->ev1) cudaEventDestroy(b->ev1);
     for (auto ev : b->fork_join)
@@ -368,7 +370,8 @@ int rf_batch_create(const rf_batch_item* items, uint32_t n, const rf_batch_desc*
         off[i].dw = kNone;
         if (d->density_estimation && (it.est_radius > 0 || it.est_min > 0)) {
             std::vector<float> wts;
-            density_weights(std::min(100, it.est_radius), std::min(100, it.est_min), wts);
+            const int R = std::min(100, it.est_radius), mn = std::min(100, it.est_min);
+            if (density_reads_weights(R, mn)) density_weights(R, mn, wts);
             off[i].dw = put(wts.data(), wts.size() * sizeof(float));
         }
         b->max_prog_words = std::max(b->max_prog_words, (uint32_t)it.prog.size());

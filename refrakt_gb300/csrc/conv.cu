@@ -31,6 +31,7 @@
 #include <cuda_runtime.h>
 
 #include "conv.h"
+#include "gemm.h"
 #include "umma.cuh"
 
 namespace rfk {
@@ -44,8 +45,6 @@ constexpr int kLoadWarps = kLoaders / 32, kMmaWarp = kLoadWarps, kDrainWarp = kM
 constexpr int kMaxStages = 4;
 constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr size_t kMaxSmem = 227 * 1024;
-
-__device__ int g_conv_error;  // 0, or 1 + the role whose mbarrier wait ran out
 
 struct Geom {
     uint32_t tiles_x, tiles_y, tiles;
@@ -150,19 +149,21 @@ __device__ __forceinline__ void cp_wait_pending(uint32_t left) {
     }
 }
 
-__device__ __forceinline__ void conv_fail(int* s_fail, int code) {
-    *reinterpret_cast<volatile int*>(s_fail) = 1;
-    atomicExch(&g_conv_error, code);
-}
-__device__ __forceinline__ bool conv_failed(const int* s_fail) { return *reinterpret_cast<const volatile int*>(s_fail) != 0; }
-
 // barriers: full[stages], empty[stages], acc_full[2], acc_empty[2]
 struct Bars {
     uint64_t *full, *empty, *acc_full, *acc_empty;
     uint32_t* tmem;
     int* fail;
+    int* error;  // the host's error word
 };
-__device__ __forceinline__ Bars bars_at(unsigned char* p) {
+// b.error gets 1 loading, 2 an accumulator's release, 3 a stage, 4 an accumulator
+__device__ __forceinline__ void conv_fail(const Bars& b, int code) {
+    *reinterpret_cast<volatile int*>(b.fail) = 1;
+    umma::report_error(b.error, code);
+}
+__device__ __forceinline__ bool conv_failed(const int* s_fail) { return *reinterpret_cast<const volatile int*>(s_fail) != 0; }
+
+__device__ __forceinline__ Bars bars_at(unsigned char* p, int* error) {
     Bars b;
     b.full = reinterpret_cast<uint64_t*>(p);
     b.empty = b.full + kMaxStages;
@@ -170,6 +171,7 @@ __device__ __forceinline__ Bars bars_at(unsigned char* p) {
     b.acc_empty = b.acc_full + 2;
     b.tmem = reinterpret_cast<uint32_t*>(b.acc_empty + 2);
     b.fail = reinterpret_cast<int*>(b.tmem + 1);
+    b.error = error;
     return b;
 }
 constexpr uint32_t kBarBytes = (2 * kMaxStages + 4) * 8 + 16;
@@ -203,7 +205,7 @@ __device__ __forceinline__ void load_loop(const Bars& b, uint32_t count, uint32_
             announced++;
         }
         if (use > 0 && !umma::mbar_wait(&b.empty[st], (use - 1) & 1u, kWaitLimit)) {
-            conv_fail(b.fail, 1);
+            conv_fail(b, 1);
             break;
         }
         if (conv_failed(b.fail)) break;
@@ -444,7 +446,7 @@ template <int EPI>
 __global__ void __launch_bounds__(kThreads, 1) conv_kernel(const __grid_constant__ ConvArgs A, const __grid_constant__ Geom G) {
     constexpr bool kSums = EPI == kConvMask || EPI == kConvConcat || EPI == kConvPool;
     extern __shared__ __align__(128) unsigned char smem[];
-    const Bars B = bars_at(smem + G.bars);
+    const Bars B = bars_at(smem + G.bars, A.error);
     float* s_gb = reinterpret_cast<float*>(smem + G.bars + kBarBytes);  // 8 warps x np (kSums)
     const uint32_t base = umma::smem_u32(smem);
     const int tid = threadIdx.x, warp = tid >> 5;
@@ -502,11 +504,11 @@ __global__ void __launch_bounds__(kThreads, 1) conv_kernel(const __grid_constant
                 const uint32_t u = i >> 1;
                 if (conv_failed(B.fail)) break;
                 if (u > 0 && !umma::mbar_wait(&B.acc_empty[buf], (u - 1) & 1u, kWaitLimit)) {
-                    conv_fail(B.fail, 2);
+                    conv_fail(B, 2);
                     break;
                 }
                 if (!umma::mbar_wait(&B.full[st], use & 1u, kWaitLimit)) {
-                    conv_fail(B.fail, 3);
+                    conv_fail(B, 3);
                     break;
                 }
                 umma::fence_after_sync();
@@ -544,7 +546,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_kernel(const __grid_constant
         Tile t(G, blockIdx.x + buf * gridDim.x, 2 * gridDim.x);
         for (uint32_t i = buf; i < count; i += 2, t.next(G)) {
             if (!umma::mbar_wait(&B.acc_full[buf], (i >> 1) & 1u, kWaitLimit)) {
-                conv_fail(B.fail, 4);
+                conv_fail(B, 4);
                 break;
             }
             umma::fence_after_sync();
@@ -618,6 +620,7 @@ struct WgradLayer {
 struct WgradArgs {
     WgradLayer layer[kMaxWgradLayers];
     uint32_t layers, bars;
+    int* error;
     // the head's bias gradient, by the last CTAs of the grid
     uint32_t bias_first;
     const __nv_bfloat16* bias_dz;
@@ -786,7 +789,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) conv_wgrad_kernel(const __gr
         head_bias(W, blockIdx.x, tid);
         return;
     }
-    const Bars B = bars_at(smem + W.bars);
+    const Bars B = bars_at(smem + W.bars, W.error);
     const uint32_t base = umma::smem_u32(smem);
     uint32_t li = 0;
     while (li + 1 < W.layers && blockIdx.x >= W.layer[li + 1].first) li++;
@@ -814,7 +817,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) conv_wgrad_kernel(const __gr
         else load_segments<kPlain>(B, L, p0, p1, count, base, stage, dy, dx, tid);
         // the accumulators into gw: a warp its tensor-memory lane quarter and every fourth 16 columns
         const uint32_t q4 = (uint32_t)warp & 3u, share = (uint32_t)warp >> 2;
-        if (count && !umma::mbar_wait(&B.acc_full[0], 0u, kWaitLimit)) conv_fail(B.fail, 4);
+        if (count && !umma::mbar_wait(&B.acc_full[0], 0u, kWaitLimit)) conv_fail(B, 4);
         umma::fence_after_sync();
         if (count && !conv_failed(B.fail)) {
             const uint32_t K = L.taps * C;
@@ -844,7 +847,7 @@ __global__ void __launch_bounds__(kWgradThreads, 1) conv_wgrad_kernel(const __gr
         for (uint32_t i = 0; i < count; i++) {
             if (conv_failed(B.fail)) { ok = false; break; }
             if (!umma::mbar_wait(&B.full[st], use & 1u, kWaitLimit)) {
-                conv_fail(B.fail, 3);
+                conv_fail(B, 3);
                 ok = false;
                 break;
             }
@@ -938,7 +941,9 @@ bool conv_supported(uint32_t channels, uint32_t N, uint32_t taps) {
     return N > 0 && conv_geom(G, channels, N, taps, &smem);
 }
 
-cudaError_t launch_conv(const ConvArgs& a, ConvEpilogue epi, cudaStream_t st) {
+cudaError_t launch_conv(const ConvArgs& args, ConvEpilogue epi, cudaStream_t st) {
+    ConvArgs a = args;
+    if (!(a.error = error_word())) return cudaErrorMemoryAllocation;
     if ((a.taps != 9 && a.taps != 1) || a.n == 0 || a.h == 0 || a.w == 0 || a.N == 0 || a.ca % 8 || a.cb % 8 || a.ldb % 8 ||
         a.ldb < a.taps * (a.ca + a.cb) || (((uintptr_t)a.xa | (uintptr_t)a.xb | (uintptr_t)a.B) & 15))
         return cudaErrorInvalidValue;
@@ -1006,6 +1011,7 @@ cudaError_t launch_conv_wgrad(const WgradTask* tasks, uint32_t count, const __nv
                               float* bias_gb, cudaStream_t st) {
     if (count == 0 || count > (uint32_t)kMaxWgradLayers || bias_pixels > 0x7fffffffull) return cudaErrorInvalidValue;
     WgradArgs W{};
+    if (!(W.error = error_word())) return cudaErrorMemoryAllocation;
     W.layers = count;
     W.bias_first = bias_dz ? kBiasCtas : 0;
     W.bias_dz = bias_dz;
@@ -1074,13 +1080,6 @@ cudaError_t launch_conv_wgrad(const WgradTask* tasks, uint32_t count, const __nv
     if (e != cudaSuccess) return e;
     conv_wgrad_kernel<<<ctas, kWgradThreads, smem, st>>>(W);
     return cudaGetLastError();
-}
-
-cudaError_t conv_error(int* out) {
-    cudaError_t e = cudaMemcpyFromSymbol(out, g_conv_error, sizeof(int));
-    const int zero = 0;
-    if (e == cudaSuccess && *out) e = cudaMemcpyToSymbol(g_conv_error, &zero, sizeof(int));
-    return e;
 }
 
 }  // namespace rfk

@@ -49,6 +49,7 @@ struct ConvArgs {
     const float* target;
     float* out;
     double* loss;
+    int* error;                // set by the launcher
 };
 
 // whether launch_conv takes the shape: ca + cb a multiple of 16 (or 8 channels in all) and a tile's
@@ -68,8 +69,5 @@ constexpr int kMaxWgradLayers = 16;
 // with bias_dz (8 channels per pixel, the head's dz) also the head's bias gradient into bias_gb[0..2]
 cudaError_t launch_conv_wgrad(const WgradTask* tasks, uint32_t count, const __nv_bfloat16* bias_dz, uint64_t bias_pixels,
                               float* bias_gb, cudaStream_t st);
-
-// reads and clears the kernels' error word (0 = no bounded wait ran out)
-cudaError_t conv_error(int* out);
 
 }  // namespace rfk

@@ -20,8 +20,10 @@
 
 #include "conv.h"
 #include "denoise_ops.h"
+#include "gemm.h"
 #include "internal.h"
 #include "kernels.h"
+#include "scratch.h"
 #include "refrakt.h"
 
 using namespace rfk;
@@ -270,6 +272,7 @@ int rf_denoiser_create(const rf_denoiser_desc* desc, rf_denoiser** out) {
     if (cudaSetDevice(D->device) != cudaSuccess) return bail(fail(RF_ERR_NO_DEVICE, "rf_denoiser_create: no such device"));
     cudaError_t e = cudaStreamCreateWithFlags(&D->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(e, "stream"));
+    error_word();  // (allocates: before any capture of the denoiser's work)
     build_graph(D);
     // parameters, He-normal initialisation from a seeded generator
     const size_t np = rf_denoiser_num_params(D);
@@ -330,6 +333,7 @@ int rf_denoiser_destroy(rf_denoiser* D) {
     cudaSetDevice(D->device);
     if (D->stream) cudaStreamSynchronize(D->stream);
     for (void* p : D->allocs) cudaFree(p);
+    scratch_trim();
     if (D->stream) cudaStreamDestroy(D->stream);
     delete D;
     return RF_OK;
@@ -403,7 +407,7 @@ int rf_denoiser_features(const float* bins_rgba, uint32_t width, uint32_t height
     double* stats = nullptr;
     cudaError_t e = cudaSuccess;
     if (!(k2 > 0.0f)) {
-        e = cudaMallocAsync(&stats, 3 * sizeof(double), st);
+        e = scratch_alloc(&stats, 3, st);
         if (e == cudaSuccess) e = launch_stats(reinterpret_cast<const float4*>(bins_rgba), width, height, stats, st);
     }
     if (e == cudaSuccess)

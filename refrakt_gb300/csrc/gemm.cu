@@ -21,6 +21,8 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <atomic>
+#include <mutex>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -35,8 +37,6 @@ constexpr int kStages = 3;
 constexpr int kThreads = 128;
 constexpr uint32_t kBM = 128;
 constexpr uint32_t kWaitLimit = 1u << 22;
-
-__device__ int g_gemm_error;  // 0, or 1 + the stage whose mbarrier wait ran out
 
 template <int BN>
 __host__ __device__ constexpr size_t gemm_smem() {
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_gemm_kernel(const GemmArgs g
                 const uint32_t ps = (kb - 1) % kStages;
                 if (!umma::mbar_wait(&bar[ps], ((kb - 1) / kStages) & 1u, kWaitLimit)) {
                     *s_fail = 1;
-                    atomicExch(&g_gemm_error, 1 + (int)ps);
+                    umma::report_error(g.error, 1 + (int)ps);
                 }
             }
             const uint32_t ns = nxt % kStages;
@@ -268,7 +268,7 @@ __global__ void __launch_bounds__(kThreads, 1) umma_gemm_kernel(const GemmArgs g
         const uint32_t ls = (nk - 1) % kStages;
         if (!umma::mbar_wait(&bar[ls], ((nk - 1) / kStages) & 1u, kWaitLimit)) {
             *s_fail = 1;
-            atomicExch(&g_gemm_error, 1 + (int)ls);
+            umma::report_error(g.error, 1 + (int)ls);
         }
     }
     umma::cp_async_wait<0>();
@@ -304,9 +304,9 @@ __host__ __device__ constexpr size_t tma_smem() {
     return 1024 + (size_t)tma_stages<BN>() * (kBM * 128 + BN * 128) + (size_t)kBM * kStageLd * 4 + 256;
 }
 
-__device__ __forceinline__ void gemm_fail(int* s_fail, int code) {
+__device__ __forceinline__ void gemm_fail(const GemmArgs& g, int* s_fail, int code) {
     *reinterpret_cast<volatile int*>(s_fail) = 1;
-    atomicExch(&g_gemm_error, code);
+    umma::report_error(g.error, code);
 }
 __device__ __forceinline__ bool gemm_failed(const int* s_fail) { return *reinterpret_cast<const volatile int*>(s_fail) != 0; }
 
@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
                 for (uint32_t kb = 0; kb < c.nk; kb++, it++) {
                     const uint32_t st = it % S, use = it / S;
                     if (use > 0 && !umma::mbar_wait(&empty[st], (use - 1) & 1u, kWaitLimit)) {
-                        gemm_fail(s_fail, 1 + (int)st);
+                        gemm_fail(g, s_fail, 1 + (int)st);
                         break;
                     }
                     if (gemm_failed(s_fail)) break;
@@ -404,14 +404,14 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
                 const uint32_t idesc = umma::idesc_bf16_f32(kBM, n_tile);
                 bool ok = !gemm_failed(s_fail);
                 if (ok && u > 0 && !umma::mbar_wait(&acc_empty[buf], (u - 1) & 1u, kWaitLimit)) {
-                    gemm_fail(s_fail, 1 + 2 * S + (int)buf);
+                    gemm_fail(g, s_fail, 1 + 2 * S + (int)buf);
                     ok = false;
                 }
                 umma::fence_after_sync();
                 for (uint32_t kb = 0; ok && kb < c.nk; kb++, it++) {
                     const uint32_t st = it % S;
                     if (!umma::mbar_wait(&full[st], (it / S) & 1u, kWaitLimit)) {
-                        gemm_fail(s_fail, 1 + S + (int)st);
+                        gemm_fail(g, s_fail, 1 + S + (int)st);
                         ok = false;
                         break;
                     }
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
             const TileCoord c = tile_coord(g, t, tiles_m, tiles_n, BN);
             const uint32_t buf = i & 1u, u = i >> 1;
             if (!umma::mbar_wait(&acc_full[buf], u & 1u, kWaitLimit)) {
-                gemm_fail(s_fail, 3 + 2 * S + (int)buf);
+                gemm_fail(g, s_fail, 3 + 2 * S + (int)buf);
                 break;
             }
             umma::fence_after_sync();
@@ -527,6 +527,7 @@ cudaError_t launch_bn(const GemmArgs& g, uint32_t splits, cudaStream_t st) {
 cudaError_t launch_gemm(GemmArgs g, uint32_t splits, cudaStream_t st) {
     if (g.K % 8 || g.lda % 8 || g.ldb % 8 || g.M == 0 || g.N == 0) return cudaErrorInvalidValue;
     if (((uintptr_t)g.A | (uintptr_t)g.B) & 15) return cudaErrorInvalidValue;
+    if (!(g.error = error_word())) return cudaErrorMemoryAllocation;
     if (splits == 0) splits = 1;
     const uint32_t kblocks = (g.K + umma::kTileK - 1) / umma::kTileK;
     if (splits > kblocks && kblocks > 0) splits = kblocks;
@@ -551,6 +552,7 @@ cudaError_t launch_gemm_conv(GemmArgs g, cudaStream_t st) {
     if (!g.xa || (g.cb && !g.xb) || (uint64_t)g.n * g.h * g.w != g.M || g.K != 9u * (g.ca + g.cb) || g.ldb % 8 ||
         g.N == 0 || ((uintptr_t)g.xa | (uintptr_t)g.xb | (uintptr_t)g.B) & 15)
         return cudaErrorInvalidValue;
+    if (!(g.error = error_word())) return cudaErrorMemoryAllocation;
     g.A = nullptr;
     g.lda = 0;
     g.k_per_split = (g.K + umma::kTileK - 1) / umma::kTileK * umma::kTileK;
@@ -559,11 +561,25 @@ cudaError_t launch_gemm_conv(GemmArgs g, cudaStream_t st) {
     return launch_bn<256, true>(g, 1, st);
 }
 
-cudaError_t gemm_error(int* out) {
-    cudaError_t e = cudaMemcpyFromSymbol(out, g_gemm_error, sizeof(int));
-    const int zero = 0;
-    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_gemm_error, &zero, sizeof(int));
-    return e;
+int* error_word() {
+    static std::atomic<int*> word{nullptr};
+    static std::mutex mu;
+    int* p = word.load(std::memory_order_acquire);
+    if (p) return p;
+    std::lock_guard<std::mutex> lock(mu);
+    p = word.load(std::memory_order_relaxed);
+    if (!p && cudaHostAlloc((void**)&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) {
+        *p = 0;
+        word.store(p, std::memory_order_release);
+        return p;
+    }
+    if (!p) cudaGetLastError();
+    return p;
+}
+
+int take_error() {
+    int* p = error_word();
+    return p ? __atomic_exchange_n(p, 0, __ATOMIC_ACQ_REL) : 0;
 }
 
 }  // namespace rfk

@@ -13,11 +13,10 @@ using namespace rfk;
 
 namespace {
 
-// waits for the launch, then reads the kernels' bounded-wait error word
-int finish(const char* fn, cudaError_t e, cudaStream_t st, cudaError_t (*error)(int*) = gemm_error) {
+// waits for the launch, then takes the kernels' bounded-wait error word
+int finish(const char* fn, cudaError_t e, cudaStream_t st) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    int werr = 0;
-    if (e == cudaSuccess) e = error(&werr);
+    const int werr = take_error();
     if (e != cudaSuccess) return fail(RF_ERR_CUDA, std::string(fn) + ": " + cudaGetErrorString(e));
     if (werr) return fail(RF_ERR_CUDA, std::string(fn) + ": an mbarrier wait ran out (stage " + std::to_string(werr - 1) + ")");
     return RF_OK;
@@ -86,7 +85,7 @@ extern "C" int rf_conv3x3_bf16(const void* xa, uint32_t ca, int up, const void* 
         a.bias = bias;
         a.relu = relu;
         const ConvEpilogue epi = mode == RF_GEMM_STORE_F32 ? kConvStoreF32 : mode == RF_GEMM_ATOMIC_F32 ? kConvAtomicF32 : kConvStoreBF16;
-        return finish("rf_conv3x3_bf16", launch_conv(a, epi, st), st, conv_error);
+        return finish("rf_conv3x3_bf16", launch_conv(a, epi, st), st);
     }
     GemmArgs g{};
     g.xa = static_cast<const __nv_bfloat16*>(xa);

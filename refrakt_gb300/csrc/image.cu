@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "scratch.h"
 
 namespace rfk {
 
@@ -30,6 +31,12 @@ struct DeTables {
     int R, min_r, mode;  // mode 0: curve > 0, 1: curve < 0, 2: curve == 0 (radius R)
     int wbase[102];      // offset of radius r's (r+1)^2 weights
     double wsum[101];    // the weights of a whole disc of radius r, summed in FP64
+};
+
+// the weights of radii up to kDeMaxSmemR, a kernel parameter: no upload per call
+constexpr int kSmemWeights = (kDeMaxSmemR + 1) * (kDeMaxSmemR + 2) * (2 * kDeMaxSmemR + 3) / 6;
+struct DeWeights {
+    float w[kSmemWeights];
 };
 
 __device__ __forceinline__ int de_radius(float a, const DeTables& T) {
@@ -78,8 +85,8 @@ __device__ __forceinline__ void block_sum_to(double s, double* out) {
 // for every radius up to kDeMaxSmemR (the fused path's radii).
 constexpr int kRowPrefixFloats = 1638;  // sum over r <= 12 of (r + 1) rows of 2r + 2 prefix sums
 
-__global__ void de_radius_sum_kernel(const float4* __restrict__ in, uint32_t w, uint32_t h, const DeTables T,
-                                     const float* __restrict__ weights, uint8_t* __restrict__ rad,
+__global__ void de_radius_sum_kernel(const float4* __restrict__ in, uint32_t w, uint32_t h, const __grid_constant__ DeTables T,
+                                     const __grid_constant__ DeWeights W, uint8_t* __restrict__ rad,
                                      double* __restrict__ sum_out) {
     __shared__ float s_pre[kRowPrefixFloats];
     __shared__ int s_pbase[kDeMaxSmemR + 1];
@@ -101,7 +108,7 @@ __global__ void de_radius_sum_kernel(const float4* __restrict__ in, uint32_t w, 
         pre[0] = 0.0f;
         for (int dx = -r; dx <= r; dx++) {
             const int ax = dx < 0 ? -dx : dx;
-            if (4 * (ax * ax + ay * ay) <= (2 * r + 1) * (2 * r + 1)) acc += weights[T.wbase[r] + ay * (r + 1) + ax];
+            if (4 * (ax * ax + ay * ay) <= (2 * r + 1) * (2 * r + 1)) acc += W.w[T.wbase[r] + ay * (r + 1) + ax];
             pre[dx + r + 1] = acc;
         }
     }
@@ -816,15 +823,15 @@ cudaError_t launch_density(const float4* in, uint32_t w, uint32_t h, int R, int 
                            cudaStream_t st) {
     DeTables T;
     std::vector<float> wts;
-    const bool sweep = std::max(R, min_r) <= kDeMaxSweepR;  // else the gather, which reads the weight table
+    const bool sweep = !density_reads_weights(R, min_r);
     if (sweep) de_thresholds(R, min_r, curve, T);
     else de_tables(R, min_r, curve, T, wts);
     uint8_t* rad = nullptr;
     float* dw = nullptr;
-    cudaError_t e = cudaMallocAsync(&rad, (size_t)w * h, st);
+    cudaError_t e = scratch_alloc(&rad, (size_t)w * h, st);
     if (e != cudaSuccess) return e;
     if (!sweep) {
-        e = cudaMallocAsync(&dw, wts.size() * sizeof(float), st);
+        e = scratch_alloc(&dw, wts.size(), st);
         if (e != cudaSuccess) { cudaFreeAsync(rad, st); return e; }
         cudaMemcpyAsync(dw, wts.data(), wts.size() * sizeof(float), cudaMemcpyHostToDevice, st);
     }
@@ -833,6 +840,8 @@ cudaError_t launch_density(const float4* in, uint32_t w, uint32_t h, int R, int 
     if (dw) cudaFreeAsync(dw, st);
     return e;
 }
+
+bool density_reads_weights(int R, int min_r) { return std::max(R, min_r) > kDeMaxSweepR; }
 
 size_t density_weight_count(int R, int min_r) {
     const int rmax = R > min_r ? R : min_r;
@@ -862,18 +871,19 @@ bool density_tonemap_fused(int R, int min_r, uint32_t ss) {
 // in shared memory and tonemaps it there, so the estimator's FP32 output never reaches DRAM.
 // Where that does not apply (density_tonemap_fused false: ss does not divide the tile, or radii
 // beyond the shared-memory path) the estimator writes `de_scratch`, then the statistics and
-// tonemap passes run on it.  rad: a byte per bin; dw: the weight table (density_weights);
-// stats: 3 doubles.
+// tonemap passes run on it.  rad: a byte per bin; dw: the weight table (density_weights) where
+// density_reads_weights, else unused; stats: 3 doubles.
 cudaError_t launch_density_tonemap(const float4* in, uint32_t w, uint32_t h, int R, int min_r, float curve,
                                    uint32_t ss, float gamma, float brightness, float vibrancy, float k2,
                                    float4* out_f32, uchar4* out8, uint8_t* rad, const float* dw, double* stats,
                                    float4* de_scratch, cudaStream_t st) {
     DeTables T;
     std::vector<float> wts;
-    de_tables(R, min_r, curve, T, wts);
-    const bool need_sum = !(k2 > 0.0f);
+    const bool need_sum = !(k2 > 0.0f), fused = density_tonemap_fused(R, min_r, ss);
+    if ((fused && need_sum) || density_reads_weights(R, min_r)) de_tables(R, min_r, curve, T, wts);
+    else de_thresholds(R, min_r, curve, T);
     cudaError_t e;
-    if (!density_tonemap_fused(R, min_r, ss)) {
+    if (!fused) {
         if (!de_scratch) return cudaErrorInvalidValue;
         e = launch_density_passes(in, w, h, T, de_scratch, rad, dw, st);
         if (e == cudaSuccess && need_sum) e = launch_stats(de_scratch, w, h, stats, st);
@@ -885,7 +895,9 @@ cudaError_t launch_density_tonemap(const float4* in, uint32_t w, uint32_t h, int
     if (need_sum) {
         e = cudaMemsetAsync(stats, 0, 3 * sizeof(double), st);
         if (e != cudaSuccess) return e;
-        de_radius_sum_kernel<<<1024, 256, 0, st>>>(in, w, h, T, dw, rad, stats);
+        DeWeights W;
+        std::copy(wts.begin(), wts.end(), W.w);  // at most kSmemWeights of them
+        de_radius_sum_kernel<<<1024, 256, 0, st>>>(in, w, h, T, W, rad, stats);
     } else {
         de_radius_kernel<<<1024, 256, 0, st>>>(in, (size_t)w * h, T, rad);
     }
@@ -902,7 +914,8 @@ cudaError_t launch_density_resident(const float4* in, uint32_t w, uint32_t h, in
                                     float4* out, uint8_t* rad, const float* dw, cudaStream_t st) {
     DeTables T;
     std::vector<float> wts;
-    de_tables(R, min_r, curve, T, wts);
+    if (density_reads_weights(R, min_r)) de_tables(R, min_r, curve, T, wts);
+    else de_thresholds(R, min_r, curve, T);
     return launch_density_passes(in, w, h, T, out, rad, dw, st);
 }
 

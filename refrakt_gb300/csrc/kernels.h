@@ -35,6 +35,8 @@ cudaError_t launch_probe(const uint32_t* prog, int xform, uint32_t n, const floa
 cudaError_t launch_density(const float4* in, uint32_t w, uint32_t h, int radius, int min_radius, float curve,
                            float4* out, cudaStream_t st);
 size_t density_weight_count(int radius, int min_radius);
+// radii whose estimator reads the weight table (the others compute their weights)
+bool density_reads_weights(int radius, int min_radius);
 // Kernel weights of density estimation depend on the radii alone: `density_weights` builds them on
 // the host, and `launch_density_resident` runs both passes with those weights already on the
 // device (`dw`) and a byte of radius scratch per bin (`rad`) — no allocation and no host copy,
@@ -59,7 +61,8 @@ cudaError_t launch_tonemap_filter(const float4* in, uint32_t w, uint32_t h, uint
                                   float4* out_f32, uchar4* out8, cudaStream_t st);
 // Density estimation and tonemap in one sequence (image.cu): with density_tonemap_fused the
 // estimator's output stays on chip and `de_scratch` is not touched (may be null); otherwise it is
-// the estimator's output.  rad: a byte per bin; dw: density_weights(R, min_r); stats: 3 doubles.
+// the estimator's output.  rad: a byte per bin; dw: density_weights(R, min_r) where
+// density_reads_weights, else it may be null; stats: 3 doubles.
 bool density_tonemap_fused(int radius, int min_radius, uint32_t ss);
 cudaError_t launch_density_tonemap(const float4* in, uint32_t w, uint32_t h, int radius, int min_radius, float curve,
                                    uint32_t ss, float gamma, float brightness, float vibrancy, float k2,

@@ -91,6 +91,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
     return false;
 }
 
+// reports a wait that ran out to the host (error_word, gemm.h): nonzero codes
+__device__ __forceinline__ void report_error(int* word, int code) { *reinterpret_cast<volatile int*>(word) = code; }
+
 // ---- async-proxy fences ----------------------------------------------------------------------
 // makes this thread's generic-proxy writes to shared memory visible to the tensor cores
 __device__ __forceinline__ void fence_proxy_async_smem() {
