@@ -1,9 +1,8 @@
 // The chaos game of one CTA (the body of chaos_kernel, kernels.cu, and of the genome-specialised
 // kernels compiled at run time, specialize.cpp), parameterised by the xform evaluator:
-// `Eval::apply(prog, xi, final_offset, x, y, c, op, first_run, rng)` applies regular xform xi,
-// or the final xform for xi = -1.  InterpEval interprets the compiled genome program
-// (variations.cuh); a specialised evaluator is generated per genome structure.  The kernel calls
-// apply from one site for both (a two-iteration loop), so the evaluator is inlined once.
+// `Eval::apply<FINAL>(prog, word, x, y, c, op, first_run, rng)` applies the xform of an xform_word.
+// InterpEval interprets the compiled genome program (variations.cuh); a specialised evaluator is
+// generated per genome structure (specialize.cpp).
 //
 // The reference runs one GLSL invocation per walker per pass and ping-pongs every walker
 // through memory between passes (shaders/flame.glsl:41-90, src/flame.cpp:228-330).  Here one
@@ -25,12 +24,31 @@
 
 namespace rfk {
 
+// A group's drawn xform as the slots read it: id | (its block's word offset) << 8.
+__device__ __forceinline__ uint32_t xform_word(const uint32_t* prog, int xi) {
+    return (uint32_t)xi | (prog[H_XOFF + xi] << 8);
+}
+
 struct InterpEval {
-    static __device__ __forceinline__ void apply(const uint32_t* prog, int xi, uint32_t final_off, float& x, float& y,
-                                                 float& c, float& op, bool first_run, Jsf& rng) {
-        eval_xform(prog + (xi >= 0 ? prog[H_XOFF + xi] : final_off), x, y, c, op, first_run, rng);
+    static constexpr bool kFinal = true;
+    template <bool FINAL>
+    static __device__ __forceinline__ void apply(const uint32_t* prog, uint32_t word, float& x, float& y, float& c,
+                                                 float& op, bool first_run, Jsf& rng) {
+        const uint32_t blk = (uint32_t)__cvta_generic_to_shared(prog) + 4u * (word >> 8);
+        const XformOut o = eval_xform(blk, x, y, c, first_run, rng);
+        x = o.x; y = o.y; c = o.c; op = o.op;
+        rng = o.rng;
     }
 };
+
+// The final xform on a drawn copy of the walker; op becomes the point's opacity.
+template <class Eval>
+__device__ __forceinline__ void final_xform(const uint32_t* prog, uint32_t final_off, float& x, float& y, float& c,
+                                            float& op, Jsf& rng) {
+    float o;
+    Eval::template apply<true>(prog, final_off << 8, x, y, c, o, false, rng);
+    op = o * op;
+}
 
 // The slot a thread serves in phase k of a pass: phase k covers slots [k * THREADS, (k + 1) *
 // THREADS), and warps are permuted per phase (warp w serves warp w ^ k's 32 slots), so the 256-slot
@@ -145,7 +163,7 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
     float4* s_pal = reinterpret_cast<float4*>(smem + (((size_t)A.prog_words * 4 + 15) & ~(size_t)15));
     float4* s_w = s_pal + 256;
     uint4* s_rng = reinterpret_cast<uint4*>(s_w + 2 * SLOTS);
-    int* s_xid = reinterpret_cast<int*>(s_rng + SLOTS);
+    uint32_t* s_xid = reinterpret_cast<uint32_t*>(s_rng + SLOTS);
     uint32_t* s_perm = reinterpret_cast<uint32_t*>(s_xid + 2 * G);
     uint64_t* s_bar = reinterpret_cast<uint64_t*>(((unsigned long long)(s_perm + A.steps) + 7) & ~7ull);
     // the tile splat's shared-memory histogram (splat 3)
@@ -209,7 +227,7 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
     // from its own RNG stream (the pipelined and cluster exchanges draw inside the pass loop instead)
     auto draw_group_xform = [&](uint32_t s, uint32_t ls, Jsf& rng) {
         const int xi = select_xform(s_prog, randf(rng));
-        s_xid[(s & 1) * G + ls / kGroup] = xi;
+        s_xid[(s & 1) * G + ls / kGroup] = xform_word(s_prog, xi);
         if (A.trace && A.pass0 + s < A.trace_passes)
             A.trace[(size_t)(A.pass0 + s) * A.n_groups + (ts_base + gid0 + ls) / kGroup] = (uint8_t)xi;
     };
@@ -273,7 +291,7 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
             float x = v.x, y = v.y, c = v.z;
             const uint4 r4 = s_rng[ls];
             Jsf rng{r4.x, r4.y, r4.z, r4.w};
-            const int xi = s_xid[buf * G + ls / kGroup];
+            const uint32_t xw = s_xid[buf * G + ls / kGroup];
             const bool first = A.first_run && s == 0;
             if (first) {  // flame.glsl:64: xy += randf() * .1 * PI * 2.0 * sincos(sqrt(randf()))
                 const float u1 = randf(rng);
@@ -284,22 +302,12 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
                 x = __fadd_rn(x, __fmul_rn(amp, sn));
                 y = __fadd_rn(y, __fmul_rn(amp, cs));
             }
-            // the xform, then (when drawing) the final xform on a copy — one evaluator call site
-            float ex = x, ey = y, ec = c, op = 0.0f;
-            bool fr = first;
-            for (int it = 0;; it++) {
-                float o;
-                Eval::apply(s_prog, it == 0 ? xi : -1, foff, ex, ey, ec, o, fr, rng);
-                if (it == 0) {
-                    if (reset) reset_bad_walker(ex, ey, o, rng);  // flame.glsl:68, before pos_out
-                    x = ex; y = ey; c = ec; op = o;
-                } else {
-                    op = o * op;
-                }
-                if (it == 1 || !has_final) break;
-                fr = false;
-            }
+            // the xform: the walker's next state; then (when drawing) the final xform on the copy that is drawn
+            float op = 0.0f;
+            Eval::template apply<false>(s_prog, xw, x, y, c, op, first, rng);
+            if (reset) reset_bad_walker(x, y, op, rng);  // flame.glsl:68, before pos_out
             s_w[(buf ^ 1) * SLOTS + ls] = make_float4(x, y, c, 0.0f);
+            if (Eval::kFinal && has_final) final_xform<Eval>(s_prog, foff, x, y, c, op, rng);
             // the group's xform for the next pass, at the point of the slot's stream where the
             // pass-barrier form draws it
             if ((PIPE || CLUSTER > 1) && k == dphase && s + 1 < A.steps) draw_group_xform(s + 1, ls, rng);
@@ -308,8 +316,8 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
             if (CLUSTER > 1 && k == SPT - 1) cluster_arrive();
             if (A.draw) {
                 if (op > 0.0f) emitted++;
-                const float px = fmaf(A.ss[0], ex, fmaf(A.ss[2], ey, A.ss[4]));
-                const float py = fmaf(A.ss[1], ex, fmaf(A.ss[3], ey, A.ss[5]));
+                const float px = fmaf(A.ss[0], x, fmaf(A.ss[2], y, A.ss[4]));
+                const float py = fmaf(A.ss[1], x, fmaf(A.ss[3], y, A.ss[5]));
                 uint32_t bin = kNoBin, local = kNoBin;
                 float4 val = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 if (px >= 0.0f && py >= 0.0f && px < W && py < H && op > 0.0f) {
@@ -318,7 +326,7 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
                     bin = row * A.W + bx;
                     if (tile_bins && bx - A.tile_x0 < A.tile_w && row - A.tile_y0 < A.tile_h)
                         local = (row - A.tile_y0) * A.tile_w + (bx - A.tile_x0);
-                    const float4 col = s_pal[palette_index(ec)];
+                    const float4 col = s_pal[palette_index(c)];
                     val = make_float4(col.x, col.y, col.z, op);
                     drawn++;
                 }

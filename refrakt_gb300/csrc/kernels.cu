@@ -135,14 +135,17 @@ __global__ void animate_kernel(const uint32_t* base, uint32_t words, uint32_t T,
 // single dispatch() per point, for parity tests
 __global__ void probe_kernel(const uint32_t* prog, int xform, uint32_t n, const float* in, uint32_t* rng,
                              int first_run, float* out) {
+    __shared__ uint32_t s_prog[kProgMaxWords];
+    for (uint32_t k = threadIdx.x; k < prog[H_WORDS]; k += blockDim.x) s_prog[k] = prog[k];
+    __syncthreads();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const uint32_t off = (xform < 0) ? prog[H_FINAL] : prog[H_XOFF + xform];
+    const uint32_t off = (xform < 0) ? s_prog[H_FINAL] : s_prog[H_XOFF + xform];
     Jsf s{rng[4 * i], rng[4 * i + 1], rng[4 * i + 2], rng[4 * i + 3]};
-    float x = in[3 * i], y = in[3 * i + 1], c = in[3 * i + 2], op;
-    eval_xform(prog + off, x, y, c, op, first_run != 0, s);
-    out[4 * i] = x; out[4 * i + 1] = y; out[4 * i + 2] = c; out[4 * i + 3] = op;
-    rng[4 * i] = s.a; rng[4 * i + 1] = s.b; rng[4 * i + 2] = s.c; rng[4 * i + 3] = s.d;
+    const XformOut o = eval_xform((uint32_t)__cvta_generic_to_shared(s_prog + off), in[3 * i], in[3 * i + 1],
+                                  in[3 * i + 2], first_run != 0, s);
+    out[4 * i] = o.x; out[4 * i + 1] = o.y; out[4 * i + 2] = o.c; out[4 * i + 3] = o.op;
+    rng[4 * i] = o.rng.a; rng[4 * i + 1] = o.rng.b; rng[4 * i + 2] = o.rng.c; rng[4 * i + 3] = o.rng.d;
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -39,12 +39,12 @@ struct BinTarget {
     __device__ __forceinline__ uint32_t* at_count(uint32_t bin) const { return count + ((size_t)bin << cs); }
 };
 
+// (no kernel that splats reads the bins, so neither is a barrier to the compiler's other accesses)
 __device__ __forceinline__ void red_add_f32x4(float4* p, float a, float b, float c, float d) {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d)
-                 : "memory");
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d));
 }
 __device__ __forceinline__ void red_add_u32x1(uint32_t* p, uint32_t v) {
-    asm volatile("red.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+    asm volatile("red.global.add.u32 [%0], %1;" ::"l"(p), "r"(v));
 }
 
 __device__ __forceinline__ void splat_global(const BinTarget& t, uint32_t bin, float4 v) {

@@ -72,23 +72,26 @@ __device__ __forceinline__ void precalc(Pre& p, float x, float y, uint32_t m) {
 
 __device__ __forceinline__ float mod2f(float x, float y) { return x - y * truncf(x / y); }  // math.glsl:13
 
-struct VaryOut {  // a variation's value and the slot's RNG state after it
-    float x, y;
-    Jsf rng;
+// words of a genome program in shared memory, by 32-bit address
+struct SharedWords {
+    uint32_t a;
+    __device__ __forceinline__ float operator[](int i) const {
+        float v;
+        asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a + 4u * i));
+        return v;
+    }
+    __device__ __forceinline__ uint32_t u(int i) const {
+        uint32_t v;
+        asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a + 4u * i));
+        return v;
+    }
+    __device__ __forceinline__ SharedWords operator+(uint32_t n) const { return SharedWords{a + 4u * n}; }
 };
 
-#ifndef RFK_VARY_INLINE
-#define RFK_VARY_ATTR static __device__ __noinline__
-#else
-#define RFK_VARY_ATTR static __device__ __forceinline__
-#endif
-
-// Unweighted value of variation `id` (radial_blur applies its weight internally).  Kept out of
-// line: the 68 cases inlined into the chaos loop need ~120 registers and spill heavily at 64;
-// as a call, the loop stays within 64 registers and only the case taken pays for its own.
-// Everything passes by value so nothing is materialised on the stack.
-__device__ __forceinline__ float2 vary_impl(uint32_t id, const Pre p, float w, const float* __restrict__ aff,
-                                            const float* __restrict__ P, Jsf& rng) {
+// Unweighted value of variation `id` (radial_blur applies its weight internally); Words: the program
+// block's floats (const float* or SharedWords).
+template <class Words>
+__device__ __forceinline__ float2 vary_impl(uint32_t id, const Pre p, float w, const Words aff, const Words P, Jsf& rng) {
     const float x = p.x, y = p.y, r = p.r, rsq = p.rsq, a = p.a, phi = p.phi;
     float s, c;
     switch (id) {
@@ -271,54 +274,52 @@ __device__ __forceinline__ float2 vary_impl(uint32_t id, const Pre p, float w, c
     return make_float2(__int_as_float(0x7fffffff), __int_as_float(0x7fffffff));
 }
 
-RFK_VARY_ATTR VaryOut vary_call(uint32_t id, const Pre p, float w, const float* __restrict__ aff,
-                                const float* __restrict__ P, Jsf rng) {
-    const float2 v = vary_impl(id, p, w, aff, P, rng);
-    return VaryOut{v.x, v.y, rng};
-}
+struct XformOut {  // a walker's state after an xform, the xform's opacity and the slot's RNG state
+    float x, y, c, op;
+    Jsf rng;
+};
 
-__device__ __forceinline__ float2 vary(uint32_t id, const Pre& p, float w, const float* __restrict__ aff,
-                                       const float* __restrict__ P, Jsf& rng) {
-    const VaryOut o = vary_call(id, p, w, aff, P, rng);
-    rng = o.rng;
-    return make_float2(o.x, o.y);
-}
-
-// dispatch() of one xform block: src/variation_table.cpp:97-165 (affine prelude, pre_xform
-// terms, precalcs, weighted terms in map order, post) and :241-243 (colour, opacity).
-__device__ __forceinline__ void eval_xform(const uint32_t* __restrict__ blk, float& x, float& y, float& c,
-                                           float& op, bool first_run, Jsf& rng) {
-    const float* fb = reinterpret_cast<const float*>(blk);
+// The interpreter: dispatch() of the xform block at shared-memory address `blk`: src/variation_table.cpp:97-165
+// (affine prelude, pre_xform terms, precalcs, weighted terms in map order, post) and :241-243 (colour,
+// opacity).  Out of line, with the 68 cases inlined at one site: the cases in the chaos loop itself spill
+// heavily at its 64 registers, and a call per term instead moves some 25 registers for each (interpreted, 39.8 M
+// points: the 1080p genome 1824 -> 1454 us, a 5-xform one 1392 -> 1242 us).  Everything passes by value so
+// nothing is materialised on the stack.
+static __device__ __noinline__ XformOut eval_xform(uint32_t blk, float x, float y, float c, bool first_run, Jsf rng) {
+    const SharedWords fb{blk};
     float vx = fmaf(fb[X_AFF + 0], x, fmaf(fb[X_AFF + 2], y, fb[X_AFF + 4]));
     float vy = fmaf(fb[X_AFF + 1], x, fmaf(fb[X_AFF + 3], y, fb[X_AFF + 5]));
-    const uint32_t npre = blk[X_NPRE], nterm = blk[X_NTERM];
-    const uint32_t* e = blk + X_TERMS;
-    Pre pc;
-    for (uint32_t k = 0; k < npre; k++, e += 3) {
-        pc.x = vx; pc.y = vy;
-        const float wt = __uint_as_float(e[1]);
-        const float2 d = vary(e[0] & 0xffu, pc, wt, fb + X_AFF, fb + e[2], rng);
-        vx = __fadd_rn(vx, __fmul_rn(wt, d.x));
-        vy = __fadd_rn(vy, __fmul_rn(wt, d.y));
-    }
-    precalc(pc, vx, vy, blk[X_MASK]);
+    const uint32_t npre = fb.u(X_NPRE), n = npre + fb.u(X_NTERM);
+    SharedWords e = fb + X_TERMS;
+    Pre pc{};
     float rx = 0.0f, ry = 0.0f;
-    for (uint32_t k = 0; k < nterm; k++, e += 3) {
-        const float wt = __uint_as_float(e[1]);
-        float2 d = vary(e[0] & 0xffu, pc, wt, fb + X_AFF, fb + e[2], rng);
-        if (!(e[0] & kTermNoWeightMul)) { d.x = __fmul_rn(wt, d.x); d.y = __fmul_rn(wt, d.y); }
-        if (k == 0) { rx = d.x; ry = d.y; }
+    for (uint32_t k = 0; k < n; k++, e = e + 3) {
+        if (k < npre) {
+            pc.x = vx;
+            pc.y = vy;
+        } else if (k == npre) {
+            precalc(pc, vx, vy, fb.u(X_MASK));
+        }
+        const uint32_t id = e.u(0);
+        const float wt = e[1];
+        float2 d = vary_impl(id & 0xffu, pc, wt, fb + X_AFF, fb + e.u(2), rng);
+        if (k < npre) {
+            vx = __fadd_rn(vx, __fmul_rn(wt, d.x));
+            vy = __fadd_rn(vy, __fmul_rn(wt, d.y));
+            continue;
+        }
+        if (!(id & kTermNoWeightMul)) { d.x = __fmul_rn(wt, d.x); d.y = __fmul_rn(wt, d.y); }
+        if (k == npre) { rx = d.x; ry = d.y; }
         else { rx = __fadd_rn(rx, d.x); ry = __fadd_rn(ry, d.y); }
     }
-    if (blk[X_HASPOST]) {
+    if (fb.u(X_HASPOST)) {
         const float px = fmaf(fb[X_POST + 0], rx, fmaf(fb[X_POST + 2], ry, fb[X_POST + 4]));
         const float py = fmaf(fb[X_POST + 1], rx, fmaf(fb[X_POST + 3], ry, fb[X_POST + 5]));
         rx = px; ry = py;
     }
     const float cin = first_run ? randf(rng) : c;
     c = __fadd_rn(__fmul_rn(cin, fb[X_OMCS]), __fmul_rn(fb[X_COLOR], fb[X_CS]));
-    x = rx; y = ry;
-    op = fb[X_OPACITY];
+    return XformOut{rx, ry, c, fb[X_OPACITY], rng};
 }
 
 }  // namespace rfk
