@@ -55,6 +55,9 @@ int splat_code(int splat) {
 
 namespace {
 
+constexpr size_t kListBytes = 16ull << 30;  // the lists' memory at most: 256 passes of 2.5 M walkers at three times an even spread
+constexpr uint64_t kListHot = 1024;
+constexpr size_t kListScratch = (size_t)kRangeBins * 72 + kMaxRanges * 4;  // two sets of scratch planes, flags
 constexpr size_t kInterleaveMinBytes = 256ull << 20;  // bins + counts above ~2x L2: interleave
 
 int set_device(const rf_sim* s) {
@@ -239,7 +242,8 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
         a.first_run = (first_run && done == 0) ? 1 : 0;
         a.draw = draw ? 1 : 0;
         // RF_SPLAT_AUTO's tile: settle a pending decision, then see whether this launch is timed
-        const bool tile_grid = draw && s->splat == RF_SPLAT_AUTO && s->rgba_shift == 0 && hits &&
+        const bool planes = s->rgba_shift == 0 && s->list_ranges == 0;
+        const bool tile_grid = draw && s->splat == RF_SPLAT_AUTO && planes && hits &&
                                (uint64_t)W * H <= kAutoTileMaxBins && s->tile_ev[0] && !capturing(s->stream);
         if (tile_grid && (s->auto_tile_wh[0] != W || s->auto_tile_wh[1] != H)) {
             s->auto_tile_state = 0;  // a new grid
@@ -251,9 +255,9 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
         const bool tile_warmup = tile_grid && steps >= 32 && s->auto_tile_state == 0;  // not timed: the grid's first
         if (tile_grid && steps >= 32 && s->auto_tile_state == 2) tile_timed = 0;
         if (tile_grid && steps == s->auto_tile_passes && s->auto_tile_state == 3) tile_timed = 1;
-        const bool auto_tile = draw && s->splat == RF_SPLAT_AUTO && s->rgba_shift == 0 && s->auto_tile_wh[0] == W &&
+        const bool auto_tile = draw && s->splat == RF_SPLAT_AUTO && planes && s->auto_tile_wh[0] == W &&
                                s->auto_tile_wh[1] == H && (s->auto_tile_state == 1 || tile_timed == 1);
-        a.splat = auto_tile ? 3 : splat_code(s->splat);
+        a.splat = auto_tile ? 3 : s->list_ranges ? 4 : splat_code(s->splat);
         a.reset = s->reset;
         a.rgba_shift = s->rgba_shift;
         a.count_shift = s->count_shift;
@@ -273,11 +277,17 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
         a.trace_passes = s->trace_passes;
         a.n_groups = (uint32_t)(s->N / kGroup);
         const uint32_t tile_bins = a.splat == 3 && a.draw ? a.tile_w * a.tile_h : 0u;
+        if (s->list_ranges) {
+            a.ranges = s->list_ranges;
+            a.list_cap = s->list_cap;
+            a.list_n = reinterpret_cast<uint32_t*>(s->lists + kListScratch);
+            a.list = reinterpret_cast<uint2*>(a.list_n + (((s->N / s->slots) * a.ranges + 3) & ~(size_t)3));
+        }
         int measure = -1;
         // (RF_SPLAT_AUTO's tile is timed first, in the pipelined form; the exchange after it)
         const bool tile_busy = tile_warmup || tile_timed >= 0 || (s->splat == RF_SPLAT_AUTO && s->auto_tile_state >= 2);
         const bool timed = s->spec && cluster_for_launch(s, false) == 1;  // else the cluster form, untimed
-        const int want = timed ? exchange_for_launch(s, a.draw, steps, !tile_busy, &measure) : 0;
+        const int want = timed ? exchange_for_launch(s, a.draw, steps, !tile_busy && !a.ranges, &measure) : 0;
         const int pipe = want && s->spec && use_pipe(s, tile_bins) ? 1 : 0;
         // one CTA per mixing domain, or a cluster of `cl`
         const int cl = cluster_for_launch(s, !want);
@@ -302,12 +312,22 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
         if (measure >= 0 && cudaEventRecord(s->tune_ev[2 * measure], s->stream) != cudaSuccess) measure = -1;
         if (tile_timed >= 0 && cudaEventRecord(s->tile_ev[2 * tile_timed], s->stream) != cudaSuccess) tile_timed = -1;
         cudaError_t e = s->spec ? launch_spec(s->spec, (int)threads, (int)local, a, grid,
-                                              chaos_smem(local, a.prog_words, a.steps, tile_bins, pipe), s->stream)
+                                              chaos_smem(local, a.prog_words, a.steps, tile_bins, pipe, a.ranges), s->stream)
                                 : launch_chaos((int)s->threads, (int)s->slots, a, grid, s->stream);
         if (e != cudaSuccess) return cuda_fail(e, "chaos kernel launch");
         if (measure >= 0 && cudaEventRecord(s->tune_ev[2 * measure + 1], s->stream) == cudaSuccess)
             s->tune_step = measure + 1;
         const bool tile_recorded = tile_timed >= 0 && cudaEventRecord(s->tile_ev[2 * tile_timed + 1], s->stream) == cudaSuccess;
+        if (a.ranges) {
+            RangeScratch set[2];
+            for (int k = 0; k < 2; k++) {
+                set[k].rgba = reinterpret_cast<float4*>(s->lists) + (size_t)(2 * k) * kRangeBins;
+                set[k].rgba2 = set[k].rgba + kRangeBins;
+                set[k].count = reinterpret_cast<uint32_t*>(s->lists + (size_t)kRangeBins * 64) + (size_t)k * kRangeBins;
+            }
+            RF_CUDA(launch_ranges(a, grid, set, reinterpret_cast<uint32_t*>(s->lists + kListScratch) - kMaxRanges,
+                                  s->counters + 6, s->stream));
+        }
         s->cur ^= 1;
         s->pass += steps;
         done += steps;
@@ -326,6 +346,66 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
     return RF_OK;
 }
 
+// Point lists (splat 4) for the drawing launches of a call on a grid far above L2, instead of interleaved
+// records: 80 M points of the space-filling genome on 8192 x 8192 bins 3.98 -> 1.87 ms (637 M 24.9 -> 15.7), of
+// the 1080p genome 3.50 -> 2.46.  Not for hot bins, whose points the lists' second step adds one after another while the
+// records' reductions pass under the chaos game (62 M points of the 5-xform genome on 5000 x 4001 bins, 0.3 % of
+// them in one bin: 1.63 ms with records, 1.80 with lists): the first call measures, later ones take records
+// above a share of 1 / kListHot in one bin or where an eighth of the points found their list full.
+bool lists_suit(const rf_sim* s, uint32_t W, uint32_t H) {
+    if (!s->list_asked || s->list_wh[0] != W || s->list_wh[1] != H) return true;
+    const volatile unsigned long long* h = s->list_stats;
+    return h[0] * kListHot < h[1] + (h[1] == 0) && h[2] * 8 <= s->list_points;
+}
+
+// asks for it once per genome and grid (an option: nothing fails for it)
+void measure_lists(rf_sim* s, const uint32_t* hits, uint32_t W, uint32_t H, uint64_t points) {
+    if (s->list_asked && s->list_wh[0] == W && s->list_wh[1] == H) return;
+    if (!s->list_stats && cudaHostAlloc((void**)&s->list_stats, 24, cudaHostAllocDefault) != cudaSuccess) s->list_stats = nullptr;
+    s->list_asked = false;
+    if (s->list_stats) {
+        for (int k = 0; k < 3; k++) s->list_stats[k] = 0;
+        unsigned long long* out = s->counters + 4;
+        s->list_asked = cudaMemsetAsync(out, 0, 16, s->stream) == cudaSuccess &&
+                        launch_hottest_bin(hits, (size_t)W * H, out, s->stream) == cudaSuccess &&
+                        cudaMemcpyAsync(s->list_stats, out, 24, cudaMemcpyDeviceToHost, s->stream) == cudaSuccess;
+        s->list_points = points;
+        s->list_wh[0] = W;
+        s->list_wh[1] = H;
+    }
+    if (!s->list_asked) cudaGetLastError();
+}
+
+// the lists' memory for a call of `passes` passes, four times an even spread over the ranges where it fits, at
+// least 1.25 times; false: it does not, or the sim's domains are spread over clusters
+bool reserve_lists(rf_sim* s, size_t nb, uint32_t passes) {
+    const uint32_t ranges = (uint32_t)((nb + kRangeBins - 1) >> kRangeBits);
+    // (a captured call takes records: a later call may move the lists)
+    if (s->splat != RF_SPLAT_AUTO || ranges > kMaxRanges || (s->spec && cluster_for_launch(s, true) > 1) || capturing(s->stream))
+        return false;
+    const uint64_t ctas = s->N / s->slots, points = (uint64_t)s->slots * std::min(passes, s->L);  // of a CTA
+    const size_t head = kListScratch + ((ctas * ranges + 3) & ~(uint64_t)3) * 4;
+    if (head >= kListBytes) return false;
+    const uint64_t fit = (kListBytes - head) / (ctas * ranges * 8);
+    const uint64_t cap = std::min<uint64_t>({points, std::max<uint64_t>(4 * points / ranges, 256), fit});
+    if (4 * cap * ranges < 5 * points || chaos_smem(s->slots, s->prog_words, s->L, 0, 1, ranges) > kMaxCtaSmem) return false;
+    const size_t bytes = head + ctas * ranges * cap * 8;
+    if (s->lists_bytes < bytes) {
+        cudaFree(s->lists);
+        s->lists = nullptr;
+        s->lists_bytes = 0;
+        if (cudaMalloc((void**)&s->lists, bytes) != cudaSuccess ||
+            cudaMemsetAsync(s->lists, 0, kListScratch, s->stream) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        s->lists_bytes = bytes;
+    }
+    s->list_ranges = ranges;
+    s->list_cap = (uint32_t)cap;
+    return true;
+}
+
 // The drawing passes into the caller's planes, or — for histograms well above L2 with a count
 // plane — into interleaved 32-byte records (RGBA and count in one DRAM sector) merged into the
 // caller's planes afterwards.
@@ -334,6 +414,13 @@ int draw_passes(rf_sim* s, uint32_t passes, float4* bins, uint32_t* hits, uint32
     bool il = s->bin_layout == RF_BINS_INTERLEAVED;
     if (s->bin_layout == RF_BINS_AUTO) il = hits != nullptr && nb * 20 > kInterleaveMinBytes;
     if (!il) return launch_passes(s, passes, false, true, bins, hits, W, H, ss);
+    if (s->bin_layout == RF_BINS_AUTO && lists_suit(s, W, H) && reserve_lists(s, nb, passes)) {
+        RF_CUDA(cudaMemsetAsync(s->counters + 6, 0, sizeof(unsigned long long), s->stream));
+        const int rc = launch_passes(s, passes, false, true, bins, hits, W, H, ss);
+        s->list_ranges = 0;
+        if (!rc) measure_lists(s, hits, W, H, (uint64_t)s->N * passes);
+        return rc;
+    }
     if (s->rec_n < nb) {
         cudaFree(s->rec);
         s->rec = nullptr;
@@ -683,7 +770,8 @@ int rf_sim_destroy(rf_sim* s) {
     if (!s) return RF_OK;
     cudaSetDevice(s->device);
     cudaStreamSynchronize(s->stream);
-    void* ptrs[] = {s->rec, s->walk[0], s->walk[1], s->rng, s->table, s->base_prog, s->progs, s->palette, s->counters,
+    if (s->list_stats) cudaFreeHost(s->list_stats);
+    void* ptrs[] = {s->rec, s->lists, s->walk[0], s->walk[1], s->rng, s->table, s->base_prog, s->progs, s->palette, s->counters,
                     s->trace, s->r_bins, s->r_hits, s->r_de, s->r_img, s->r_stats, s->r_rad, s->r_dw};
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -740,6 +828,7 @@ int rf_warmup(rf_sim* s, rf_flame* f, uint32_t num_passes, float tss_width) {
     if (prog != s->spec_prog) {
         reset_exchange_tuning(s);
         s->auto_tile_state = 0;
+        s->list_asked = false;
     }
     if (s->d.specialize >= 0) {
         const void* k = nullptr;

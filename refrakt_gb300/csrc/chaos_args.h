@@ -6,6 +6,10 @@
 
 namespace rfk {
 
+constexpr uint32_t kRangeBits = 21;                 // bins of a point list's range: 33 MB of colour sums
+constexpr uint32_t kRangeBins = 1u << kRangeBits;
+constexpr uint32_t kMaxRanges = 64;
+
 struct ChaosArgs {
     const uint32_t* progs;   // one compiled genome per temporal sample
     uint32_t prog_stride;    // words between copies
@@ -22,7 +26,7 @@ struct ChaosArgs {
     uint64_t seed;
     int first_run;           // pass 0 reads the start points, jitters, draws colours
     int draw;
-    int splat;               // 0: a reduction per point; 1: warp-aggregated; 2: adaptive; 3: tile (splat.cuh)
+    int splat;               // 0: a reduction per point; 1: warp-aggregated; 2: adaptive; 3: tile; 4: lists (splat.cuh)
     int reset;               // 1: walkers that leave the plane restart (reset_bad_walker, device.cuh)
     uint32_t rgba_shift;     // bin addressing (splat.cuh BinTarget): 0 and 0 for the caller's
     uint32_t count_shift;    //   planes, 1 and 3 for interleaved 32-byte records
@@ -34,6 +38,11 @@ struct ChaosArgs {
     uint32_t W, H;
     float4* bins;            // RGBA sums
     uint32_t* hits;          // counts (may be null)
+    // splat 4: CTA b's points of bin range r (kRangeBins bins each) go to the list of `list_cap` entries at
+    // list + (b * ranges + r) * list_cap; their number (it may exceed the capacity) to list_n[b * ranges + r]
+    uint32_t ranges, list_cap;
+    uint2* list;
+    uint32_t* list_n;
     const float4* palette;   // 256 entries
     unsigned long long* counters;  // [0] drawn [1] emitted [2] walker-steps
     uint8_t* trace;          // xform id per (pass, 256-group), may be null

@@ -69,9 +69,10 @@ __device__ __forceinline__ int draw_phase(int tid) {
 //   program words (prog_words), palette float4[256], walker exchange float4 [2][SLOTS],
 //   JSF32 states uint4[SLOTS], group xform ids int[2][SLOTS/256], per-pass permutation ids
 //   uint32[steps], (8-byte aligned) the pipelined exchange's two mbarriers; with the tile splat
-//   (16-byte aligned) the tile's float4 RGBA sums and uint32 counts
+//   (16-byte aligned) the tile's float4 RGBA sums and uint32 counts; with the list splat (16-byte
+//   aligned) a count per bin range
 __host__ __device__ inline size_t chaos_smem_bytes(int slots, uint32_t prog_words, uint32_t steps,
-                                                   uint32_t tile_bins = 0, int pipe = 0) {
+                                                   uint32_t tile_bins = 0, int pipe = 0, uint32_t ranges = 0) {
     size_t b = ((size_t)prog_words * 4 + 15) & ~(size_t)15;
     b += 256 * 16;
     b += (size_t)2 * slots * 16;
@@ -80,6 +81,7 @@ __host__ __device__ inline size_t chaos_smem_bytes(int slots, uint32_t prog_word
     b += (size_t)steps * 4;
     if (pipe) b = ((b + 7) & ~(size_t)7) + 16;
     if (tile_bins) b = ((b + 15) & ~(size_t)15) + (size_t)tile_bins * 20;
+    if (ranges) b = ((b + 15) & ~(size_t)15) + (size_t)ranges * 4;
     return b;
 }
 
@@ -176,7 +178,12 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
         tt.count = reinterpret_cast<uint32_t*>(tt.rgba + tile_bins);
     }
 
+    const bool listed = SPLAT == 4 || (SPLAT < 0 && A.splat == 4);
+    const uint32_t ranges = listed && A.draw ? A.ranges : 0u;
+    uint32_t* s_list = reinterpret_cast<uint32_t*>(smem + ((chaos_smem_bytes(SLOTS, A.prog_words, A.steps, 0, PIPE) + 15) & ~(size_t)15));
+
     const int tid = threadIdx.x;
+    for (uint32_t i = tid; i < ranges; i += THREADS) s_list[i] = 0u;
     for (uint32_t i = tid; i < tile_bins; i += THREADS) {
         tt.rgba[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         tt.count[i] = 0u;
@@ -318,7 +325,7 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
                 if (op > 0.0f) emitted++;
                 const float px = fmaf(A.ss[0], x, fmaf(A.ss[2], y, A.ss[4]));
                 const float py = fmaf(A.ss[1], x, fmaf(A.ss[3], y, A.ss[5]));
-                uint32_t bin = kNoBin, local = kNoBin;
+                uint32_t bin = kNoBin, local = kNoBin, pi = 0;
                 float4 val = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 if (px >= 0.0f && py >= 0.0f && px < W && py < H && op > 0.0f) {
                     const uint32_t bx = (uint32_t)px, by = (uint32_t)py;
@@ -326,8 +333,11 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
                     bin = row * A.W + bx;
                     if (tile_bins && bx - A.tile_x0 < A.tile_w && row - A.tile_y0 < A.tile_h)
                         local = (row - A.tile_y0) * A.tile_w + (bx - A.tile_x0);
-                    const float4 col = s_pal[palette_index(c)];
-                    val = make_float4(col.x, col.y, col.z, op);
+                    pi = palette_index(c);
+                    if (SPLAT != 4) {
+                        const float4 col = s_pal[pi];
+                        val = make_float4(col.x, col.y, col.z, op);
+                    }
                     drawn++;
                 }
                 const BinTarget t{A.bins, A.hits, A.rgba_shift, A.count_shift};
@@ -339,10 +349,13 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
                     splat_adaptive(t, bin, val);
                 } else if constexpr (SPLAT == 3) {
                     splat_tile(t, tt, bin, local, val);
+                } else if constexpr (SPLAT == 4) {
+                    splat_list(A, t, s_list, s_pal, bin, pi, op);
                 } else {
                     if (A.splat == 1) splat_warp(t, bin, val);
                     else if (A.splat == 2) splat_adaptive(t, bin, val);
                     else if (A.splat == 3) splat_tile(t, tt, bin, local, val);
+                    else if (A.splat == 4) splat_list(A, t, s_list, s_pal, bin, pi, op);
                     else splat_global(t, bin, val);
                 }
             }
@@ -361,6 +374,10 @@ __device__ __forceinline__ void chaos_body(const ChaosArgs& A) {
             red_add_f32x4(t.at_rgba(row * A.W + col), v.x, v.y, v.z, v.w);
             if (t.count) red_add_u32x1(t.at_count(row * A.W + col), n);
         }
+    }
+    if (ranges) {
+        __syncthreads();
+        for (uint32_t i = tid; i < ranges; i += THREADS) A.list_n[blockIdx.x * ranges + i] = s_list[i];
     }
     // each slot's final walker and state were written by the thread that owns the slot
     const int out_buf = A.steps & 1;

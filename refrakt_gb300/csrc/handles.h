@@ -69,6 +69,17 @@ struct rf_sim {
     uint32_t rgba_shift = 0, count_shift = 0;  // BinTarget addressing of the next launches
     float4* rec = nullptr;       // interleaved bin records (32 B per bin), all zero between calls
     size_t rec_n = 0;
+    // the list splat's memory: scratch planes of one range (all zero between calls), then the counts and the
+    // lists of list_ctas x list_ranges x list_cap entries; list_ranges 0: the next launches have none
+    unsigned char* lists = nullptr;
+    size_t lists_bytes = 0;
+    uint32_t list_ranges = 0, list_cap = 0;
+    // after the first list call of a genome and grid (pinned, zero until they have arrived): the hits of the
+    // hottest bin, of all bins, and the points of the call that found their list full; those points' number
+    unsigned long long* list_stats = nullptr;
+    uint64_t list_points = 0;
+    uint32_t list_wh[2] = {0, 0};
+    bool list_asked = false;
     // rf_render scratch
     float4* r_bins = nullptr;
     uint32_t* r_hits = nullptr;

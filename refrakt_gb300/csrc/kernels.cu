@@ -3,6 +3,8 @@
 // table, temporal-sample animation and the single-step probe.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "chaos_body.cuh"
 #include "kernels.h"
 
@@ -35,6 +37,171 @@ __global__ void merge_records_kernel(float4* __restrict__ rec, size_t n, float4*
 
 cudaError_t launch_merge_records(float4* rec, size_t n, float4* bins, uint32_t* hits, cudaStream_t st) {
     merge_records_kernel<<<152 * 16, 256, 0, st>>>(rec, n, bins, hits);
+    return cudaGetLastError();
+}
+
+// One step of adding the point lists (chaos_args.h, splat 4) to the planes: range `range`'s lists into scratch
+// planes that stay in L2, and range - 1's scratch planes (the other set) into the caller's, cleared.  The
+// first half is bound by the SMs' requests to L2 (a reduction or two per point), the second by DRAM (the
+// planes read and written once), so they run side by side, in interleaved CTAs of one launch.  80 M points
+// of the space-filling genome on 8192 x 8192 bins: lists written by the chaos kernel in 0.76 ms, added in
+// 33 steps of 20 to 48 us (of which 335 us are the reductions, 156 us reading the lists, 430 us the planes,
+// 130 us launches), 1.85 ms in all; interleaved records written at random and merged took 2.9 + 0.8 ms.
+// Ranges of 2^20 or 2^19 bins: 1.93, 2.19 ms.
+//
+// Where a range's lists hold fewer than 2^24 points in all (UNIT), a point of opacity 1 takes one reduction:
+// the alpha sum of such points is their exact count.  The others go to a second set with a count plane.
+// Otherwise every point takes its colour's reduction and its count's.
+struct RangeArgs {
+    const uint2* list;
+    const uint32_t* list_n;
+    uint32_t cap, ranges, ctas, range, nb;
+    const float4* palette;
+    RangeScratch set[2];
+    uint32_t* mixed;  // per range: its lists hold points of another opacity than 1
+    unsigned long long* over;  // points that found their list full
+    float4* bins;
+    uint32_t* hits;
+};
+constexpr uint32_t kRangeThreads = 512, kMergeCtas = 1024;
+
+template <bool UNIT>
+__device__ __forceinline__ void range_add(const RangeArgs& R, uint32_t cta, float4* s_pal) {
+    const size_t at = (size_t)cta * R.ranges + R.range;
+    const uint32_t wanted = R.list_n[at], n = min(wanted, R.cap);
+    if (n == 0) return;
+    if (wanted > n && threadIdx.x == 0) atomicAdd(R.over, (unsigned long long)(wanted - n));
+    const uint2* list = R.list + at * R.cap;
+    const RangeScratch& S = R.set[R.range & 1];
+    if (threadIdx.x < 256) s_pal[threadIdx.x] = R.palette[threadIdx.x];
+    __syncthreads();
+    constexpr int U = 4;  // entries in flight per thread
+    for (uint32_t i0 = 0; i0 < n; i0 += kRangeThreads * U) {
+        uint2 e[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const uint32_t i = i0 + kRangeThreads * u + threadIdx.x;
+            e[u] = i < n ? __ldcs(list + i) : make_uint2(kNoBin, 0u);
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const uint32_t bin = e[u].x == kNoBin ? kNoBin : e[u].x & (kRangeBins - 1);
+            const float op = __uint_as_float(e[u].y);
+            const float4 c = s_pal[e[u].x >> 24];
+            const float4 v = make_float4(c.x, c.y, c.z, op);
+            if (UNIT) {
+                const bool other = bin != kNoBin && op != 1.0f;
+                splat_adaptive(BinTarget{S.rgba, nullptr, 0u, 0u}, other ? kNoBin : bin, v);
+                if (__any_sync(0xffffffffu, other)) {
+                    splat_adaptive(BinTarget{S.rgba2, S.count, 0u, 0u}, other ? bin : kNoBin, v);
+                    if (other) R.mixed[R.range] = 1u;
+                }
+            } else {
+                splat_adaptive(BinTarget{S.rgba, S.count, 0u, 0u}, bin, v);
+            }
+        }
+    }
+}
+
+template <bool UNIT>
+__device__ __forceinline__ void range_merge(const RangeArgs& R, uint32_t cta) {
+    const uint32_t r = R.range - 1, first = r << kRangeBits, n = min(R.nb - first, kRangeBins);
+    const RangeScratch& S = R.set[r & 1];
+    const bool mixed = UNIT && R.mixed[r] != 0;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    constexpr uint32_t kStep = kMergeCtas * kRangeThreads;
+    constexpr int U = 2;
+    for (uint32_t i0 = cta * kRangeThreads + threadIdx.x; i0 < n; i0 += kStep * U) {
+        float4 v[U], b[U];
+        uint32_t c[U], h[U];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const uint32_t i = i0 + kStep * u;
+            v[u] = zero;
+            c[u] = 0u;
+            if (i >= n) continue;
+            if (UNIT) {
+                v[u] = S.rgba[i];
+                c[u] = (uint32_t)v[u].w;
+                if (v[u].w != 0.0f) S.rgba[i] = zero;
+                if (mixed) {
+                    if (const uint32_t m = S.count[i]) {
+                        const float4 w = S.rgba2[i];
+                        v[u] = make_float4(v[u].x + w.x, v[u].y + w.y, v[u].z + w.z, v[u].w + w.w);
+                        c[u] += m;
+                        S.rgba2[i] = zero;
+                        S.count[i] = 0u;
+                    }
+                }
+            } else {
+                c[u] = S.count[i];
+                if (c[u]) {
+                    v[u] = S.rgba[i];
+                    S.rgba[i] = zero;
+                    S.count[i] = 0u;
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (c[u]) {
+                b[u] = __ldcs(R.bins + first + i0 + kStep * u);
+                h[u] = __ldcs(R.hits + first + i0 + kStep * u);
+            }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+            if (c[u]) {
+                __stcs(R.bins + first + i0 + kStep * u,
+                       make_float4(b[u].x + v[u].x, b[u].y + v[u].y, b[u].z + v[u].z, b[u].w + v[u].w));
+                __stcs(R.hits + first + i0 + kStep * u, h[u] + c[u]);
+            }
+    }
+}
+
+template <bool UNIT>
+__global__ void __launch_bounds__(kRangeThreads, 4) range_step_kernel(const __grid_constant__ RangeArgs R) {
+    __shared__ float4 s_pal[256];
+    const uint32_t adds = R.range < R.ranges ? R.ctas : 0u, merges = R.range > 0 ? kMergeCtas : 0u;
+    const uint32_t both = 2 * min(adds, merges);
+    const bool add = blockIdx.x < both ? (blockIdx.x & 1u) == 0u : adds > merges;
+    const uint32_t cta = blockIdx.x < both ? blockIdx.x >> 1 : blockIdx.x - both / 2;
+    if (add) range_add<UNIT>(R, cta, s_pal);
+    else range_merge<UNIT>(R, cta);
+}
+
+cudaError_t launch_ranges(const ChaosArgs& a, uint32_t ctas, const RangeScratch set[2], uint32_t* mixed,
+                          unsigned long long* over, cudaStream_t st) {
+    RangeArgs R{a.list, a.list_n, a.list_cap, a.ranges, ctas, 0, a.W * a.H, a.palette, {set[0], set[1]}, mixed, over, a.bins, a.hits};
+    const bool unit = (uint64_t)a.list_cap * ctas < (1u << 24);
+    cudaError_t e = cudaMemsetAsync(mixed, 0, kMaxRanges * sizeof(uint32_t), st);
+    for (; R.range <= a.ranges && e == cudaSuccess; R.range++) {
+        const uint32_t grid = (R.range < a.ranges ? ctas : 0u) + (R.range > 0 ? kMergeCtas : 0u);
+        if (unit) range_step_kernel<true><<<grid, kRangeThreads, 0, st>>>(R);
+        else range_step_kernel<false><<<grid, kRangeThreads, 0, st>>>(R);
+        e = cudaGetLastError();
+    }
+    return e;
+}
+
+// out[0]: the hits of the hottest bin, out[1]: of all bins (both 0 on entry)
+__global__ void __launch_bounds__(256) hottest_bin_kernel(const uint32_t* __restrict__ hits, size_t n, unsigned long long* out) {
+    uint32_t most = 0;
+    unsigned long long sum = 0;
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
+        const uint32_t h = hits[i];
+        most = max(most, h);
+        sum += h;
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if ((threadIdx.x & 31) == 0 && sum) {
+        atomicMax(out, (unsigned long long)most);
+        atomicAdd(out + 1, sum);
+    }
+}
+
+cudaError_t launch_hottest_bin(const uint32_t* hits, size_t n, unsigned long long* out, cudaStream_t st) {
+    hottest_bin_kernel<<<152 * 8, 256, 0, st>>>(hits, n, out);
     return cudaGetLastError();
 }
 
@@ -151,14 +318,15 @@ __global__ void probe_kernel(const uint32_t* prog, int xform, uint32_t n, const 
 // ---------------------------------------------------------------------------------------------
 // host launchers
 // ---------------------------------------------------------------------------------------------
-size_t chaos_smem(int slots, uint32_t prog_words, uint32_t steps, uint32_t tile_bins, int pipe) {
-    return chaos_smem_bytes(slots, prog_words, steps, tile_bins, pipe);
+size_t chaos_smem(int slots, uint32_t prog_words, uint32_t steps, uint32_t tile_bins, int pipe, uint32_t ranges) {
+    return chaos_smem_bytes(slots, prog_words, steps, tile_bins, pipe, ranges);
 }
 
 template <int THREADS, int SPT>
 static cudaError_t launch_chaos_t(const ChaosArgs& a, uint32_t grid, cudaStream_t st) {
     const size_t smem = chaos_smem_bytes(THREADS * SPT, a.prog_words, a.steps,
-                                         a.splat == 3 && a.draw ? a.tile_w * a.tile_h : 0u);
+                                         a.splat == 3 && a.draw ? a.tile_w * a.tile_h : 0u, 0,
+                                         a.splat == 4 && a.draw ? a.ranges : 0u);
     auto kern = chaos_kernel<THREADS, SPT>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

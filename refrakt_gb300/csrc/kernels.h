@@ -14,7 +14,8 @@ namespace rfk {
 
 
 
-size_t chaos_smem(int slots, uint32_t prog_words, uint32_t steps, uint32_t tile_bins = 0, int pipe = 0);
+size_t chaos_smem(int slots, uint32_t prog_words, uint32_t steps, uint32_t tile_bins = 0, int pipe = 0,
+                  uint32_t ranges = 0);
 constexpr size_t kMaxCtaSmem = 232448;  // dynamic shared memory a CTA may opt into (227 KB)
 // CTAs per mixing domain that a simulation of `domains` domains of `slots` should spread over (the
 // cluster exchange, chaos_body.cuh), 1 for none: the most (8, 4, 2) that leave each CTA a 256-slot
@@ -22,6 +23,15 @@ constexpr size_t kMaxCtaSmem = 232448;  // dynamic shared memory a CTA may opt i
 int chaos_cluster(int slots, uint64_t domains, uint32_t prog_words, uint32_t steps);
 bool chaos_shape_supported(int threads, int slots);
 cudaError_t launch_chaos(int threads, int slots, const ChaosArgs& a, uint32_t grid, cudaStream_t st);
+// scratch planes of kRangeBins bins each, all zero between launches (kernels.cu)
+struct RangeScratch {
+    float4 *rgba, *rgba2;
+    uint32_t* count;
+};
+// the lists of a launch of `ctas` CTAs with splat 4 into its planes; mixed: kMaxRanges words
+cudaError_t launch_ranges(const ChaosArgs& a, uint32_t ctas, const RangeScratch set[2], uint32_t* mixed,
+                          unsigned long long* over, cudaStream_t st);
+cudaError_t launch_hottest_bin(const uint32_t* hits, size_t n, unsigned long long* out, cudaStream_t st);
 cudaError_t launch_merge_records(float4* rec, size_t n, float4* bins, uint32_t* hits, cudaStream_t st);
 cudaError_t launch_init_rng(uint4* rng, uint64_t n, uint64_t seed, cudaStream_t st);
 cudaError_t launch_shuffle_table(uint16_t* out, uint32_t n, uint32_t count, uint64_t seed, cudaStream_t st,

@@ -19,9 +19,14 @@
 //                  the warp as splat_adaptive does), the others to splat_global; the chaos
 //                  kernel adds the tile's non-empty bins to the histogram once per launch, so
 //                  the L2 sees a few reductions per bin per CTA instead of one per point.
+//   splat_list   — for bin grids far above L2: the point goes to a list of its CTA and bin range (8 bytes:
+//                  bin within the range, palette index, opacity) instead of to a random DRAM sector; the
+//                  lists are then added range by range, each range's bins staying in L2 (range_step_kernel).
+//                  Warps whose neighbouring lanes share a bin aggregate as splat_adaptive does, and
+//                  points that find their list full go to the bins.
 #pragma once
 
-#include "rtc_types.h"
+#include "chaos_args.h"
 
 namespace rfk {
 
@@ -155,6 +160,27 @@ __device__ __forceinline__ void splat_adaptive(const BinTarget& t, uint32_t bin,
     const uint32_t other = __shfl_xor_sync(0xffffffffu, bin, 1);
     if (__any_sync(0xffffffffu, bin != kNoBin && bin == other)) splat_warp(t, bin, v);
     else splat_global(t, bin, v);
+}
+
+// Every lane of the warp must call this; `pal` is the palette in shared memory, `palette` the point's entry
+// in it, s_list the CTA's count of points per range.
+__device__ __forceinline__ void splat_list(const ChaosArgs& A, const BinTarget& t, uint32_t* s_list, const float4* pal,
+                                           uint32_t bin, uint32_t palette, float op) {
+    const uint32_t other = __shfl_xor_sync(0xffffffffu, bin, 1);
+    const bool compact = __any_sync(0xffffffffu, bin != kNoBin && bin == other);
+    bool listed = false;
+    if (!compact && bin != kNoBin) {
+        const uint32_t r = bin >> kRangeBits;
+        const uint32_t pos = atomicAdd(&s_list[r], 1u);
+        listed = pos < A.list_cap;
+        if (listed)
+            __stcs(A.list + (size_t)(blockIdx.x * A.ranges + r) * A.list_cap + pos,
+                   make_uint2((bin & (kRangeBins - 1)) | (palette << 24), __float_as_uint(op)));
+    }
+    if (__any_sync(0xffffffffu, bin != kNoBin && !listed)) {
+        const float4 c = pal[palette];
+        splat_adaptive(t, listed ? kNoBin : bin, make_float4(c.x, c.y, c.z, op));
+    }
 }
 
 }  // namespace rfk
