@@ -56,8 +56,9 @@ int splat_code(int splat) {
 namespace {
 
 constexpr size_t kListBytes = 16ull << 30;  // the lists' memory at most: 256 passes of 2.5 M walkers at three times an even spread
+constexpr size_t kListMinBins = 1u << 25;
 constexpr uint64_t kListHot = 1024;
-constexpr size_t kListScratch = (size_t)kRangeBins * 72 + kMaxRanges * 4;  // two sets of scratch planes, flags
+constexpr size_t kListScratch = ((size_t)72 << kMaxRangeBits) + kMaxRanges * sizeof(RangeState);  // two sets of scratch planes
 constexpr size_t kInterleaveMinBytes = 256ull << 20;  // bins + counts above ~2x L2: interleave
 
 int set_device(const rf_sim* s) {
@@ -279,6 +280,7 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
         const uint32_t tile_bins = a.splat == 3 && a.draw ? a.tile_w * a.tile_h : 0u;
         if (s->list_ranges) {
             a.ranges = s->list_ranges;
+            a.range_bits = s->list_range_bits;
             a.list_cap = s->list_cap;
             a.list_n = reinterpret_cast<uint32_t*>(s->lists + kListScratch);
             a.list = reinterpret_cast<uint2*>(a.list_n + (((s->N / s->slots) * a.ranges + 3) & ~(size_t)3));
@@ -320,12 +322,13 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
         const bool tile_recorded = tile_timed >= 0 && cudaEventRecord(s->tile_ev[2 * tile_timed + 1], s->stream) == cudaSuccess;
         if (a.ranges) {
             RangeScratch set[2];
+            const size_t n = (size_t)1 << kMaxRangeBits;
             for (int k = 0; k < 2; k++) {
-                set[k].rgba = reinterpret_cast<float4*>(s->lists) + (size_t)(2 * k) * kRangeBins;
-                set[k].rgba2 = set[k].rgba + kRangeBins;
-                set[k].count = reinterpret_cast<uint32_t*>(s->lists + (size_t)kRangeBins * 64) + (size_t)k * kRangeBins;
+                set[k].rgba = reinterpret_cast<float4*>(s->lists) + 2 * k * n;
+                set[k].rgba2 = set[k].rgba + n;
+                set[k].count = reinterpret_cast<uint32_t*>(s->lists + n * 64) + k * n;
             }
-            RF_CUDA(launch_ranges(a, grid, set, reinterpret_cast<uint32_t*>(s->lists + kListScratch) - kMaxRanges,
+            RF_CUDA(launch_ranges(a, grid, set, reinterpret_cast<RangeState*>(s->lists + kListScratch) - kMaxRanges,
                                   s->counters + 6, s->stream));
         }
         s->cur ^= 1;
@@ -347,8 +350,9 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
 }
 
 // Point lists (splat 4) for the drawing launches of a call on a grid far above L2, instead of interleaved
-// records: 80 M points of the space-filling genome on 8192 x 8192 bins 3.98 -> 1.87 ms (637 M 24.9 -> 15.7), of
-// the 1080p genome 3.50 -> 2.46.  Not for hot bins, whose points the lists' second step adds one after another while the
+// records.  80 M points of the space-filling genome, of the 1080p genome, ms with records and with lists: 8192 x
+// 8192 bins 3.94, 1.84 and 3.49, 2.47 (637 M points 24.9, 11.7); 8192 x 4608 3.26, 1.65 and 2.50, 2.28; 6000 x
+// 4000 2.58, 1.56 and 1.88, 2.28; 4099 x 3301 1.68, 1.49 and 1.69, 2.29: from kListMinBins bins on.  Not for hot bins, whose points the lists' second step adds one after another while the
 // records' reductions pass under the chaos game (62 M points of the 5-xform genome on 5000 x 4001 bins, 0.3 % of
 // them in one bin: 1.63 ms with records, 1.80 with lists): the first call measures, later ones take records
 // above a share of 1 / kListHot in one bin or where an eighth of the points found their list full.
@@ -379,7 +383,11 @@ void measure_lists(rf_sim* s, const uint32_t* hits, uint32_t W, uint32_t H, uint
 // the lists' memory for a call of `passes` passes, four times an even spread over the ranges where it fits, at
 // least 1.25 times; false: it does not, or the sim's domains are spread over clusters
 bool reserve_lists(rf_sim* s, size_t nb, uint32_t passes) {
-    const uint32_t ranges = (uint32_t)((nb + kRangeBins - 1) >> kRangeBits);
+    // ranges of 2^21 bins; of 2^20 where more than 2^23 points of a launch fall into one on average, so that
+    // most stay below the 2^24 of a single reduction per point (637 M points on 8192 x 8192 bins: 13.9 -> 11.7 ms)
+    uint32_t bits = kMaxRangeBits;
+    if ((s->N * std::min(passes, s->L) >> 23) << bits > nb && nb <= (uint64_t)kMaxRanges << (bits - 1)) bits--;
+    const uint32_t ranges = (uint32_t)((nb + (1u << bits) - 1) >> bits);
     // (a captured call takes records: a later call may move the lists)
     if (s->splat != RF_SPLAT_AUTO || ranges > kMaxRanges || (s->spec && cluster_for_launch(s, true) > 1) || capturing(s->stream))
         return false;
@@ -402,6 +410,7 @@ bool reserve_lists(rf_sim* s, size_t nb, uint32_t passes) {
         s->lists_bytes = bytes;
     }
     s->list_ranges = ranges;
+    s->list_range_bits = bits;
     s->list_cap = (uint32_t)cap;
     return true;
 }
@@ -414,7 +423,7 @@ int draw_passes(rf_sim* s, uint32_t passes, float4* bins, uint32_t* hits, uint32
     bool il = s->bin_layout == RF_BINS_INTERLEAVED;
     if (s->bin_layout == RF_BINS_AUTO) il = hits != nullptr && nb * 20 > kInterleaveMinBytes;
     if (!il) return launch_passes(s, passes, false, true, bins, hits, W, H, ss);
-    if (s->bin_layout == RF_BINS_AUTO && lists_suit(s, W, H) && reserve_lists(s, nb, passes)) {
+    if (s->bin_layout == RF_BINS_AUTO && nb >= kListMinBins && lists_suit(s, W, H) && reserve_lists(s, nb, passes)) {
         RF_CUDA(cudaMemsetAsync(s->counters + 6, 0, sizeof(unsigned long long), s->stream));
         const int rc = launch_passes(s, passes, false, true, bins, hits, W, H, ss);
         s->list_ranges = 0;

@@ -6,8 +6,7 @@
 
 namespace rfk {
 
-constexpr uint32_t kRangeBits = 21;                 // bins of a point list's range: 33 MB of colour sums
-constexpr uint32_t kRangeBins = 1u << kRangeBits;
+constexpr uint32_t kMaxRangeBits = 21;  // bins of a point list's range, at most: 33 MB of colour sums
 constexpr uint32_t kMaxRanges = 64;
 
 struct ChaosArgs {
@@ -38,9 +37,9 @@ struct ChaosArgs {
     uint32_t W, H;
     float4* bins;            // RGBA sums
     uint32_t* hits;          // counts (may be null)
-    // splat 4: CTA b's points of bin range r (kRangeBins bins each) go to the list of `list_cap` entries at
+    // splat 4: CTA b's points of bin range r (2^range_bits bins each) go to the list of `list_cap` entries at
     // list + (b * ranges + r) * list_cap; their number (it may exceed the capacity) to list_n[b * ranges + r]
-    uint32_t ranges, list_cap;
+    uint32_t ranges, range_bits, list_cap;
     uint2* list;
     uint32_t* list_n;
     const float4* palette;   // 256 entries

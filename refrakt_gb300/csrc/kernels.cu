@@ -46,31 +46,51 @@ cudaError_t launch_merge_records(float4* rec, size_t n, float4* bins, uint32_t* 
 // planes read and written once), so they run side by side, in interleaved CTAs of one launch.  80 M points
 // of the space-filling genome on 8192 x 8192 bins: lists written by the chaos kernel in 0.76 ms, added in
 // 33 steps of 20 to 48 us (of which 335 us are the reductions, 156 us reading the lists, 430 us the planes,
-// 130 us launches), 1.85 ms in all; interleaved records written at random and merged took 2.9 + 0.8 ms.
-// Ranges of 2^20 or 2^19 bins: 1.93, 2.19 ms.
+// 130 us launches), 1.84 ms in all; interleaved records written at random and merged took 2.9 + 0.8 ms.
+// Ranges of 2^20 bins 1.95 ms; 256 threads, 4 CTAs per SM (spills), half the merging CTAs 1.87 to 1.94.
 //
-// Where a range's lists hold fewer than 2^24 points in all (UNIT), a point of opacity 1 takes one reduction:
-// the alpha sum of such points is their exact count.  The others go to a second set with a count plane.
-// Otherwise every point takes its colour's reduction and its count's.
+// Where a range's lists hold fewer than 2^24 points (range_count_kernel), a point of opacity 1 takes one
+// reduction: the alpha sum of such points is their exact count.  The others go to a second set with a count
+// plane.  In a fuller range every point takes its colour's reduction and its count's (80 M points on 8192 x 4608
+// bins: 2.4 instead of 1.65 ms).
 struct RangeArgs {
     const uint2* list;
     const uint32_t* list_n;
-    uint32_t cap, ranges, ctas, range, nb;
+    uint32_t cap, ranges, range_bits, ctas, range, nb;
     const float4* palette;
     RangeScratch set[2];
-    uint32_t* mixed;  // per range: its lists hold points of another opacity than 1
-    unsigned long long* over;  // points that found their list full
+    RangeState* state;  // per range
     float4* bins;
     uint32_t* hits;
 };
 constexpr uint32_t kRangeThreads = 512, kMergeCtas = 1024;
 
+// a CTA per range: the points in its lists, and those that found their list full
+__global__ void __launch_bounds__(256) range_count_kernel(const uint32_t* __restrict__ list_n, uint32_t ctas, uint32_t ranges,
+                                                          uint32_t cap, RangeState* state, unsigned long long* over) {
+    __shared__ unsigned long long s_sum[2];
+    if (threadIdx.x < 2) s_sum[threadIdx.x] = 0;
+    __syncthreads();
+    unsigned long long in = 0, out = 0;
+    for (uint32_t c = threadIdx.x; c < ctas; c += 256) {
+        const uint32_t n = list_n[(size_t)c * ranges + blockIdx.x];
+        in += min(n, cap);
+        out += n - min(n, cap);
+    }
+    atomicAdd(&s_sum[0], in);
+    atomicAdd(&s_sum[1], out);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        state[blockIdx.x] = RangeState{s_sum[0] < (1u << 24) ? 1u : 0u, 0u};
+        if (s_sum[1]) atomicAdd(over, s_sum[1]);
+    }
+}
+
 template <bool UNIT>
 __device__ __forceinline__ void range_add(const RangeArgs& R, uint32_t cta, float4* s_pal) {
     const size_t at = (size_t)cta * R.ranges + R.range;
-    const uint32_t wanted = R.list_n[at], n = min(wanted, R.cap);
+    const uint32_t n = min(R.list_n[at], R.cap);
     if (n == 0) return;
-    if (wanted > n && threadIdx.x == 0) atomicAdd(R.over, (unsigned long long)(wanted - n));
     const uint2* list = R.list + at * R.cap;
     const RangeScratch& S = R.set[R.range & 1];
     if (threadIdx.x < 256) s_pal[threadIdx.x] = R.palette[threadIdx.x];
@@ -85,7 +105,7 @@ __device__ __forceinline__ void range_add(const RangeArgs& R, uint32_t cta, floa
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
-            const uint32_t bin = e[u].x == kNoBin ? kNoBin : e[u].x & (kRangeBins - 1);
+            const uint32_t bin = e[u].x == kNoBin ? kNoBin : e[u].x & 0xffffffu;
             const float op = __uint_as_float(e[u].y);
             const float4 c = s_pal[e[u].x >> 24];
             const float4 v = make_float4(c.x, c.y, c.z, op);
@@ -94,7 +114,7 @@ __device__ __forceinline__ void range_add(const RangeArgs& R, uint32_t cta, floa
                 splat_adaptive(BinTarget{S.rgba, nullptr, 0u, 0u}, other ? kNoBin : bin, v);
                 if (__any_sync(0xffffffffu, other)) {
                     splat_adaptive(BinTarget{S.rgba2, S.count, 0u, 0u}, other ? bin : kNoBin, v);
-                    if (other) R.mixed[R.range] = 1u;
+                    if (other) R.state[R.range].mixed = 1u;
                 }
             } else {
                 splat_adaptive(BinTarget{S.rgba, S.count, 0u, 0u}, bin, v);
@@ -105,9 +125,9 @@ __device__ __forceinline__ void range_add(const RangeArgs& R, uint32_t cta, floa
 
 template <bool UNIT>
 __device__ __forceinline__ void range_merge(const RangeArgs& R, uint32_t cta) {
-    const uint32_t r = R.range - 1, first = r << kRangeBits, n = min(R.nb - first, kRangeBins);
+    const uint32_t r = R.range - 1, first = r << R.range_bits, n = min(R.nb - first, 1u << R.range_bits);
     const RangeScratch& S = R.set[r & 1];
-    const bool mixed = UNIT && R.mixed[r] != 0;
+    const bool mixed = UNIT && R.state[r].mixed != 0;
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     constexpr uint32_t kStep = kMergeCtas * kRangeThreads;
     constexpr int U = 2;
@@ -158,26 +178,30 @@ __device__ __forceinline__ void range_merge(const RangeArgs& R, uint32_t cta) {
     }
 }
 
-template <bool UNIT>
-__global__ void __launch_bounds__(kRangeThreads, 4) range_step_kernel(const __grid_constant__ RangeArgs R) {
+__global__ void __launch_bounds__(kRangeThreads, 3) range_step_kernel(const __grid_constant__ RangeArgs R) {
     __shared__ float4 s_pal[256];
     const uint32_t adds = R.range < R.ranges ? R.ctas : 0u, merges = R.range > 0 ? kMergeCtas : 0u;
     const uint32_t both = 2 * min(adds, merges);
     const bool add = blockIdx.x < both ? (blockIdx.x & 1u) == 0u : adds > merges;
     const uint32_t cta = blockIdx.x < both ? blockIdx.x >> 1 : blockIdx.x - both / 2;
-    if (add) range_add<UNIT>(R, cta, s_pal);
-    else range_merge<UNIT>(R, cta);
+    const bool unit = R.state[add ? R.range : R.range - 1].unit != 0;
+    if (add) {
+        if (unit) range_add<true>(R, cta, s_pal);
+        else range_add<false>(R, cta, s_pal);
+    } else {
+        if (unit) range_merge<true>(R, cta);
+        else range_merge<false>(R, cta);
+    }
 }
 
-cudaError_t launch_ranges(const ChaosArgs& a, uint32_t ctas, const RangeScratch set[2], uint32_t* mixed,
+cudaError_t launch_ranges(const ChaosArgs& a, uint32_t ctas, const RangeScratch set[2], RangeState* state,
                           unsigned long long* over, cudaStream_t st) {
-    RangeArgs R{a.list, a.list_n, a.list_cap, a.ranges, ctas, 0, a.W * a.H, a.palette, {set[0], set[1]}, mixed, over, a.bins, a.hits};
-    const bool unit = (uint64_t)a.list_cap * ctas < (1u << 24);
-    cudaError_t e = cudaMemsetAsync(mixed, 0, kMaxRanges * sizeof(uint32_t), st);
+    RangeArgs R{a.list, a.list_n, a.list_cap, a.ranges, a.range_bits, ctas, 0, a.W * a.H, a.palette, {set[0], set[1]}, state, a.bins, a.hits};
+    range_count_kernel<<<a.ranges, 256, 0, st>>>(a.list_n, ctas, a.ranges, a.list_cap, state, over);
+    cudaError_t e = cudaGetLastError();
     for (; R.range <= a.ranges && e == cudaSuccess; R.range++) {
         const uint32_t grid = (R.range < a.ranges ? ctas : 0u) + (R.range > 0 ? kMergeCtas : 0u);
-        if (unit) range_step_kernel<true><<<grid, kRangeThreads, 0, st>>>(R);
-        else range_step_kernel<false><<<grid, kRangeThreads, 0, st>>>(R);
+        range_step_kernel<<<grid, kRangeThreads, 0, st>>>(R);
         e = cudaGetLastError();
     }
     return e;

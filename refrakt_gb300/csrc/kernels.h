@@ -23,13 +23,17 @@ constexpr size_t kMaxCtaSmem = 232448;  // dynamic shared memory a CTA may opt i
 int chaos_cluster(int slots, uint64_t domains, uint32_t prog_words, uint32_t steps);
 bool chaos_shape_supported(int threads, int slots);
 cudaError_t launch_chaos(int threads, int slots, const ChaosArgs& a, uint32_t grid, cudaStream_t st);
-// scratch planes of kRangeBins bins each, all zero between launches (kernels.cu)
+// scratch planes of a range's bins each, all zero between launches (kernels.cu)
 struct RangeScratch {
     float4 *rgba, *rgba2;
     uint32_t* count;
 };
-// the lists of a launch of `ctas` CTAs with splat 4 into its planes; mixed: kMaxRanges words
-cudaError_t launch_ranges(const ChaosArgs& a, uint32_t ctas, const RangeScratch set[2], uint32_t* mixed,
+struct RangeState {
+    uint32_t unit, mixed;  // fewer than 2^24 points in the range's lists; among them some of opacity other than 1
+};
+// the lists of a launch of `ctas` CTAs with splat 4 into its planes; points that found their list full are
+// added to *over
+cudaError_t launch_ranges(const ChaosArgs& a, uint32_t ctas, const RangeScratch set[2], RangeState* state,
                           unsigned long long* over, cudaStream_t st);
 cudaError_t launch_hottest_bin(const uint32_t* hits, size_t n, unsigned long long* out, cudaStream_t st);
 cudaError_t launch_merge_records(float4* rec, size_t n, float4* bins, uint32_t* hits, cudaStream_t st);

@@ -170,12 +170,12 @@ __device__ __forceinline__ void splat_list(const ChaosArgs& A, const BinTarget& 
     const bool compact = __any_sync(0xffffffffu, bin != kNoBin && bin == other);
     bool listed = false;
     if (!compact && bin != kNoBin) {
-        const uint32_t r = bin >> kRangeBits;
+        const uint32_t r = bin >> A.range_bits;
         const uint32_t pos = atomicAdd(&s_list[r], 1u);
         listed = pos < A.list_cap;
         if (listed)
             __stcs(A.list + (size_t)(blockIdx.x * A.ranges + r) * A.list_cap + pos,
-                   make_uint2((bin & (kRangeBins - 1)) | (palette << 24), __float_as_uint(op)));
+                   make_uint2((bin & ((1u << A.range_bits) - 1)) | (palette << 24), __float_as_uint(op)));
     }
     if (__any_sync(0xffffffffu, bin != kNoBin && !listed)) {
         const float4 c = pal[palette];
