@@ -332,9 +332,9 @@ __device__ __forceinline__ TileCoord tile_coord(const GemmArgs& g, uint32_t t, u
 template <int BN>
 __global__ void __launch_bounds__(kTmaThreads, 1)
     umma_gemm_tma_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                         const GemmArgs g, uint32_t splits) {
+                         const GemmArgs g, uint32_t splits, uint32_t bn) {
     constexpr int S = tma_stages<BN>();
-    constexpr uint32_t kA = kBM * 128, kB = BN * 128;  // bytes of one stage's A and B blocks
+    constexpr uint32_t kA = kBM * 128, kB = BN * 128;  // bytes of one stage's A and B blocks (B: bn rows of it used)
     constexpr uint32_t kCols = BN < 32 ? 32 : BN;      // one accumulator; two are allocated
     extern __shared__ __align__(16) unsigned char smem_raw[];
     unsigned char* smem = smem_raw + ((1024u - (umma::smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
     const uint32_t base = umma::smem_u32(smem);
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t tiles_m = (g.M + kBM - 1) / kBM, tiles_n = (g.N + BN - 1) / BN;
+    const uint32_t tiles_m = (g.M + kBM - 1) / kBM, tiles_n = (g.N + bn - 1) / bn;
     const uint32_t tiles = tiles_m * tiles_n * splits;
 
     if (warp == 1) umma::tmem_alloc(s_tmem, 2 * kCols);
@@ -370,10 +370,10 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
     const uint32_t tmem = *s_tmem;
 
     if (warp == 0) {
-        if (lane == 0) {
+        if (umma::elect_one()) {
             uint32_t it = 0;  // K blocks issued by this CTA
             for (uint32_t t = blockIdx.x; t < tiles && !gemm_failed(s_fail); t += gridDim.x) {
-                const TileCoord c = tile_coord(g, t, tiles_m, tiles_n, BN);
+                const TileCoord c = tile_coord(g, t, tiles_m, tiles_n, bn);
                 for (uint32_t kb = 0; kb < c.nk; kb++, it++) {
                     const uint32_t st = it % S, use = it / S;
                     if (use > 0 && !umma::mbar_wait(&empty[st], (use - 1) & 1u, kWaitLimit)) {
@@ -381,7 +381,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
                         break;
                     }
                     if (gemm_failed(s_fail)) break;
-                    umma::mbar_arrive_expect_tx(&full[st], kA + kB);
+                    umma::mbar_arrive_expect_tx(&full[st], kA + bn * 128);
                     const uint32_t a = base + st * (kA + kB), b = a + kA;
                     const int kx = (int)(c.k0 + kb * umma::kTileK);
                     umma::tma_load_2d(a, &tmA, kx, (int)c.m0, &full[st]);
@@ -394,13 +394,13 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (umma::elect_one()) {
             uint32_t it = 0, i = 0;  // K blocks consumed, tiles done by this CTA
             for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x, i++) {
-                const TileCoord c = tile_coord(g, t, tiles_m, tiles_n, BN);
+                const TileCoord c = tile_coord(g, t, tiles_m, tiles_n, bn);
                 const uint32_t buf = i & 1u, u = i >> 1;
                 const uint32_t n_rem = g.N - c.n0;
-                const uint32_t n_tile = ((n_rem < (uint32_t)BN ? n_rem : (uint32_t)BN) + 15u) & ~15u;
+                const uint32_t n_tile = ((n_rem < bn ? n_rem : bn) + 15u) & ~15u;
                 const uint32_t idesc = umma::idesc_bf16_f32(kBM, n_tile);
                 bool ok = !gemm_failed(s_fail);
                 if (ok && u > 0 && !umma::mbar_wait(&acc_empty[buf], (u - 1) & 1u, kWaitLimit)) {
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
         float* rows = stage_out;
         uint32_t i = 0;
         for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x, i++) {
-            const TileCoord c = tile_coord(g, t, tiles_m, tiles_n, BN);
+            const TileCoord c = tile_coord(g, t, tiles_m, tiles_n, bn);
             const uint32_t buf = i & 1u, u = i >> 1;
             if (!umma::mbar_wait(&acc_full[buf], u & 1u, kWaitLimit)) {
                 gemm_fail(g, s_fail, 3 + 2 * S + (int)buf);
@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
             umma::fence_after_sync();
             if (gemm_failed(s_fail)) break;
             const uint32_t n_rem = g.N - c.n0;
-            const uint32_t n_tile = ((n_rem < (uint32_t)BN ? n_rem : (uint32_t)BN) + 15u) & ~15u;
+            const uint32_t n_tile = ((n_rem < bn ? n_rem : bn) + 15u) & ~15u;
             if (c.nk > 0 || g.mode != kGemmAtomicF32)
                 warp_epilogue(g, rows, tmem + buf * kCols, q, (uint32_t)lane, c.m0, c.n0, n_tile, c.nk > 0);
             umma::fence_before_sync();
@@ -481,11 +481,32 @@ bool encode_operand(CUtensorMap* m, const __nv_bfloat16* p, uint32_t inner, uint
                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The tile width (columns, a multiple of 16, at most BN) whose last round of tiles leaves the fewest SMs
+// idle: the rounds of tiles times a tile's time, which is the width's on the tensor cores, 64 columns and
+// half the width's where reading the operands from shared memory takes longer, and 24 columns' worth for
+// the rest.  4096 x 4096 has 512 tiles of 256 columns, 3.4 rounds of 152 SMs that take 4; 608 of 224 columns
+// are 4 rounds to the tile (a call of K = 4096 117 -> 105 us, with elect_one; 8192 x 8192 unchanged).  A
+// product of one round takes narrower tiles on more SMs (512 x 4096 x 4096: 47 -> 41 us).
+template <int BN>
+uint32_t tile_width(const GemmArgs& g, uint32_t splits, uint64_t resident) {
+    if (BN < 256) return BN;
+    const uint64_t rows = (uint64_t)((g.M + kBM - 1) / kBM) * splits;
+    uint32_t best = BN;
+    uint64_t least = ~0ull;
+    for (uint32_t bn = BN; bn >= 64; bn -= 16) {
+        const uint64_t tiles = rows * ((g.N + bn - 1) / bn), rounds = (tiles + resident - 1) / resident;
+        const uint64_t cost = rounds * (std::max(bn, 64 + bn / 2) + 24);
+        if (cost < least) {
+            least = cost;
+            best = bn;
+        }
+    }
+    return best;
+}
+
 // false (nothing launched) when a tensor map cannot be encoded for these operands
 template <int BN>
 bool launch_tma_bn(const GemmArgs& g, uint32_t splits, cudaStream_t st, cudaError_t* err) {
-    CUtensorMap ta, tb;
-    if (!encode_operand(&ta, g.A, g.K, g.M, g.lda, kBM) || !encode_operand(&tb, g.B, g.K, g.N, g.ldb, BN)) return false;
     const size_t smem = tma_smem<BN>();
     *err = cudaFuncSetAttribute(umma_gemm_tma_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (*err != cudaSuccess) return true;
@@ -501,12 +522,15 @@ bool launch_tma_bn(const GemmArgs& g, uint32_t splits, cudaStream_t st, cudaErro
     int dev = 0, sms = 0;
     if ((*err = cudaGetDevice(&dev)) != cudaSuccess) return true;
     if ((*err = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return true;
+    const uint64_t resident = (uint64_t)std::max(1, sms * std::max(1, per_sm));
+    const uint32_t bn = tile_width<BN>(g, splits, resident);
+    CUtensorMap ta, tb;
+    if (!encode_operand(&ta, g.A, g.K, g.M, g.lda, kBM) || !encode_operand(&tb, g.B, g.K, g.N, g.ldb, bn)) return false;
     // fewer than two rounds of tiles: one CTA per tile, so a second-round tile goes to whichever SM
     // frees first rather than to a fixed CTA
-    const uint64_t tiles = (uint64_t)((g.M + kBM - 1) / kBM) * ((g.N + BN - 1) / BN) * splits;
-    const uint64_t resident = (uint64_t)std::max(1, sms * std::max(1, per_sm));
+    const uint64_t tiles = (uint64_t)((g.M + kBM - 1) / kBM) * ((g.N + bn - 1) / bn) * splits;
     const uint32_t grid = (uint32_t)(tiles < 2 * resident ? tiles : resident);
-    umma_gemm_tma_kernel<BN><<<grid, kTmaThreads, smem, st>>>(ta, tb, g, splits);
+    umma_gemm_tma_kernel<BN><<<grid, kTmaThreads, smem, st>>>(ta, tb, g, splits, bn);
     *err = cudaGetLastError();
     return true;
 }
