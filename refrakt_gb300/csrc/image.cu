@@ -33,16 +33,20 @@ struct DeTables {
     double wsum[101];    // the weights of a whole disc of radius r, summed in FP64
 };
 
-// the weights of radii up to kDeMaxSmemR, a kernel parameter: no upload per call
-constexpr int kSmemWeights = (kDeMaxSmemR + 1) * (kDeMaxSmemR + 2) * (2 * kDeMaxSmemR + 3) / 6;
-struct DeWeights {
-    float w[kSmemWeights];
+// the weight coefficients (de_weight_params) of radii up to kDeMaxSmemR
+struct DeSmallParams {
+    float4 r[kDeMaxSmemR + 1];
 };
 
 __device__ __forceinline__ int de_radius(float a, const DeTables& T) {
     int r;
     if (T.mode == 2) r = T.R;
-    else {
+    else if (T.R <= 16) {
+        // thresholds are monotone: the number that hold.  Every lane reads the same threshold; the search below
+        // reads another one per lane, which the constant cache serves one after another
+        r = 0;
+        for (int k = 0; k < T.R; k++) r += (T.mode == 0 ? a <= T.thr[k] : a >= T.thr[k]) ? 1 : 0;
+    } else {
         // thresholds are monotone: binary search for the largest k with the condition true
         int lo = 0, hi = T.R;
         while (lo < hi) {
@@ -55,11 +59,27 @@ __device__ __forceinline__ int de_radius(float a, const DeTables& T) {
     return r > T.min_r ? r : T.min_r;  // max(min, min(R, int(R / a^curve))), density_vert.glsl:35-44
 }
 
+// The densities of a thread's next kAhead bins, loaded together: with one load in flight per thread the passes
+// over all bins are bound by memory latency (8.3 M bins: the radii 31 -> 27 us, the statistics 62 -> 43, also for
+// want of FP64 rate; 20 us at the copy bandwidth).
+constexpr int kAhead = 4;
+__device__ __forceinline__ void load_densities(const float4* __restrict__ in, size_t i, size_t stride, size_t n,
+                                               float (&a)[kAhead]) {
+#pragma unroll
+    for (int u = 0; u < kAhead; u++) a[u] = i + u * stride < n ? in[i + u * stride].w : 0.0f;
+}
+
 // pass 1: radius per bin (255 = empty)
-__global__ void de_radius_kernel(const float4* __restrict__ in, size_t n, const DeTables T, uint8_t* __restrict__ rad) {
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const float a = in[i].w;
-        rad[i] = (a == 0.0f || a != a) ? (uint8_t)255 : (uint8_t)de_radius(a, T);
+__global__ void de_radius_kernel(const float4* __restrict__ in, size_t n, const __grid_constant__ DeTables T,
+                                 uint8_t* __restrict__ rad) {
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += kAhead * stride) {
+        float a[kAhead];
+        load_densities(in, i, stride, n, a);
+#pragma unroll
+        for (int u = 0; u < kAhead; u++)
+            if (i + u * stride < n)
+                rad[i + u * stride] = (a[u] == 0.0f || a[u] != a[u]) ? (uint8_t)255 : (uint8_t)de_radius(a[u], T);
     }
 }
 
@@ -82,14 +102,18 @@ __device__ __forceinline__ void block_sum_to(double s, double* out) {
 // log-density scale's sum (k2 = W * H / sum a) without a pass over the output.  A whole disc's
 // weights come from T.wsum; a disc cut by the grid's edge adds, per row inside the grid,
 // the difference of two prefix sums of that row's FP32 weights, staged per CTA in shared memory
-// for every radius up to kDeMaxSmemR (the fused path's radii).
+// for every radius up to kDeMaxSmemR (the fused path's radii), from the weights' coefficients: reading the table
+// from a kernel parameter, a lane at a time, took a third of the pass on small grids (512 x 512: 13 -> 9 us;
+// 3840 x 2160 45 us, bound by the instructions per bin).
 constexpr int kRowPrefixFloats = 1638;  // sum over r <= 12 of (r + 1) rows of 2r + 2 prefix sums
 
 __global__ void de_radius_sum_kernel(const float4* __restrict__ in, uint32_t w, uint32_t h, const __grid_constant__ DeTables T,
-                                     const __grid_constant__ DeWeights W, uint8_t* __restrict__ rad,
+                                     const __grid_constant__ DeSmallParams P, uint8_t* __restrict__ rad,
                                      double* __restrict__ sum_out) {
     __shared__ float s_pre[kRowPrefixFloats];
     __shared__ int s_pbase[kDeMaxSmemR + 1];
+    __shared__ float4 s_par[kDeMaxSmemR + 1];
+    if (threadIdx.x <= kDeMaxSmemR) s_par[threadIdx.x] = P.r[threadIdx.x];
     const int rmax = min(kDeMaxSmemR, T.R > T.min_r ? T.R : T.min_r);
     if (threadIdx.x == 0) {
         int off = 0;
@@ -104,11 +128,13 @@ __global__ void de_radius_sum_kernel(const float4* __restrict__ in, uint32_t w, 
         const int r = q / (rmax + 1), ay = q % (rmax + 1);
         if (r < 1 || ay > r) continue;
         float* pre = s_pre + s_pbase[r] + ay * (2 * r + 2);
+        const float4 c = s_par[r];
+        const float ny2 = -(float)(ay * ay);
         float acc = 0.0f;
         pre[0] = 0.0f;
-        for (int dx = -r; dx <= r; dx++) {
-            const int ax = dx < 0 ? -dx : dx;
-            if (4 * (ax * ax + ay * ay) <= (2 * r + 1) * (2 * r + 1)) acc += W.w[T.wbase[r] + ay * (r + 1) + ax];
+        for (int dx = -r; dx <= r; dx++) {  // the table's weights as the sweep computes them (de_add)
+            const float nx2 = -(float)(dx * dx);
+            acc += fmaxf(fmaf(ny2, c.y, fmaf(nx2, c.y, c.x)) + fmaf(ny2, c.w, fmaf(nx2, c.w, c.z)), 0.0f);
             pre[dx + r + 1] = acc;
         }
     }
@@ -120,15 +146,19 @@ __global__ void de_radius_sum_kernel(const float4* __restrict__ in, uint32_t w, 
     __syncthreads();
     const uint32_t n = w * h;  // < 2^32 (the caller's grids hold fewer bins)
     float s = 0.0f;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float a = in[i].w;
+    const size_t stride = (size_t)gridDim.x * blockDim.x, first = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    float ahead[2] = {first < n ? in[first].w : 0.0f, first + stride < n ? in[first + stride].w : 0.0f};  // the next two
+    for (size_t i = first; i < n; i += stride) {
+        const float a = ahead[0];
+        ahead[0] = ahead[1];
+        ahead[1] = i + 2 * stride < n ? in[i + 2 * stride].w : 0.0f;
         if (a == 0.0f || a != a) {
             rad[i] = 255;
             continue;
         }
         const int r = de_radius(a, T);
         rad[i] = (uint8_t)r;
-        const int y = (int)(i / w), x = (int)(i - (uint32_t)y * w);
+        const int y = (int)((uint32_t)i / w), x = (int)((uint32_t)i - (uint32_t)y * w);
         if (x >= r && y >= r && x + r < (int)w && y + r < (int)h) {  // the whole disc (r = 0: weight 1)
             s = fmaf(a, s_wsum[r], s);
             continue;
@@ -597,14 +627,23 @@ __global__ void de_gather_global_kernel(const float4* __restrict__ in, const uin
 
 // FP64 sum and max of the density channel, count of non-empty bins
 __global__ void stats_kernel(const float4* __restrict__ in, size_t n, double* out) {
-    double s = 0.0, m = 0.0;
-    unsigned long long nz = 0;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-        const double a = (double)in[i].w;
-        s += a;
-        m = a > m ? a : m;
-        nz += (a > 0.0) ? 1 : 0;
+    // (the maximum and the count in FP32 and 32 bits, the sum alone at this part's low FP64 rate)
+    double s = 0.0;
+    float top = 0.0f;
+    uint32_t count = 0;
+    const size_t stride = (size_t)gridDim.x * blockDim.x;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += kAhead * stride) {
+        float a[kAhead];
+        load_densities(in, i, stride, n, a);
+#pragma unroll
+        for (int u = 0; u < kAhead; u++) {
+            s += (double)a[u];
+            top = a[u] > top ? a[u] : top;
+            count += a[u] > 0.0f ? 1u : 0u;
+        }
     }
+    double m = (double)top;
+    unsigned long long nz = count;
     for (int o = 16; o > 0; o >>= 1) {
         s += __shfl_down_sync(0xffffffffu, s, o);
         m = fmax(m, __shfl_down_sync(0xffffffffu, m, o));
@@ -652,54 +691,87 @@ __global__ void tonemap_kernel(const float4* __restrict__ in, uint32_t w, uint32
 // reference, which ignores flam3's filter and filter_shape, flame.cpp:166-176): output pixel
 // (ox, oy) is the weighted sum, by the separable taps c[i] c[j], of the log-scaled bins of the
 // fwidth x fwidth window starting at (ox ss - pad, oy ss - pad), pad = (fwidth - ss) / 2, then
-// tonemap_finish.  A CTA stages the log-scaled bins of its tile's windows once in shared memory.
+// tonemap_finish.  A CTA stages the log-scaled bins of its tile's windows once in shared memory, sums each of
+// their rows along x once per output column, then the rows of each output pixel: 6 + 6 rows' worth of
+// shared-memory reads per pixel at ss = 2 and 6 taps instead of 36.  A row's bins are stored by their column
+// modulo ss (up to 8), so that a warp's neighbouring pixels read neighbouring 16 bytes.  3840 x 2160 bins to 1920 x
+// 1080: 139 -> 106 us (25 us at the copy bandwidth; bound by the instructions of every bin's log scale).
 struct FilterArgs {
     int fwidth, pad;
-    int tw, th;        // output pixels per CTA tile
+    int tw, th;        // output pixels per CTA tile (tw a power of two)
     float taps[kMaxFilterTaps];
 };
+struct FilterTile {
+    int rw, rh, mod, cols;  // bins of the tile's windows; columns of one residue modulo mod
+    __host__ __device__ FilterTile(const FilterArgs& F, int ss)
+        : rw(F.tw * ss + F.fwidth - ss), rh(F.th * ss + F.fwidth - ss), mod(ss <= 8 ? ss : 1), cols((rw + mod - 1) / mod) {}
+    __host__ __device__ size_t bytes(const FilterArgs& F) const { return ((size_t)rh * mod * cols + (size_t)rh * F.tw) * 16; }
+};
+constexpr size_t kFilterSmem = 200 * 1024;
 
 __global__ void __launch_bounds__(256) tonemap_filter_kernel(const float4* __restrict__ in, uint32_t w, uint32_t h,
-                                                             uint32_t ss, float gamma, float brightness,
+                                                             uint32_t ss_, float gamma, float brightness,
                                                              float vibrancy, float k2, const double* __restrict__ stats,
-                                                             const FilterArgs F, float4* __restrict__ out_f32,
-                                                             uchar4* __restrict__ out8) {
+                                                             const __grid_constant__ FilterArgs F,
+                                                             float4* __restrict__ out_f32, uchar4* __restrict__ out8) {
     extern __shared__ __align__(16) unsigned char smem[];
-    float4* s_l = reinterpret_cast<float4*>(smem);
-    const int rw = F.tw * (int)ss + F.fwidth - (int)ss, rh = F.th * (int)ss + F.fwidth - (int)ss;
+    const int ss = (int)ss_;
+    const FilterTile t(F, ss);
+    float4* s_l = reinterpret_cast<float4*>(smem);      // [row][column % mod][column / mod]
+    float4* s_r = s_l + (size_t)t.rh * t.mod * t.cols;  // [row][output column]
     const int ox0 = blockIdx.x * F.tw, oy0 = blockIdx.y * F.th;
-    const int gx0 = ox0 * (int)ss - F.pad, gy0 = oy0 * (int)ss - F.pad;
+    const int gx0 = ox0 * ss - F.pad, gy0 = oy0 * ss - F.pad;
     const float k = tonemap_scale(k2, stats, w, h);
-    for (int i = threadIdx.x; i < rw * rh; i += blockDim.x) {
-        const int gx = gx0 + i % rw, gy = gy0 + i / rw;
-        float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (gx >= 0 && gy >= 0 && gx < (int)w && gy < (int)h) {
-            const float4 c = in[(size_t)gy * w + gx];
-            if (c.w > 0.0f) {
-                const float ls = tonemap_log_scale(c.w, k, brightness);
-                v = make_float4(c.x * ls, c.y * ls, c.z * ls, c.w * ls);
+    constexpr int kLoads = 3;  // rows of a warp at a time: one after another they take as many latencies more
+    for (int x = threadIdx.x & 31; x < t.rw; x += 32) {
+        const int gx = gx0 + x, col = x / t.mod;
+        const bool in_x = gx >= 0 && gx < (int)w;
+        float4* dst = s_l + (x - col * t.mod) * t.cols + col;
+        for (int y0 = threadIdx.x >> 5; y0 < t.rh; y0 += 8 * kLoads) {
+            float4 c[kLoads];
+#pragma unroll
+            for (int u = 0; u < kLoads; u++) {
+                const int y = y0 + 8 * u, gy = gy0 + y;
+                c[u] = in_x && y < t.rh && gy >= 0 && gy < (int)h ? in[(size_t)gy * w + gx] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+#pragma unroll
+            for (int u = 0; u < kLoads; u++) {
+                if (y0 + 8 * u >= t.rh) break;
+                float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (c[u].w > 0.0f) {
+                    const float ls = tonemap_log_scale(c[u].w, k, brightness);
+                    v = make_float4(c[u].x * ls, c[u].y * ls, c[u].z * ls, c[u].w * ls);
+                }
+                dst[(y0 + 8 * u) * t.mod * t.cols] = v;
             }
         }
-        s_l[i] = v;
     }
     __syncthreads();
-    const uint32_t ow = w / ss, oh = h / ss;
-    for (int p = threadIdx.x; p < F.tw * F.th; p += blockDim.x) {
-        const int px = p % F.tw, py = p / F.tw;
-        const uint32_t ox = ox0 + px, oy = oy0 + py;
-        if (ox >= ow || oy >= oh) continue;
-        float4 acc = make_float4(0, 0, 0, 0);
-        for (int j = 0; j < F.fwidth; j++) {
-            const float4* row = s_l + (size_t)(py * (int)ss + j) * rw + px * (int)ss;
-            float4 r = make_float4(0, 0, 0, 0);
-            for (int i = 0; i < F.fwidth; i++) {
-                const float4 v = row[i];
+    // tw divides 256: a thread keeps its column
+    const int px = (int)threadIdx.x & (F.tw - 1), step = 256 / F.tw;
+    const float4* column = s_l + (t.mod == ss ? px : px * ss);
+    for (int y = (int)threadIdx.x / F.tw; y < t.rh; y += step) {
+        float4 r = make_float4(0, 0, 0, 0);
+        const float4* at = column + (size_t)y * t.mod * t.cols;
+        for (int i = 0; i < F.fwidth; at++)  // one bin of each residue after the other, then the next column
+            for (int res = 0; res < t.mod && i < F.fwidth; res++, i++) {
+                const float4 v = at[res * t.cols];
                 const float c = F.taps[i];
                 r.x = fmaf(v.x, c, r.x);
                 r.y = fmaf(v.y, c, r.y);
                 r.z = fmaf(v.z, c, r.z);
                 r.w = fmaf(v.w, c, r.w);
             }
+        s_r[y * F.tw + px] = r;
+    }
+    __syncthreads();
+    const uint32_t ow = w / ss_, oh = h / ss_;
+    for (int py = (int)threadIdx.x / F.tw; py < F.th; py += step) {
+        const uint32_t ox = ox0 + px, oy = oy0 + py;
+        if (ox >= ow || oy >= oh) continue;
+        float4 acc = make_float4(0, 0, 0, 0);
+        for (int j = 0; j < F.fwidth; j++) {
+            const float4 r = s_r[(py * ss + j) * F.tw + px];
             const float c = F.taps[j];
             acc.x = fmaf(r.x, c, acc.x);
             acc.y = fmaf(r.y, c, acc.y);
@@ -754,17 +826,21 @@ cudaError_t launch_tonemap_filter(const float4* in, uint32_t w, uint32_t h, uint
     F.fwidth = filter_taps(ss, radius, shape, F.taps);
     if (F.fwidth < 0) return cudaErrorInvalidValue;
     F.pad = (F.fwidth - (int)ss) / 2;
-    // the largest tile whose staged windows fit in 96 KB of shared memory
+    // the largest tile whose staged windows and row sums fit in 64 KB of shared memory (three CTAs an SM), else
+    // in all of it
     static const int tiles[][2] = {{32, 8}, {16, 8}, {8, 8}, {8, 4}, {4, 4}, {2, 2}, {1, 1}};
     size_t smem = 0;
-    for (const auto& t : tiles) {
-        F.tw = t[0];
-        F.th = t[1];
-        smem = (size_t)(F.tw * ss + F.fwidth - ss) * (F.th * ss + F.fwidth - ss) * sizeof(float4);
-        if (smem <= 96 * 1024) break;
+    for (const size_t limit : {(size_t)64 * 1024, kFilterSmem}) {
+        for (const auto& t : tiles) {
+            F.tw = t[0];
+            F.th = t[1];
+            smem = FilterTile(F, (int)ss).bytes(F);
+            if (smem <= limit) break;
+        }
+        if (smem <= limit) break;
     }
-    if (smem > 96 * 1024) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(tonemap_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+    if (smem > kFilterSmem) return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(tonemap_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kFilterSmem);
     if (e != cudaSuccess) return e;
     const uint32_t ow = w / ss, oh = h / ss;
     const dim3 grid((ow + F.tw - 1) / F.tw, (oh + F.th - 1) / F.th);
@@ -895,9 +971,11 @@ cudaError_t launch_density_tonemap(const float4* in, uint32_t w, uint32_t h, int
     if (need_sum) {
         e = cudaMemsetAsync(stats, 0, 3 * sizeof(double), st);
         if (e != cudaSuccess) return e;
-        DeWeights W;
-        std::copy(wts.begin(), wts.end(), W.w);  // at most kSmemWeights of them
-        de_radius_sum_kernel<<<1024, 256, 0, st>>>(in, w, h, T, W, rad, stats);
+        DeParams P{};
+        DeSmallParams S;
+        de_weight_params(kDeMaxSmemR, P);
+        std::copy(P.r, P.r + kDeMaxSmemR + 1, S.r);
+        de_radius_sum_kernel<<<1024, 256, 0, st>>>(in, w, h, T, S, rad, stats);
     } else {
         de_radius_kernel<<<1024, 256, 0, st>>>(in, (size_t)w * h, T, rad);
     }
