@@ -399,12 +399,14 @@ bool reserve_lists(rf_sim* s, size_t nb, uint32_t passes) {
     if (4 * cap * ranges < 5 * points || chaos_smem(s->slots, s->prog_words, s->L, 0, 1, ranges) > kMaxCtaSmem) return false;
     const size_t bytes = head + ctas * ranges * cap * 8;
     if (s->lists_bytes < bytes) {
+        if (bytes >= s->lists_refused) return false;
         cudaFree(s->lists);
         s->lists = nullptr;
         s->lists_bytes = 0;
         if (cudaMalloc((void**)&s->lists, bytes) != cudaSuccess ||
             cudaMemsetAsync(s->lists, 0, kListScratch, s->stream) != cudaSuccess) {
             cudaGetLastError();
+            s->lists_refused = bytes;
             return false;
         }
         s->lists_bytes = bytes;

@@ -72,7 +72,7 @@ struct rf_sim {
     // the list splat's memory: scratch planes of one range (all zero between calls), then the counts and the
     // lists of list_ctas x list_ranges x list_cap entries; list_ranges 0: the next launches have none
     unsigned char* lists = nullptr;
-    size_t lists_bytes = 0;
+    size_t lists_bytes = 0, lists_refused = ~(size_t)0;  // refused: a size the device had no memory for
     uint32_t list_ranges = 0, list_range_bits = 0, list_cap = 0;
     // after the first list call of a genome and grid (pinned, zero until they have arrived): the hits of the
     // hottest bin, of all bins, and the points of the call that found their list full; those points' number
