@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <type_traits>
 #include <vector>
 
 #include "kernels.h"
@@ -59,28 +60,38 @@ __device__ __forceinline__ int de_radius(float a, const DeTables& T) {
     return r > T.min_r ? r : T.min_r;  // max(min, min(R, int(R / a^curve))), density_vert.glsl:35-44
 }
 
-// The densities of a thread's next kAhead bins, loaded together: with one load in flight per thread the passes
+// The densities of a thread's next AHEAD bins, loaded together: with one load in flight per thread the passes
 // over all bins are bound by memory latency (8.3 M bins: the radii 31 -> 27 us, the statistics 62 -> 43, also for
-// want of FP64 rate; 20 us at the copy bandwidth).
-constexpr int kAhead = 4;
+// want of FP64 rate; 20 us at the copy bandwidth).  Below kAheadBins a thread has few bins or one: 1.
+constexpr size_t kAheadBins = 1u << 20;
+template <int AHEAD>
 __device__ __forceinline__ void load_densities(const float4* __restrict__ in, size_t i, size_t stride, size_t n,
-                                               float (&a)[kAhead]) {
+                                               float (&a)[AHEAD]) {
 #pragma unroll
-    for (int u = 0; u < kAhead; u++) a[u] = i + u * stride < n ? in[i + u * stride].w : 0.0f;
+    for (int u = 0; u < AHEAD; u++) a[u] = i + u * stride < n ? in[i + u * stride].w : 0.0f;
 }
 
+// CTAs of 256 threads for a pass over n bins
+static unsigned pass_ctas(size_t n) { return (unsigned)std::min<size_t>(1024, (n + 255) / 256); }
+
 // pass 1: radius per bin (255 = empty)
+template <int AHEAD>
 __global__ void de_radius_kernel(const float4* __restrict__ in, size_t n, const __grid_constant__ DeTables T,
                                  uint8_t* __restrict__ rad) {
     const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += kAhead * stride) {
-        float a[kAhead];
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += AHEAD * stride) {
+        float a[AHEAD];
         load_densities(in, i, stride, n, a);
 #pragma unroll
-        for (int u = 0; u < kAhead; u++)
+        for (int u = 0; u < AHEAD; u++)
             if (i + u * stride < n)
                 rad[i + u * stride] = (a[u] == 0.0f || a[u] != a[u]) ? (uint8_t)255 : (uint8_t)de_radius(a[u], T);
     }
+}
+
+static void launch_radius(const float4* in, size_t n, const DeTables& T, uint8_t* rad, cudaStream_t st) {
+    if (n >= kAheadBins) de_radius_kernel<4><<<pass_ctas(n), 256, 0, st>>>(in, n, T, rad);
+    else de_radius_kernel<1><<<pass_ctas(n), 256, 0, st>>>(in, n, T, rad);
 }
 
 // block-wide FP64 sum, added to *out by one thread per block (blockDim.x a multiple of 32, <= 1024)
@@ -267,6 +278,9 @@ struct DeParams {
     float4 r[kDeMaxSweepR + 1];
 };
 
+template <bool WHOLE>
+using DeParamsFor = std::conditional_t<WHOLE, DeSmallParams, DeParams>;  // as few parameter bytes per launch as it takes
+
 // the tonemap a DE kernel applies to its own output (TM = true)
 struct TmArgs {
     uint32_t ss;
@@ -421,7 +435,7 @@ __host__ __device__ constexpr size_t de_smem_bytes(int rows, int R, bool whole) 
 // memory (over the staging) and are tonemapped there.
 template <bool WHOLE, bool TM, int ROWS>
 __global__ void __launch_bounds__(kDeThreads, 3) de_sweep_kernel(const float4* __restrict__ in, const uint8_t* __restrict__ rad,
-                                                                 uint32_t w, uint32_t h, int R, const __grid_constant__ DeParams P,
+                                                                 uint32_t w, uint32_t h, int R, const __grid_constant__ DeParamsFor<WHOLE> P,
                                                                  float4* __restrict__ out, const TmArgs tm) {
     extern __shared__ __align__(16) unsigned char smem[];
     constexpr int cta_rows = 4 * ROWS;
@@ -444,13 +458,18 @@ __global__ void __launch_bounds__(kDeThreads, 3) de_sweep_kernel(const float4* _
 #pragma unroll
         for (int c = 0; c < 4; c++) acc.v[q][c] = 0;
     if constexpr (WHOLE) {
+        // the warps whose outputs lie in one 32 x 8 tile look through its discs together (2 rows per warp, the
+        // image of 522 x 290 bins at radius 5: 34.8 -> 33.0 us a call)
+        constexpr int kShare = kTileH / ROWS, kTiles = 8 / kShare;
+        __shared__ int s_tile[2][kTiles];  // the largest radius, the number of discs of radius >= 2
+        if (kShare > 1 && threadIdx.x < 2 * kTiles) (&s_tile[0][0])[threadIdx.x] = 0;
         de_stage(in, rad, (int)w, (int)h, tx0 - R, ty0 - R, pitch, 0, all, s_c, s_r);
         __syncthreads();
         // of the discs that reach the warp's 32 x 8 tile: the largest radius, and the number of those of
         // radius >= 2
         int rmax = 0, big = 0;
         const uint8_t* tr = s_r + (y0 & ~(kTileH - 1)) * pitch + x0;
-        for (int i = 0; i < kTileH + 2 * R; i++) {
+        for (int i = (warp >> 1) % kShare; i < kTileH + 2 * R; i += kShare) {
             const int dy = i - R, md = dy < 0 ? -dy : (dy > kTileH - 1 ? dy - (kTileH - 1) : 0);
             for (int x = lane; x < kTileW + 2 * R; x += 32) {
                 const int r = (int)tr[i * pitch + x] - 1, dx = x - R;
@@ -461,6 +480,16 @@ __global__ void __launch_bounds__(kDeThreads, 3) de_sweep_kernel(const float4* _
         }
         rmax = __reduce_max_sync(0xffffffffu, rmax);
         big = __reduce_add_sync(0xffffffffu, big);
+        if (kShare > 1) {
+            const int t = ((warp >> 1) / kShare) * 2 + (warp & 1);
+            if (lane == 0) {
+                atomicMax(&s_tile[0][t], rmax);
+                atomicAdd(&s_tile[1][t], big);
+            }
+            __syncthreads();
+            rmax = s_tile[0][t];
+            big = s_tile[1][t];
+        }
         const float4* wc = s_c + y0 * pitch + x0;  // the warp's window
         const uint8_t* wr = s_r + y0 * pitch + x0;
         const bool small_first = 9 + big < (2 * rmax + 1) * (2 * rmax + 1);
@@ -566,10 +595,12 @@ template <int ROWS>
 static cudaError_t launch_de_rows(int R, const DeParams& P, const float4* in, const uint8_t* rad, uint32_t w, uint32_t h,
                                   float4* out, cudaStream_t st, const TmArgs* tm) {
     const bool whole = R <= kDeMaxSmemR;
+    DeSmallParams S;
+    std::copy(P.r, P.r + kDeMaxSmemR + 1, S.r);
     const dim3 grid((w + kCtaW - 1) / kCtaW, (h + 4 * ROWS - 1) / (4 * ROWS));
     const size_t smem = de_smem_bytes(ROWS, R, whole);  // (a fused CTA's outputs fit in its staging)
-    if (tm) de_sweep_kernel<true, true, ROWS><<<grid, kDeThreads, smem, st>>>(in, rad, w, h, R, P, out, *tm);
-    else if (whole) de_sweep_kernel<true, false, ROWS><<<grid, kDeThreads, smem, st>>>(in, rad, w, h, R, P, out, TmArgs{});
+    if (tm) de_sweep_kernel<true, true, ROWS><<<grid, kDeThreads, smem, st>>>(in, rad, w, h, R, S, out, *tm);
+    else if (whole) de_sweep_kernel<true, false, ROWS><<<grid, kDeThreads, smem, st>>>(in, rad, w, h, R, S, out, TmArgs{});
     else de_sweep_kernel<false, false, ROWS><<<grid, kDeThreads, smem, st>>>(in, rad, w, h, R, P, out, TmArgs{});
     return cudaGetLastError();
 }
@@ -582,7 +613,7 @@ static cudaError_t launch_de_sweep(int R, const float4* in, const uint8_t* rad, 
                                    cudaStream_t st, const TmArgs* tm = nullptr) {
     cudaError_t e = density_prepare();
     if (e != cudaSuccess) return e;
-    DeParams P;
+    DeParams P{};
     de_weight_params(R, P);
     const auto ctas = [&](uint32_t rows) { return (uint64_t)((w + kCtaW - 1) / kCtaW) * ((h + 4 * rows - 1) / (4 * rows)); };
     if (ctas(8) >= 12 * 152) return launch_de_rows<8>(R, P, in, rad, w, h, out, st, tm);
@@ -626,17 +657,18 @@ __global__ void de_gather_global_kernel(const float4* __restrict__ in, const uin
 }
 
 // FP64 sum and max of the density channel, count of non-empty bins
+template <int AHEAD>
 __global__ void stats_kernel(const float4* __restrict__ in, size_t n, double* out) {
     // (the maximum and the count in FP32 and 32 bits, the sum alone at this part's low FP64 rate)
     double s = 0.0;
     float top = 0.0f;
     uint32_t count = 0;
     const size_t stride = (size_t)gridDim.x * blockDim.x;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += kAhead * stride) {
-        float a[kAhead];
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += AHEAD * stride) {
+        float a[AHEAD];
         load_densities(in, i, stride, n, a);
 #pragma unroll
-        for (int u = 0; u < kAhead; u++) {
+        for (int u = 0; u < AHEAD; u++) {
             s += (double)a[u];
             top = a[u] > top ? a[u] : top;
             count += a[u] > 0.0f ? 1u : 0u;
@@ -929,7 +961,7 @@ size_t density_weight_count(int R, int min_r) {
 static cudaError_t launch_density_passes(const float4* in, uint32_t w, uint32_t h, const DeTables& T, float4* out,
                                          uint8_t* rad, const float* dw, cudaStream_t st) {
     const size_t n = (size_t)w * h;
-    de_radius_kernel<<<1024, 256, 0, st>>>(in, n, T, rad);
+    launch_radius(in, n, T, rad, st);
     const int rmax = T.R > T.min_r ? T.R : T.min_r;
     if (rmax <= kDeMaxSweepR) return launch_de_sweep(rmax, in, rad, w, h, out, st);
     de_gather_global_kernel<<<dim3((w + 127) / 128, h), 128, 0, st>>>(in, rad, w, h, dw, T, out);
@@ -977,7 +1009,7 @@ cudaError_t launch_density_tonemap(const float4* in, uint32_t w, uint32_t h, int
         std::copy(P.r, P.r + kDeMaxSmemR + 1, S.r);
         de_radius_sum_kernel<<<1024, 256, 0, st>>>(in, w, h, T, S, rad, stats);
     } else {
-        de_radius_kernel<<<1024, 256, 0, st>>>(in, (size_t)w * h, T, rad);
+        launch_radius(in, (size_t)w * h, T, rad, st);
     }
     const TmArgs tm{ss, gamma, brightness, vibrancy, k2, need_sum ? stats : nullptr, out_f32, out8};
     return launch_de_sweep(R > min_r ? R : min_r, in, rad, w, h, nullptr, st, &tm);
@@ -1000,7 +1032,9 @@ cudaError_t launch_density_resident(const float4* in, uint32_t w, uint32_t h, in
 cudaError_t launch_stats(const float4* in, uint32_t w, uint32_t h, double* out3, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(out3, 0, 3 * sizeof(double), st);
     if (e != cudaSuccess) return e;
-    stats_kernel<<<1024, 256, 0, st>>>(in, (size_t)w * h, out3);
+    const size_t n = (size_t)w * h;
+    if (n >= kAheadBins) stats_kernel<4><<<1024, 256, 0, st>>>(in, n, out3);
+    else stats_kernel<1><<<1024, 256, 0, st>>>(in, n, out3);
     return cudaGetLastError();
 }
 
