@@ -482,7 +482,7 @@ def run_native(args):
         # pass, then the tiles) plus a radius byte per bin, and never write the estimator's output
         tail_bytes = W * H * 16 + W_OUT * H_OUT * 4
         peak_, _ = _peaks()
-        image_passes = {"kernels": "de_radius_sum_kernel + de_tile_kernel<9, tonemap>" if DE else
+        image_passes = {"kernels": "de_radius_sum_kernel + de_sweep_kernel (tonemap)" if DE else
                                    "stats_kernel + tonemap_kernel",
                         "ms": tail_ms, "algorithmic_bytes": tail_bytes,
                         "gbs": tail_bytes / (tail_ms * 1e-3) / 1e9 if tail_ms > 0 else None, "peak_gbs": peak_}
