@@ -510,7 +510,8 @@ class Sim:
     def set_exchange(self, mode):
         """Walker exchange of the specialised chaos kernel (rf_set_exchange): EXCHANGE_BARRIER,
         EXCHANGE_PIPELINED or EXCHANGE_AUTO (default: the faster of the two, timed on the first
-        two drawing launches of >= 32 passes); every form gives the same results."""
+        two drawing launches of >= 32 passes; a simulation of fewer mixing domains than SMs
+        spreads each over a thread-block cluster); every form gives the same results."""
         _check(library().rf_set_exchange(self._h, int(mode)))
 
     def exchange(self):

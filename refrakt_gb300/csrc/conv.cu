@@ -24,7 +24,7 @@
 // Bound: the copies' shared-memory writes, a wavefront per 16 bytes (72 copies of 41 wavefronts per tile
 // of 80 channels, of its 2,930 cycles; the 45 MMAs' operand reads, 40 wavefronts each, take 1,800).
 // Measured, bf16, one call: 48 upsampled + 32 channels to 32 at 1920 x 1080 885 us as a gathered im2col
-// GEMM, 201 us here; 32 to 32 at 16 x 256 x 256 (the kernel) 238 -> 59 us.
+// GEMM, 192 us here; 32 to 32 at 16 x 256 x 256 (the kernel) 238 -> 59 us.
 #include <algorithm>
 
 #include <cuda_bf16.h>
