@@ -497,9 +497,11 @@ __global__ void __launch_bounds__(kDeThreads, 3) de_sweep_kernel(const float4* _
             for (int i = max(0, R - 1); i < min(ROWS + R + 1, ROWS + 2 * R); i++)
                 de_row<ROWS, 2, kSmall>(acc, wc + i * pitch, wr + i * pitch, s_p, R, i - R);
             if (big)
-                for (int i = 0; i < ROWS + 2 * R; i++) de_row<ROWS, 2, kLarge>(acc, wc + i * pitch, wr + i * pitch, s_p, R, i - R);
+                for (int i = R - rmax; i < ROWS + R + rmax; i++)
+                    de_row<ROWS, 2, kLarge>(acc, wc + i * pitch, wr + i * pitch, s_p, R, i - R);
         } else {
-            for (int i = 0; i < ROWS + 2 * R; i++) de_row<ROWS, 2, kAll>(acc, wc + i * pitch, wr + i * pitch, s_p, R, i - R);
+            for (int i = R - rmax; i < ROWS + R + rmax; i++)
+                de_row<ROWS, 2, kAll>(acc, wc + i * pitch, wr + i * pitch, s_p, R, i - R);
         }
         __syncthreads();
     } else {
