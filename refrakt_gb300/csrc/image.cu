@@ -21,6 +21,7 @@
 
 #include "kernels.h"
 #include "scratch.h"
+#include "umma.cuh"
 
 namespace rfk {
 
@@ -266,8 +267,8 @@ __device__ __forceinline__ uchar4 to_rgba8(float4 o) {
 //
 // Bound: instruction issue (62 % of the slots at 24 warps per SM; about 70 instructions per source and
 // 8 outputs).  Density estimation of 3840 x 2160 bins at 1000 points per bin: 990 us as one output per
-// thread over the box of the tile's largest radius, 642 here; 960 x 540 at radius 20 1,090 us as a gather
-// from global memory, 344 here.
+// thread over the box of the tile's largest radius, 598 here; 960 x 540 at radius 20 1,090 us as a gather
+// from global memory, 330 here.
 constexpr int kTileW = 32, kTileH = 8;     // the tile whose discs set the order of its sums
 constexpr int kDeThreads = 256;
 constexpr int kCtaW = 2 * kTileW;          // a CTA: 8 warps, two side by side, each 32 x ROWS outputs
@@ -403,26 +404,37 @@ __device__ __forceinline__ void de_row(DeAcc<ROWS>& acc, const float4* s_c, cons
     }
 }
 
-// staged rows [row0, row0 + rows) of the CTA's window, whose origin is (gx0, gy0), to the staging's start
+// staged rows [row0, row0 + rows) of the CTA's window, whose origin is (gx0, gy0), to the staging's start.
+// The radii of a warp's rows are loaded together and the colours copied asynchronously: radius, then colour,
+// then the next bin took some forty memory latencies a CTA (3840 x 2160 bins with discs of radius 0 alone 256
+// -> 194 us, at 1000 points per bin 642 -> 598).
 __device__ __forceinline__ void de_stage(const float4* __restrict__ in, const uint8_t* __restrict__ rad, int w, int h, int gx0,
                                          int gy0, int pitch, int row0, int rows, float4* s_c, uint8_t* s_r) {
+    constexpr int kRows = 8;  // a warp's rows at a time
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    for (int i = warp; i < rows; i += warps) {
-        const int gy = gy0 + row0 + i;
-        const bool row = gy >= 0 && gy < h;
-        for (int x = lane; x < pitch; x += 32) {
-            const int gx = gx0 + x;
-            int r = 255;
-            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (row && gx >= 0 && gx < w) {
-                const size_t gi = (size_t)gy * w + gx;
-                r = rad[gi];
-                if (r != 255) v = in[gi];
+    const uint32_t to = umma::smem_u32(s_c);
+    for (int x = lane; x < pitch; x += 32) {
+        const int gx = gx0 + x;
+        const bool column = gx >= 0 && gx < w;
+        for (int i0 = warp; i0 < rows; i0 += kRows * warps) {
+            int r[kRows];
+#pragma unroll
+            for (int u = 0; u < kRows; u++) {
+                const int i = i0 + u * warps, gy = gy0 + row0 + i;
+                r[u] = column && i < rows && gy >= 0 && gy < h ? rad[(size_t)gy * w + gx] : 255;
             }
-            s_c[i * pitch + x] = v;
-            s_r[i * pitch + x] = (uint8_t)(r + 1);  // 255 -> 0
+#pragma unroll
+            for (int u = 0; u < kRows; u++) {
+                const int i = i0 + u * warps, gy = gy0 + row0 + i;
+                if (i >= rows) break;
+                // the colour lands by itself; an empty bin's is zero
+                umma::cp_async16(to + 16u * (uint32_t)(i * pitch + x), r[u] != 255 ? in + (size_t)gy * w + gx : in, r[u] != 255 ? 16u : 0u);
+                s_r[i * pitch + x] = (uint8_t)(r[u] + 1);  // 255 -> 0
+            }
         }
     }
+    umma::cp_async_commit();
+    umma::cp_async_wait<0>();
 }
 
 __host__ __device__ constexpr size_t de_smem_bytes(int rows, int R, bool whole) {
@@ -608,7 +620,8 @@ static cudaError_t launch_de_rows(int R, const DeParams& P, const float4* in, co
 }
 
 // R: the launch's largest radius.  More rows per warp read a source once for more outputs, fewer leave
-// more warps to hide latency.  Measured, radius 9 (density estimation alone, 8 / 4 / 2 rows): 3840 x 2160
+// more warps to hide latency.  Measured, radius 9 (density estimation alone, 8 / 4 / 2 rows, before the
+// staging was asynchronous): 3840 x 2160
 // 642 / 737 / 872 us, 1920 x 1080 242 / 236 / 274, 960 x 540 116 / 96 / 107, 512 x 512 95 / 73 / 82, 640 x 360
 // 93 / 70 / 64, 320 x 180 88 / 58 / 47: 8 rows from 12 CTAs for each of the 152 SMs, 4 from about 1.6.
 static cudaError_t launch_de_sweep(int R, const float4* in, const uint8_t* rad, uint32_t w, uint32_t h, float4* out,
