@@ -295,7 +295,8 @@ RF_API int  rf_sim_counters(rf_sim* s, uint64_t out[3]);
 
 /* Adaptive density estimation: out (float4 per bin) = every bin with a > 0 spread over a disc
    of radius max(min, min(R, int(R / a^curve))), kernel (1 - d^2) * (2/pi) / r^2 with
-   d = |offset| / (r + 0.5); r = 0 copies the bin.  R <= 100 (main.cpp:502). */
+   d = |offset| / (r + 0.5); r = 0 copies the bin.  R <= 100 (main.cpp:502).  A bin whose colour is
+   not finite changes the outputs of its own disc alone; one whose density is NaN counts as empty. */
 RF_API int rf_density_estimate(const float* bins_rgba, uint32_t width, uint32_t height, int radius,
                         int min_radius, float curve, float* out_rgba, void* stream);
 /* rf_density_estimate without any device allocation (no counterpart in the reference).
