@@ -200,9 +200,10 @@ __device__ __forceinline__ float4 tonemap_finish(float r, float g, float b, floa
     const float rgb[3] = {r, g, b};
     float res[3];
     for (int q = 0; q < 3; q++) {
-        // at vibrancy 1 the first term is zero for every finite colour (a negative one's NaN clamps to 0, as
-        // its second term does): three of a pixel's four powers are not needed
-        const bool plain = vibrancy == 1.0f && fabsf(rgb[q]) < INFINITY;
+        // at vibrancy 1 the first term is zero where the power is finite, as it is of every finite colour at
+        // gamma >= 1 (a negative one's NaN clamps to 0, as its second term does): three of a pixel's four
+        // powers are not needed.  A power that overflows makes the sum NaN, which clamps to 0
+        const bool plain = vibrancy == 1.0f && gamma >= 1.0f && fabsf(rgb[q]) < INFINITY;
         const float v = (plain ? 0.0f : powf(rgb[q], ig) * (1.0f - vibrancy)) + gf * rgb[q] * vibrancy;
         res[q] = fminf(fmaxf(v, 0.0f), 1.0f);
     }
