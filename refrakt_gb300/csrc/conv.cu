@@ -938,7 +938,7 @@ bool conv_supported(uint32_t channels, uint32_t N, uint32_t taps) {
     Geom G{};
     size_t smem = 0;
     geom_tiles(G, 1, 1, 1, taps, channels);
-    return N > 0 && conv_geom(G, channels, N, taps, &smem);
+    return N > 0 && conv_geom(G, channels, N, taps, &smem) && (N - 1) / G.np < 65535;  // column groups: grid.y
 }
 
 cudaError_t launch_conv(const ConvArgs& args, ConvEpilogue epi, cudaStream_t st) {

@@ -52,8 +52,8 @@ struct ConvArgs {
     int* error;                // set by the launcher
 };
 
-// whether launch_conv takes the shape: ca + cb a multiple of 16 (or 8 channels in all) and a tile's
-// operands within an SM's shared memory
+// whether launch_conv takes the shape: ca + cb a multiple of 16 (or 8 channels in all), a tile's
+// operands within an SM's shared memory and no more column groups than a grid has rows
 bool conv_supported(uint32_t channels, uint32_t N, uint32_t taps);
 cudaError_t launch_conv(const ConvArgs& a, ConvEpilogue epi, cudaStream_t st);
 
