@@ -113,9 +113,11 @@ __device__ __forceinline__ bool xbar_wait(uint64_t* b, uint32_t parity) {
 
 // The cluster exchange: a mixing domain spread over the CTAs of a thread-block cluster, each with its
 // share of the slots in its own shared memory.  A pass's walkers are read from the CTA that holds them
-// (distributed shared memory); one cluster barrier per pass replaces the CTA's.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// (distributed shared memory); one cluster barrier per pass replaces the CTA's.  (Not the .aligned forms: they
+// follow code in which lanes part -- the evaluator's branches, the walker reset, the group's draw -- and those forms
+// are undefined unless the warp has met again.  The 65,536 walkers of the CLUSTER comment below: no difference.)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 __device__ __forceinline__ float4 cluster_load(const float4* local, uint32_t rank) {
     uint32_t a = (uint32_t)__cvta_generic_to_shared(local);
     float4 v;
