@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_kernel(const __grid_constant
             wide = ((reinterpret_cast<uintptr_t>(A.C) & 31u) == 0) && A.ldc % 16u == 0;
         Tile t(G, blockIdx.x + buf * gridDim.x, 2 * gridDim.x);
         for (uint32_t i = buf; i < count; i += 2, t.next(G)) {
-            if (!umma::mbar_wait(&B.acc_full[buf], (i >> 1) & 1u, kWaitLimit)) {
+            if (!umma::mbar_wait_warp(&B.acc_full[buf], (i >> 1) & 1u, kWaitLimit)) {
                 conv_fail(B, 4);
                 break;
             }
@@ -817,9 +817,9 @@ __global__ void __launch_bounds__(kWgradThreads, 1) conv_wgrad_kernel(const __gr
         else load_segments<kPlain>(B, L, p0, p1, count, base, stage, dy, dx, tid);
         // the accumulators into gw: a warp its tensor-memory lane quarter and every fourth 16 columns
         const uint32_t q4 = (uint32_t)warp & 3u, share = (uint32_t)warp >> 2;
-        if (count && !umma::mbar_wait(&B.acc_full[0], 0u, kWaitLimit)) conv_fail(B, 4);
+        if (count && !umma::mbar_wait_warp(&B.acc_full[0], 0u, kWaitLimit)) conv_fail(B, 4);
         umma::fence_after_sync();
-        if (count && !conv_failed(B.fail)) {
+        if (count && !__any_sync(0xffffffffu, conv_failed(B.fail))) {
             const uint32_t K = L.taps * C;
             for (uint32_t mt = 0; mt < L.mtiles; mt++) {
                 const uint32_t m = mt * 128u + 32u * q4 + lane, dy = m / C, c = m - dy * C;

@@ -434,12 +434,12 @@ __global__ void __launch_bounds__(kTmaThreads, 1)
         for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x, i++) {
             const TileCoord c = tile_coord(g, t, tiles_m, tiles_n, bn);
             const uint32_t buf = i & 1u, u = i >> 1;
-            if (!umma::mbar_wait(&acc_full[buf], u & 1u, kWaitLimit)) {
+            if (!umma::mbar_wait_warp(&acc_full[buf], u & 1u, kWaitLimit)) {
                 gemm_fail(g, s_fail, 3 + 2 * S + (int)buf);
                 break;
             }
             umma::fence_after_sync();
-            if (gemm_failed(s_fail)) break;
+            if (__any_sync(0xffffffffu, gemm_failed(s_fail))) break;
             const uint32_t n_rem = g.N - c.n0;
             const uint32_t n_tile = ((n_rem < bn ? n_rem : bn) + 15u) & ~15u;
             if (c.nk > 0 || g.mode != kGemmAtomicF32)

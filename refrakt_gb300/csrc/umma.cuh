@@ -91,6 +91,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
     return false;
 }
 
+// the same by a whole warp, which is converged and of one mind afterwards: true when every lane's wait ended
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint32_t limit) {
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit)) != 0;
+}
+
 // reports a wait that ran out to the host (error_word, gemm.h): nonzero codes
 __device__ __forceinline__ void report_error(int* word, int code) { *reinterpret_cast<volatile int*>(word) = code; }
 
@@ -145,9 +150,12 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
                  : "memory");
 }
 
-// 32 lanes x 32 bit, 16 consecutive columns: lane i of the warp receives row (lane base + i)
+// 32 lanes x 32 bit, 16 consecutive columns: lane i of the warp receives row (lane base + i).  Every lane of the
+// warp calls it; they meet first, for the instructions are undefined in a warp that has parted (a store under a
+// condition, a wait's loop).
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
+    __syncwarp();
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
         "%15}, [%16];"
