@@ -72,18 +72,16 @@ __device__ __forceinline__ void precalc(Pre& p, float x, float y, uint32_t m) {
 
 __device__ __forceinline__ float mod2f(float x, float y) { return x - y * truncf(x / y); }  // math.glsl:13
 
-// words of a genome program in shared memory, by 32-bit address
+// words of a genome program in shared memory, by 32-bit address.  Plain loads, which the compiler keeps in order with
+// the stores of the program and the barriers (loads as inline assembly without a memory clobber are none to it, so it
+// may reuse a rewritten program's words).
 struct SharedWords {
     uint32_t a;
     __device__ __forceinline__ float operator[](int i) const {
-        float v;
-        asm("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a + 4u * i));
-        return v;
+        return *static_cast<const float*>(__cvta_shared_to_generic(a + 4u * i));
     }
     __device__ __forceinline__ uint32_t u(int i) const {
-        uint32_t v;
-        asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(a + 4u * i));
-        return v;
+        return *static_cast<const uint32_t*>(__cvta_shared_to_generic(a + 4u * i));
     }
     __device__ __forceinline__ SharedWords operator+(uint32_t n) const { return SharedWords{a + 4u * n}; }
 };
