@@ -46,8 +46,8 @@ enum rf_status {
     RF_ERR_NEEDS_WARMUP = 7,  /* rf_draw_to_bins before rf_warmup for this flame (flame.hpp:86) */
     RF_ERR_IO = 8,            /* file could not be read or written */
     RF_ERR_NO_DEVICE = 9,     /* no CUDA device of the supported architecture */
-    RF_ERR_TIMEOUT = 10       /* a bounded device-side wait gave up (a chaos launch's walker exchange);
-                                 the results of that launch are invalid */
+    RF_ERR_TIMEOUT = 10       /* a bounded device-side wait gave up (a chaos launch's walker exchange, a
+                                 denoiser's convolution); the results of that launch are invalid */
 };
 
 typedef struct rf_compiler rf_compiler;
@@ -479,7 +479,9 @@ RF_API int rf_conv3x3_bf16(const void* xa, uint32_t ca, int up, const void* xb, 
  * masters), FP32 accumulation on the tcgen05 tensor cores; forward, backward and Adam are the
  * library's own kernels.  Tensors are device memory, NHWC: features bf16 [n, h, w, 8], images
  * and targets FP32 [n, h, w, 3]; h and w multiples of 8.  The denoiser runs on its own stream
- * (or the one set by rf_denoiser_set_stream); train_step with loss != NULL synchronises.
+ * (or the one set by rf_denoiser_set_stream); train_step with loss != NULL synchronises.  A
+ * kernel's bounded wait that runs out makes the denoiser's next synchronising call (that
+ * train_step, sync, get_params, set_params, gradients) return RF_ERR_TIMEOUT, once.
  * ---------------------------------------------------------------------------------------- */
 typedef struct rf_denoiser rf_denoiser;
 typedef struct {

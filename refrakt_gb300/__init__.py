@@ -29,7 +29,7 @@ BINS_AUTO, BINS_DIRECT, BINS_INTERLEAVED = 0, 1, 2
 FILTER_GAUSSIAN, FILTER_BOX, FILTER_TRIANGLE, FILTER_HERMITE = 0, 1, 2, 3
 
 STATUS = {0: "OK", 1: "INVALID_ARG", 2: "PARSE", 3: "UNKNOWN_NAME", 4: "UNSUPPORTED", 5: "CAPACITY",
-          6: "CUDA", 7: "NEEDS_WARMUP", 8: "IO", 9: "NO_DEVICE"}
+          6: "CUDA", 7: "NEEDS_WARMUP", 8: "IO", 9: "NO_DEVICE", 10: "TIMEOUT"}
 
 
 class RefraktError(RuntimeError):

@@ -156,7 +156,7 @@ struct Bars {
     int* fail;
     int* error;  // the host's error word
 };
-// b.error gets 1 loading, 2 an accumulator's release, 3 a stage, 4 an accumulator
+// b.error gets 1 a stage to load, 2 an accumulator's release, 3 a loaded stage, 4 an accumulator (conv_error)
 __device__ __forceinline__ void conv_fail(const Bars& b, int code) {
     *reinterpret_cast<volatile int*>(b.fail) = 1;
     umma::report_error(b.error, code);
@@ -941,10 +941,8 @@ bool conv_supported(uint32_t channels, uint32_t N, uint32_t taps) {
     return N > 0 && conv_geom(G, channels, N, taps, &smem) && (N - 1) / G.np < 65535;  // column groups: grid.y
 }
 
-cudaError_t launch_conv(const ConvArgs& args, ConvEpilogue epi, cudaStream_t st) {
-    ConvArgs a = args;
-    if (!(a.error = error_word())) return cudaErrorMemoryAllocation;
-    if ((a.taps != 9 && a.taps != 1) || a.n == 0 || a.h == 0 || a.w == 0 || a.N == 0 || a.ca % 8 || a.cb % 8 || a.ldb % 8 ||
+cudaError_t launch_conv(const ConvArgs& a, ConvEpilogue epi, cudaStream_t st) {
+    if (!a.error || (a.taps != 9 && a.taps != 1) || a.n == 0 || a.h == 0 || a.w == 0 || a.N == 0 || a.ca % 8 || a.cb % 8 || a.ldb % 8 ||
         a.ldb < a.taps * (a.ca + a.cb) || (((uintptr_t)a.xa | (uintptr_t)a.xb | (uintptr_t)a.B) & 15))
         return cudaErrorInvalidValue;
     Geom G{};
@@ -1008,10 +1006,10 @@ static uint32_t wgrad_parts(const WgradLayer& L) {
 }
 
 cudaError_t launch_conv_wgrad(const WgradTask* tasks, uint32_t count, const __nv_bfloat16* bias_dz, uint64_t bias_pixels,
-                              float* bias_gb, cudaStream_t st) {
-    if (count == 0 || count > (uint32_t)kMaxWgradLayers || bias_pixels > 0x7fffffffull) return cudaErrorInvalidValue;
+                              float* bias_gb, int* error, cudaStream_t st) {
+    if (!error || count == 0 || count > (uint32_t)kMaxWgradLayers || bias_pixels > 0x7fffffffull) return cudaErrorInvalidValue;
     WgradArgs W{};
-    if (!(W.error = error_word())) return cudaErrorMemoryAllocation;
+    W.error = error;
     W.layers = count;
     W.bias_first = bias_dz ? kBiasCtas : 0;
     W.bias_dz = bias_dz;

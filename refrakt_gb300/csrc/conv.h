@@ -49,13 +49,17 @@ struct ConvArgs {
     const float* target;
     float* out;
     double* loss;
-    int* error;                // set by the launcher
+    int* error;                // the caller's ErrorWord (error_word.h): conv_error's codes
 };
 
 // whether launch_conv takes the shape: ca + cb a multiple of 16 (or 8 channels in all), a tile's
 // operands within an SM's shared memory and no more column groups than a grid has rows
 bool conv_supported(uint32_t channels, uint32_t N, uint32_t taps);
 cudaError_t launch_conv(const ConvArgs& a, ConvEpilogue epi, cudaStream_t st);
+// what the wait that a code of ConvArgs.error names was for
+inline const char* conv_error(int code) {
+    return code == 1 ? "a stage to load" : code == 2 ? "an accumulator's release" : code == 3 ? "a loaded stage" : "an accumulator";
+}
 
 // gw[co][tap (ca + cb) + c] += sum over pixels of dz[p][co] x[p shifted by tap][c] for every task in
 // one launch; of `conv` xa, xb, ca, cb, up, n, h, w, taps and dz (ldz channels per
@@ -68,6 +72,6 @@ struct WgradTask {
 constexpr int kMaxWgradLayers = 16;
 // with bias_dz (8 channels per pixel, the head's dz) also the head's bias gradient into bias_gb[0..2]
 cudaError_t launch_conv_wgrad(const WgradTask* tasks, uint32_t count, const __nv_bfloat16* bias_dz, uint64_t bias_pixels,
-                              float* bias_gb, cudaStream_t st);
+                              float* bias_gb, int* error, cudaStream_t st);
 
 }  // namespace rfk

@@ -20,7 +20,7 @@
 
 #include "conv.h"
 #include "denoise_ops.h"
-#include "gemm.h"
+#include "error_word.h"
 #include "internal.h"
 #include "kernels.h"
 #include "scratch.h"
@@ -69,12 +69,22 @@ struct rf_denoiser {
     AdamLayers adam{};
     double* loss = nullptr;
     uint32_t step = 0;
+    ErrorWord error;                // of every convolution and weight-gradient launch
     std::vector<void*> allocs;
 };
 
 namespace {
 
 int cuda_fail(cudaError_t e, const char* what) { return fail(RF_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e)); }
+
+// waits for the denoiser's stream; RF_ERR_TIMEOUT when a bounded wait of a kernel launched before ran out
+int sync(rf_denoiser* D, const char* fn) {
+    const cudaError_t e = cudaStreamSynchronize(D->stream);
+    if (e != cudaSuccess) return cuda_fail(e, fn);
+    if (const int code = D->error.take())
+        return fail(RF_ERR_TIMEOUT, std::string(fn) + ": a convolution's wait for " + conv_error(code) + " ran out; the results are invalid");
+    return RF_OK;
+}
 
 template <class T>
 cudaError_t dalloc(rf_denoiser* d, T** p, size_t n, bool zero = false) {
@@ -156,6 +166,7 @@ ConvArgs layer_input(rf_denoiser* D, size_t i, const __nv_bfloat16* input) {
     a.h = D->H >> c.level;
     a.w = D->W >> c.level;
     a.taps = c.taps;
+    a.error = D->error.get();
     return a;
 }
 
@@ -221,6 +232,7 @@ int train(rf_denoiser* D, const __nv_bfloat16* input, const float* target, float
         gx.B = c.wf16;
         gx.ldb = c.ldf();
         gx.N = c.ca + c.cb;
+        gx.error = D->error.get();
         ConvEpilogue epi = kConvMask;
         int into = c.src_a;  // the layer whose output gradient this completes
         if (c.cb > 0) {
@@ -240,7 +252,7 @@ int train(rf_denoiser* D, const __nv_bfloat16* input, const float* target, float
     }
     const Conv& head = D->convs[D->out_conv];
     e = launch_conv_wgrad(tasks.data(), (uint32_t)tasks.size(), D->acts[D->out_conv].dz, level_pixels(D->N, D->H, D->W, 0),
-                          head.gb, D->stream);
+                          head.gb, D->error.get(), D->stream);
     if (e != cudaSuccess) return cuda_fail(e, "weight gradients");
     return update(D, lr, ++D->step);
 }
@@ -272,7 +284,7 @@ int rf_denoiser_create(const rf_denoiser_desc* desc, rf_denoiser** out) {
     if (cudaSetDevice(D->device) != cudaSuccess) return bail(fail(RF_ERR_NO_DEVICE, "rf_denoiser_create: no such device"));
     cudaError_t e = cudaStreamCreateWithFlags(&D->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) return bail(cuda_fail(e, "stream"));
-    error_word();  // (allocates: before any capture of the denoiser's work)
+    if (!D->error.acquire()) return bail(cuda_fail(cudaErrorMemoryAllocation, "rf_denoiser_create: error word"));
     build_graph(D);
     // parameters, He-normal initialisation from a seeded generator
     const size_t np = rf_denoiser_num_params(D);
@@ -348,9 +360,7 @@ int rf_denoiser_set_stream(rf_denoiser* D, void* stream) {
 int rf_denoiser_sync(rf_denoiser* D) {
     if (!D) return fail(RF_ERR_INVALID_ARG, "rf_denoiser_sync: null");
     cudaSetDevice(D->device);
-    cudaError_t e = cudaStreamSynchronize(D->stream);
-    if (e != cudaSuccess) return cuda_fail(e, "rf_denoiser_sync");
-    return RF_OK;
+    return sync(D, "rf_denoiser_sync");
 }
 
 int rf_denoiser_num_layers(const rf_denoiser* D) { return D ? (int)D->convs.size() : -1; }
@@ -385,8 +395,8 @@ size_t rf_denoiser_num_params(const rf_denoiser* D) {
 int rf_denoiser_get_params(rf_denoiser* D, float* host, size_t cap) {
     if (!D || !host || cap < rf_denoiser_num_params(D)) return fail(RF_ERR_INVALID_ARG, "rf_denoiser_get_params: bad arguments");
     cudaSetDevice(D->device);
-    cudaError_t e = cudaStreamSynchronize(D->stream);
-    if (e == cudaSuccess) e = cudaMemcpy(host, D->w, rf_denoiser_num_params(D) * sizeof(float), cudaMemcpyDeviceToHost);
+    if (int rc = sync(D, "rf_denoiser_get_params")) return rc;
+    const cudaError_t e = cudaMemcpy(host, D->w, rf_denoiser_num_params(D) * sizeof(float), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(e, "rf_denoiser_get_params");
     return RF_OK;
 }
@@ -394,8 +404,8 @@ int rf_denoiser_get_params(rf_denoiser* D, float* host, size_t cap) {
 int rf_denoiser_set_params(rf_denoiser* D, const float* host, size_t count) {
     if (!D || !host || count != rf_denoiser_num_params(D)) return fail(RF_ERR_INVALID_ARG, "rf_denoiser_set_params: bad arguments");
     cudaSetDevice(D->device);
-    cudaError_t e = cudaStreamSynchronize(D->stream);
-    if (e == cudaSuccess) e = cudaMemcpy(D->w, host, count * sizeof(float), cudaMemcpyHostToDevice);
+    if (int rc = sync(D, "rf_denoiser_set_params")) return rc;
+    const cudaError_t e = cudaMemcpy(D->w, host, count * sizeof(float), cudaMemcpyHostToDevice);
     if (e != cudaSuccess) return cuda_fail(e, "rf_denoiser_set_params");
     return refresh_bf16(D);
 }
@@ -438,8 +448,8 @@ int rf_denoiser_train_step(rf_denoiser* D, const void* feats, const float* targe
     if (loss) {
         double l = 0;
         cudaError_t e = cudaMemcpyAsync(&l, D->loss, sizeof(double), cudaMemcpyDeviceToHost, D->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(D->stream);
         if (e != cudaSuccess) return cuda_fail(e, "rf_denoiser_train_step");
+        if (int rc = sync(D, "rf_denoiser_train_step")) return rc;
         *loss = l / (3.0 * (double)n * h * w);
     }
     return RF_OK;
@@ -448,8 +458,8 @@ int rf_denoiser_train_step(rf_denoiser* D, const void* feats, const float* targe
 int rf_denoiser_gradients(rf_denoiser* D, float* host, size_t cap) {
     if (!D || !host || cap < rf_denoiser_num_params(D)) return fail(RF_ERR_INVALID_ARG, "rf_denoiser_gradients: bad arguments");
     cudaSetDevice(D->device);
-    cudaError_t e = cudaStreamSynchronize(D->stream);
-    if (e == cudaSuccess) e = cudaMemcpy(host, D->g, rf_denoiser_num_params(D) * sizeof(float), cudaMemcpyDeviceToHost);
+    if (int rc = sync(D, "rf_denoiser_gradients")) return rc;
+    const cudaError_t e = cudaMemcpy(host, D->g, rf_denoiser_num_params(D) * sizeof(float), cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return cuda_fail(e, "rf_denoiser_gradients");
     return RF_OK;
 }

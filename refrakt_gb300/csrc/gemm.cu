@@ -21,8 +21,6 @@
 #include <cudaTypedefs.h>
 
 #include <algorithm>
-#include <atomic>
-#include <mutex>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -550,8 +548,7 @@ cudaError_t launch_bn(const GemmArgs& g, uint32_t splits, cudaStream_t st) {
 
 cudaError_t launch_gemm(GemmArgs g, uint32_t splits, cudaStream_t st) {
     if (g.K % 8 || g.lda % 8 || g.ldb % 8 || g.M == 0 || g.N == 0) return cudaErrorInvalidValue;
-    if (((uintptr_t)g.A | (uintptr_t)g.B) & 15) return cudaErrorInvalidValue;
-    if (!(g.error = error_word())) return cudaErrorMemoryAllocation;
+    if ((((uintptr_t)g.A | (uintptr_t)g.B) & 15) || !g.error) return cudaErrorInvalidValue;
     if (splits == 0) splits = 1;
     const uint32_t kblocks = (g.K + umma::kTileK - 1) / umma::kTileK;
     if (splits > kblocks && kblocks > 0) splits = kblocks;
@@ -574,36 +571,14 @@ cudaError_t launch_gemm_conv(GemmArgs g, cudaStream_t st) {
     if (g.ca % 8 || g.cb % 8 || g.ca + g.cb == 0 || g.n == 0 || g.h == 0 || g.w == 0 || g.h > 65535 || g.w > 65535)
         return cudaErrorInvalidValue;
     if (!g.xa || (g.cb && !g.xb) || (uint64_t)g.n * g.h * g.w != g.M || g.K != 9u * (g.ca + g.cb) || g.ldb % 8 ||
-        g.N == 0 || ((uintptr_t)g.xa | (uintptr_t)g.xb | (uintptr_t)g.B) & 15)
+        g.N == 0 || ((uintptr_t)g.xa | (uintptr_t)g.xb | (uintptr_t)g.B) & 15 || !g.error)
         return cudaErrorInvalidValue;
-    if (!(g.error = error_word())) return cudaErrorMemoryAllocation;
     g.A = nullptr;
     g.lda = 0;
     g.k_per_split = (g.K + umma::kTileK - 1) / umma::kTileK * umma::kTileK;
     if (g.N <= 64) return launch_bn<64, true>(g, 1, st);
     if (g.N <= 128) return launch_bn<128, true>(g, 1, st);
     return launch_bn<256, true>(g, 1, st);
-}
-
-int* error_word() {
-    static std::atomic<int*> word{nullptr};
-    static std::mutex mu;
-    int* p = word.load(std::memory_order_acquire);
-    if (p) return p;
-    std::lock_guard<std::mutex> lock(mu);
-    p = word.load(std::memory_order_relaxed);
-    if (!p && cudaHostAlloc((void**)&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) {
-        *p = 0;
-        word.store(p, std::memory_order_release);
-        return p;
-    }
-    if (!p) cudaGetLastError();
-    return p;
-}
-
-int take_error() {
-    int* p = error_word();
-    return p ? __atomic_exchange_n(p, 0, __ATOMIC_ACQ_REL) : 0;
 }
 
 }  // namespace rfk

@@ -27,7 +27,7 @@ struct GemmArgs {
     const __nv_bfloat16* xb;
     uint32_t ca, cb, n, h, w;
     int up;
-    int* error;              // set by the launcher: error_word()
+    int* error;              // the caller's ErrorWord (error_word.h): which wait of the kernel ran out
 };
 
 // splits > 1 partitions K over grid.z and requires kGemmAtomicF32 (C accumulates)
@@ -35,12 +35,5 @@ cudaError_t launch_gemm(GemmArgs g, uint32_t splits, cudaStream_t st);
 // C = im2col(xa, xb) * B^T without materialising the im2col matrix; M = n h w, K = 9 (ca + cb),
 // ca and cb multiples of 8, one split
 cudaError_t launch_gemm_conv(GemmArgs g, cudaStream_t st);
-// The tensor-core kernels' error word (these and conv.cu's): pinned host memory that a kernel writes
-// only when a bounded wait runs out, so the host reads it after a synchronisation without a copy (two
-// copies of the word took 20 us per call).  Allocated on the first call, outside stream capture; null
-// when that fails.
-int* error_word();
-// its value, cleared; call after the stream was synchronised (0 = no bounded wait ran out)
-int take_error();
 
 }  // namespace rfk

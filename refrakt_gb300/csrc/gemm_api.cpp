@@ -5,6 +5,7 @@
 #include <string>
 
 #include "conv.h"
+#include "error_word.h"
 #include "gemm.h"
 #include "internal.h"
 #include "refrakt.h"
@@ -13,14 +14,16 @@ using namespace rfk;
 
 namespace {
 
-// waits for the launch, then takes the kernels' bounded-wait error word
-int finish(const char* fn, cudaError_t e, cudaStream_t st) {
+// waits for the launch, then takes the call's error word; conv: the code is one of conv.cu's
+int finish(const char* fn, cudaError_t e, cudaStream_t st, ErrorWord& word, bool conv) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    const int werr = take_error();
     if (e != cudaSuccess) return fail(RF_ERR_CUDA, std::string(fn) + ": " + cudaGetErrorString(e));
-    if (werr) return fail(RF_ERR_CUDA, std::string(fn) + ": an mbarrier wait ran out (stage " + std::to_string(werr - 1) + ")");
-    return RF_OK;
+    const int code = word.take();
+    if (!code) return RF_OK;
+    return fail(RF_ERR_CUDA, std::string(fn) + ": an mbarrier wait ran out (" +
+                                 (conv ? "for " + std::string(conv_error(code)) : "code " + std::to_string(code)) + ")");
 }
+int no_word(const char* fn) { return fail(RF_ERR_CUDA, std::string(fn) + ": " + cudaGetErrorString(cudaErrorMemoryAllocation)); }
 
 }  // namespace
 
@@ -46,8 +49,11 @@ extern "C" int rf_gemm_bf16(const void* A, const void* B, void* C, uint32_t M, u
     g.mode = mode;
     g.bias = bias;
     g.relu = relu;
+    ErrorWord word;
+    if (!word.acquire()) return no_word("rf_gemm_bf16");
+    g.error = word.get();
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    return finish("rf_gemm_bf16", launch_gemm(g, splits, st), st);
+    return finish("rf_gemm_bf16", launch_gemm(g, splits, st), st, word, false);
 }
 
 extern "C" int rf_conv3x3_bf16(const void* xa, uint32_t ca, int up, const void* xb, uint32_t cb, uint32_t n,
@@ -63,6 +69,8 @@ extern "C" int rf_conv3x3_bf16(const void* xa, uint32_t ca, int up, const void* 
     if ((((uintptr_t)xa) | ((uintptr_t)xb) | ((uintptr_t)B)) & 15)
         return fail(RF_ERR_INVALID_ARG, "rf_conv3x3_bf16: operands must be 16-byte aligned");
     if (mode < RF_GEMM_STORE_F32 || mode > RF_GEMM_ATOMIC_F32) return fail(RF_ERR_INVALID_ARG, "rf_conv3x3_bf16: bad mode");
+    ErrorWord word;
+    if (!word.acquire()) return no_word("rf_conv3x3_bf16");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     // channels in whole K steps and a tile's operands within shared memory: the staged-tile kernel
     // (conv.cu); other channel counts gather im2col rows (gemm.cu)
@@ -84,8 +92,9 @@ extern "C" int rf_conv3x3_bf16(const void* xa, uint32_t ca, int up, const void* 
         a.ldc = ldc;
         a.bias = bias;
         a.relu = relu;
+        a.error = word.get();
         const ConvEpilogue epi = mode == RF_GEMM_STORE_F32 ? kConvStoreF32 : mode == RF_GEMM_ATOMIC_F32 ? kConvAtomicF32 : kConvStoreBF16;
-        return finish("rf_conv3x3_bf16", launch_conv(a, epi, st), st);
+        return finish("rf_conv3x3_bf16", launch_conv(a, epi, st), st, word, true);
     }
     GemmArgs g{};
     g.xa = static_cast<const __nv_bfloat16*>(xa);
@@ -106,5 +115,6 @@ extern "C" int rf_conv3x3_bf16(const void* xa, uint32_t ca, int up, const void* 
     g.mode = mode;
     g.bias = bias;
     g.relu = relu;
-    return finish("rf_conv3x3_bf16", launch_gemm_conv(g, st), st);
+    g.error = word.get();
+    return finish("rf_conv3x3_bf16", launch_gemm_conv(g, st), st, word, false);
 }

@@ -96,7 +96,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, u
     return __all_sync(0xffffffffu, mbar_wait(bar, parity, limit)) != 0;
 }
 
-// reports a wait that ran out to the host (error_word, gemm.h): nonzero codes
+// reports a wait that ran out to the host (error_word.h): nonzero codes
 __device__ __forceinline__ void report_error(int* word, int code) { *reinterpret_cast<volatile int*>(word) = code; }
 
 // ---- async-proxy fences ----------------------------------------------------------------------
