@@ -220,9 +220,14 @@ int check_exchange(rf_sim* s) {
     return RF_OK;
 }
 
-// the chaos kernel reads these counters as unsigned long long
+// the geometry of a call's point lists in rf_sim.lists (reserve_lists)
+struct ListShape {
+    uint32_t ranges = 0, range_bits = 0, cap = 0;
+};
+
+// lists: the points go through them (splat 4); null: to the planes
 int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4* bins, uint32_t* hits,
-                  uint32_t W, uint32_t H, const float ss[6]) {
+                  uint32_t W, uint32_t H, const float ss[6], const ListShape* lists = nullptr) {
     uint32_t done = 0;
     while (done < passes) {
         const uint32_t steps = std::min(s->L, passes - done);
@@ -243,7 +248,7 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
         a.first_run = (first_run && done == 0) ? 1 : 0;
         a.draw = draw ? 1 : 0;
         // RF_SPLAT_AUTO's tile: settle a pending decision, then see whether this launch is timed
-        const bool planes = s->rgba_shift == 0 && s->list_ranges == 0;
+        const bool planes = s->rgba_shift == 0 && !lists;
         const bool tile_grid = draw && s->splat == RF_SPLAT_AUTO && planes && hits &&
                                (uint64_t)W * H <= kAutoTileMaxBins && s->tile_ev[0] && !capturing(s->stream);
         if (tile_grid && (s->auto_tile_wh[0] != W || s->auto_tile_wh[1] != H)) {
@@ -258,7 +263,7 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
         if (tile_grid && steps == s->auto_tile_passes && s->auto_tile_state == 3) tile_timed = 1;
         const bool auto_tile = draw && s->splat == RF_SPLAT_AUTO && planes && s->auto_tile_wh[0] == W &&
                                s->auto_tile_wh[1] == H && (s->auto_tile_state == 1 || tile_timed == 1);
-        a.splat = auto_tile ? 3 : s->list_ranges ? 4 : splat_code(s->splat);
+        a.splat = auto_tile ? 3 : lists ? 4 : splat_code(s->splat);
         a.reset = s->reset;
         a.rgba_shift = s->rgba_shift;
         a.count_shift = s->count_shift;
@@ -278,10 +283,10 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
         a.trace_passes = s->trace_passes;
         a.n_groups = (uint32_t)(s->N / kGroup);
         const uint32_t tile_bins = a.splat == 3 && a.draw ? a.tile_w * a.tile_h : 0u;
-        if (s->list_ranges) {
-            a.ranges = s->list_ranges;
-            a.range_bits = s->list_range_bits;
-            a.list_cap = s->list_cap;
+        if (lists) {
+            a.ranges = lists->ranges;
+            a.range_bits = lists->range_bits;
+            a.list_cap = lists->cap;
             a.list_n = reinterpret_cast<uint32_t*>(s->lists + kListScratch);
             a.list = reinterpret_cast<uint2*>(a.list_n + (((s->N / s->slots) * a.ranges + 3) & ~(size_t)3));
         }
@@ -382,7 +387,7 @@ void measure_lists(rf_sim* s, const uint32_t* hits, uint32_t W, uint32_t H, uint
 
 // the lists' memory for a call of `passes` passes, four times an even spread over the ranges where it fits, at
 // least 1.25 times; false: it does not, or the sim's domains are spread over clusters
-bool reserve_lists(rf_sim* s, size_t nb, uint32_t passes) {
+bool reserve_lists(rf_sim* s, size_t nb, uint32_t passes, ListShape& shape) {
     // ranges of 2^21 bins; of 2^20 where more than 2^23 points of a launch fall into one on average, so that
     // most stay below the 2^24 of a single reduction per point (637 M points on 8192 x 8192 bins: 13.9 -> 11.7 ms)
     uint32_t bits = kMaxRangeBits;
@@ -411,9 +416,7 @@ bool reserve_lists(rf_sim* s, size_t nb, uint32_t passes) {
         }
         s->lists_bytes = bytes;
     }
-    s->list_ranges = ranges;
-    s->list_range_bits = bits;
-    s->list_cap = (uint32_t)cap;
+    shape = ListShape{ranges, bits, (uint32_t)cap};
     return true;
 }
 
@@ -425,10 +428,10 @@ int draw_passes(rf_sim* s, uint32_t passes, float4* bins, uint32_t* hits, uint32
     bool il = s->bin_layout == RF_BINS_INTERLEAVED;
     if (s->bin_layout == RF_BINS_AUTO) il = hits != nullptr && nb * 20 > kInterleaveMinBytes;
     if (!il) return launch_passes(s, passes, false, true, bins, hits, W, H, ss);
-    if (s->bin_layout == RF_BINS_AUTO && nb >= kListMinBins && lists_suit(s, W, H) && reserve_lists(s, nb, passes)) {
+    ListShape lists;
+    if (s->bin_layout == RF_BINS_AUTO && nb >= kListMinBins && lists_suit(s, W, H) && reserve_lists(s, nb, passes, lists)) {
         RF_CUDA(cudaMemsetAsync(s->counters + 6, 0, sizeof(unsigned long long), s->stream));
-        const int rc = launch_passes(s, passes, false, true, bins, hits, W, H, ss);
-        s->list_ranges = 0;
+        const int rc = launch_passes(s, passes, false, true, bins, hits, W, H, ss, &lists);
         if (!rc) measure_lists(s, hits, W, H, (uint64_t)s->N * passes);
         return rc;
     }

@@ -69,11 +69,10 @@ struct rf_sim {
     uint32_t rgba_shift = 0, count_shift = 0;  // BinTarget addressing of the next launches
     float4* rec = nullptr;       // interleaved bin records (32 B per bin), all zero between calls
     size_t rec_n = 0;
-    // the list splat's memory: scratch planes of one range (all zero between calls), then the counts and the
-    // lists of list_ctas x list_ranges x list_cap entries; list_ranges 0: the next launches have none
+    // the list splat's memory: two sets of scratch planes of one range (all zero between calls), then a count and a
+    // list per CTA and range
     unsigned char* lists = nullptr;
     size_t lists_bytes = 0, lists_refused = ~(size_t)0;  // refused: a size the device had no memory for
-    uint32_t list_ranges = 0, list_range_bits = 0, list_cap = 0;
     // after the first list call of a genome and grid (pinned, zero until they have arrived): the hits of the
     // hottest bin, of all bins, and the points of the call that found their list full; those points' number
     unsigned long long* list_stats = nullptr;
