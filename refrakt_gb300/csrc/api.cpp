@@ -334,7 +334,7 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
                 set[k].count = reinterpret_cast<uint32_t*>(s->lists + n * 64) + k * n;
             }
             RF_CUDA(launch_ranges(a, grid, set, reinterpret_cast<RangeState*>(s->lists + kListScratch) - kMaxRanges,
-                                  s->counters + 6, s->stream));
+                                  s->counters + 4, s->stream));
         }
         s->cur ^= 1;
         s->pass += steps;
@@ -359,26 +359,26 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
 // 8192 bins 3.94, 1.84 and 3.49, 2.47 (637 M points 24.9, 11.7); 8192 x 4608 3.26, 1.65 and 2.50, 2.28; 6000 x
 // 4000 2.58, 1.56 and 1.88, 2.28; 4099 x 3301 1.68, 1.49 and 1.69, 2.29: from kListMinBins bins on.  Not for hot bins, whose points the lists' second step adds one after another while the
 // records' reductions pass under the chaos game (62 M points of the 5-xform genome on 5000 x 4001 bins, 0.3 % of
-// them in one bin: 1.63 ms with records, 1.80 with lists): the first call measures, later ones take records
-// above a share of 1 / kListHot in one bin or where an eighth of the points found their list full.
+// them in one bin: 1.63 ms with records, 1.80 with lists): the first call measures its points (not the caller's
+// plane, which may hold others), later ones take records above a share of 1 / kListHot in one bin or where an
+// eighth of the points found their list full.
 bool lists_suit(const rf_sim* s, uint32_t W, uint32_t H) {
     if (!s->list_asked || s->list_wh[0] != W || s->list_wh[1] != H) return true;
     const volatile unsigned long long* h = s->list_stats;
-    return h[0] * kListHot < h[1] + (h[1] == 0) && h[2] * 8 <= s->list_points;
+    return (double)h[0] * kListHot * s->list_launches < (double)h[1] + (h[1] == 0) && h[2] * 8 <= s->list_points;
 }
 
-// asks for it once per genome and grid (an option: nothing fails for it)
-void measure_lists(rf_sim* s, const uint32_t* hits, uint32_t W, uint32_t H, uint64_t points) {
+// asks for the statistics of the call's launches (counters[4..6], launch_ranges), once per genome and grid (an
+// option: nothing fails for it)
+void measure_lists(rf_sim* s, uint32_t W, uint32_t H, uint32_t passes) {
     if (s->list_asked && s->list_wh[0] == W && s->list_wh[1] == H) return;
     if (!s->list_stats && cudaHostAlloc((void**)&s->list_stats, 24, cudaHostAllocDefault) != cudaSuccess) s->list_stats = nullptr;
     s->list_asked = false;
     if (s->list_stats) {
         for (int k = 0; k < 3; k++) s->list_stats[k] = 0;
-        unsigned long long* out = s->counters + 4;
-        s->list_asked = cudaMemsetAsync(out, 0, 16, s->stream) == cudaSuccess &&
-                        launch_hottest_bin(hits, (size_t)W * H, out, s->stream) == cudaSuccess &&
-                        cudaMemcpyAsync(s->list_stats, out, 24, cudaMemcpyDeviceToHost, s->stream) == cudaSuccess;
-        s->list_points = points;
+        s->list_asked = cudaMemcpyAsync(s->list_stats, s->counters + 4, 24, cudaMemcpyDeviceToHost, s->stream) == cudaSuccess;
+        s->list_points = s->N * passes;
+        s->list_launches = (double)passes / std::min(passes, s->L);
         s->list_wh[0] = W;
         s->list_wh[1] = H;
     }
@@ -430,9 +430,9 @@ int draw_passes(rf_sim* s, uint32_t passes, float4* bins, uint32_t* hits, uint32
     if (!il) return launch_passes(s, passes, false, true, bins, hits, W, H, ss);
     ListShape lists;
     if (s->bin_layout == RF_BINS_AUTO && nb >= kListMinBins && lists_suit(s, W, H) && reserve_lists(s, nb, passes, lists)) {
-        RF_CUDA(cudaMemsetAsync(s->counters + 6, 0, sizeof(unsigned long long), s->stream));
+        RF_CUDA(cudaMemsetAsync(s->counters + 4, 0, 3 * sizeof(unsigned long long), s->stream));
         const int rc = launch_passes(s, passes, false, true, bins, hits, W, H, ss, &lists);
-        if (!rc) measure_lists(s, hits, W, H, (uint64_t)s->N * passes);
+        if (!rc && passes) measure_lists(s, W, H, passes);
         return rc;
     }
     if (s->rec_n < nb) {

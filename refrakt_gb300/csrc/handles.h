@@ -73,10 +73,12 @@ struct rf_sim {
     // list per CTA and range
     unsigned char* lists = nullptr;
     size_t lists_bytes = 0, lists_refused = ~(size_t)0;  // refused: a size the device had no memory for
-    // after the first list call of a genome and grid (pinned, zero until they have arrived): the hits of the
-    // hottest bin, of all bins, and the points of the call that found their list full; those points' number
+    // after the first list call of a genome and grid (pinned, zero until they have arrived): the most points that a
+    // launch's lists held of one bin, the points in the call's lists, and those that found their list full; the call's
+    // points and launches (full ones)
     unsigned long long* list_stats = nullptr;
     uint64_t list_points = 0;
+    double list_launches = 1;
     uint32_t list_wh[2] = {0, 0};
     bool list_asked = false;
     // rf_render scratch

@@ -62,12 +62,13 @@ struct RangeArgs {
     RangeState* state;  // per range
     float4* bins;
     uint32_t* hits;
+    unsigned long long* stats;  // launch_ranges
 };
 constexpr uint32_t kRangeThreads = 512, kMergeCtas = 1024;
 
 // a CTA per range: the points in its lists, and those that found their list full
 __global__ void __launch_bounds__(256) range_count_kernel(const uint32_t* __restrict__ list_n, uint32_t ctas, uint32_t ranges,
-                                                          uint32_t cap, RangeState* state, unsigned long long* over) {
+                                                          uint32_t cap, RangeState* state, unsigned long long* stats) {
     __shared__ unsigned long long s_sum[2];
     if (threadIdx.x < 2) s_sum[threadIdx.x] = 0;
     __syncthreads();
@@ -82,7 +83,8 @@ __global__ void __launch_bounds__(256) range_count_kernel(const uint32_t* __rest
     __syncthreads();
     if (threadIdx.x == 0) {
         state[blockIdx.x] = RangeState{s_sum[0] < (1u << 24) ? 1u : 0u, 0u};
-        if (s_sum[1]) atomicAdd(over, s_sum[1]);
+        atomicAdd(stats + 1, s_sum[0]);
+        if (s_sum[1]) atomicAdd(stats + 2, s_sum[1]);
     }
 }
 
@@ -131,6 +133,7 @@ __device__ __forceinline__ void range_merge(const RangeArgs& R, uint32_t cta) {
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     constexpr uint32_t kStep = kMergeCtas * kRangeThreads;
     constexpr int U = 2;
+    uint32_t most = 0;
     for (uint32_t i0 = cta * kRangeThreads + threadIdx.x; i0 < n; i0 += kStep * U) {
         float4 v[U], b[U];
         uint32_t c[U], h[U];
@@ -163,6 +166,8 @@ __device__ __forceinline__ void range_merge(const RangeArgs& R, uint32_t cta) {
             }
         }
 #pragma unroll
+        for (int u = 0; u < U; u++) most = max(most, c[u]);
+#pragma unroll
         for (int u = 0; u < U; u++)
             if (c[u]) {
                 b[u] = __ldcs(R.bins + first + i0 + kStep * u);
@@ -176,6 +181,8 @@ __device__ __forceinline__ void range_merge(const RangeArgs& R, uint32_t cta) {
                 __stcs(R.hits + first + i0 + kStep * u, h[u] + c[u]);
             }
     }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0 && most > *(volatile unsigned long long*)R.stats) atomicMax(R.stats, (unsigned long long)most);
 }
 
 __global__ void __launch_bounds__(kRangeThreads, 3) range_step_kernel(const __grid_constant__ RangeArgs R) {
@@ -195,9 +202,10 @@ __global__ void __launch_bounds__(kRangeThreads, 3) range_step_kernel(const __gr
 }
 
 cudaError_t launch_ranges(const ChaosArgs& a, uint32_t ctas, const RangeScratch set[2], RangeState* state,
-                          unsigned long long* over, cudaStream_t st) {
-    RangeArgs R{a.list, a.list_n, a.list_cap, a.ranges, a.range_bits, ctas, 0, a.W * a.H, a.palette, {set[0], set[1]}, state, a.bins, a.hits};
-    range_count_kernel<<<a.ranges, 256, 0, st>>>(a.list_n, ctas, a.ranges, a.list_cap, state, over);
+                          unsigned long long* stats, cudaStream_t st) {
+    RangeArgs R{a.list, a.list_n, a.list_cap, a.ranges, a.range_bits, ctas, 0, a.W * a.H, a.palette, {set[0], set[1]}, state, a.bins, a.hits,
+                stats};
+    range_count_kernel<<<a.ranges, 256, 0, st>>>(a.list_n, ctas, a.ranges, a.list_cap, state, stats);
     cudaError_t e = cudaGetLastError();
     for (; R.range <= a.ranges && e == cudaSuccess; R.range++) {
         const uint32_t grid = (R.range < a.ranges ? ctas : 0u) + (R.range > 0 ? kMergeCtas : 0u);
@@ -205,28 +213,6 @@ cudaError_t launch_ranges(const ChaosArgs& a, uint32_t ctas, const RangeScratch 
         e = cudaGetLastError();
     }
     return e;
-}
-
-// out[0]: the hits of the hottest bin, out[1]: of all bins (both 0 on entry)
-__global__ void __launch_bounds__(256) hottest_bin_kernel(const uint32_t* __restrict__ hits, size_t n, unsigned long long* out) {
-    uint32_t most = 0;
-    unsigned long long sum = 0;
-    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
-        const uint32_t h = hits[i];
-        most = max(most, h);
-        sum += h;
-    }
-    most = __reduce_max_sync(0xffffffffu, most);
-    for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if ((threadIdx.x & 31) == 0 && sum) {
-        atomicMax(out, (unsigned long long)most);
-        atomicAdd(out + 1, sum);
-    }
-}
-
-cudaError_t launch_hottest_bin(const uint32_t* hits, size_t n, unsigned long long* out, cudaStream_t st) {
-    hottest_bin_kernel<<<152 * 8, 256, 0, st>>>(hits, n, out);
-    return cudaGetLastError();
 }
 
 // src/flame.cpp:138-141 — slot i seeded with warmup_ctx(i + seed * N)

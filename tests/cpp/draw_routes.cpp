@@ -77,7 +77,7 @@ cudaError_t cudaEventElapsedTime(float* t, cudaEvent_t, cudaEvent_t) { *t = 1.0f
 
 // ---- fake launches ----
 static rfk::ChaosArgs g_last;  // the last drawing launch
-static unsigned long long g_hottest = 0, g_points = 1u << 20, g_over = 0;  // what the next lists hold
+static unsigned long long g_hottest = 1, g_points = 1u << 20, g_over = 0;  // what a launch's lists hold
 namespace rfk {
 size_t chaos_smem(int slots, uint32_t words, uint32_t steps, uint32_t tile, int, uint32_t) { return words * 4 + 4096 + (size_t)slots * 48 + steps * 4 + tile * 20; }
 int chaos_cluster(int, uint64_t, uint32_t, uint32_t) { return 1; }
@@ -104,18 +104,15 @@ int spec_kernel(const std::vector<uint32_t>&, int, int, int, const void**, SpecK
 std::string spec_source(const std::vector<uint32_t>&, int, int, SpecKind, int, int, int, int) { return ""; }
 int spec_compile(const std::string&, std::vector<char>&) { return RF_ERR_UNSUPPORTED; }
 bool spec_available(std::string*) { return false; }
-#ifdef HOTTEST_OF_PLANE  // (the statistics as a pass over the caller's counts)
-cudaError_t launch_hottest_bin(const uint32_t*, size_t, unsigned long long* out, cudaStream_t) {
-    const unsigned long long h = g_hottest, n = g_points;
-    enqueue([=] { out[0] = h; out[1] = n; });
+cudaError_t launch_ranges(const ChaosArgs&, uint32_t, const RangeScratch[2], RangeState*, unsigned long long* stats, cudaStream_t) {
+    const unsigned long long h = g_hottest, n = g_points, o = g_over;
+    enqueue([=] {
+        stats[0] = std::max(stats[0], h);
+        stats[1] += n;
+        stats[2] += o;
+    });
     return cudaSuccess;
 }
-cudaError_t launch_ranges(const ChaosArgs&, uint32_t, const RangeScratch[2], RangeState*, unsigned long long* over, cudaStream_t) {
-    const unsigned long long o = g_over;
-    enqueue([=] { *over += o; });
-    return cudaSuccess;
-}
-#endif
 }  // namespace rfk
 
 #define CHECK(x) do { if (!(x)) { printf("line %d: %s (%s)\n", __LINE__, #x, rf_last_error()); return 1; } } while (0)
@@ -155,7 +152,7 @@ struct Scene {
 static int failed_call() {
     Scene t(155648, 1024);
     CHECK(t.draw(8192, 8192) == RF_OK && route() == kLists);
-    g_fail_memset = t.s->counters + 6;
+    g_fail_memset = t.s->counters + 4;
     CHECK(t.draw(8192, 8192) != RF_OK && !g_fail_memset);
     CHECK(rf_set_bin_layout(t.s, RF_BINS_DIRECT) == RF_OK);
     CHECK(t.draw(640, 360) == RF_OK && route() == kPlanes && g_last.ranges == 0);
@@ -164,9 +161,26 @@ static int failed_call() {
     return 0;
 }
 
+// records from the second call on where the call's own points have a hot bin or full lists, and only there: what
+// the caller's count plane holds from elsewhere does not matter
+static int own_points() {
+    for (int k = 0; k < 6; k++) {
+        Scene t(155648, 1024);
+        const uint32_t passes = k == 4 || k == 5 ? 1024 : 16;  // 1024: four launches
+        g_hottest = k == 1 ? 1024 : k == 4 ? 1023 : k == 5 ? 1024 : 1;
+        g_over = k == 2 ? 155648 * 16 / 8 + 1 : k == 3 ? 155648 * 16 / 8 : 0;
+        memset(t.hits, 0, 1 << 20);
+        t.hits[77] = k == 0 ? 4000000000u : 0u;  // another program's points
+        CHECK(t.draw(8192, 8192, passes) == RF_OK && route() == kLists);
+        cudaStreamSynchronize(nullptr);
+        CHECK(t.draw(8192, 8192, passes) == RF_OK && route() == (k == 1 || k == 2 || k == 5 ? kRecords : kLists));
+    }
+    return 0;
+}
+
 int main(int argc, char** argv) {
     const std::string name = argc > 1 ? argv[1] : "";
-    const int rc = name == "failed_call" ? failed_call() : 2;
+    const int rc = name == "failed_call" ? failed_call() : name == "own_points" ? own_points() : 2;
     if (rc == 0) printf("OK\n");
     return rc;
 }

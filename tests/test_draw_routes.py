@@ -15,12 +15,12 @@ def routes(tmp_path_factory):
     exe = str(tmp_path_factory.mktemp("routes") / "draw_routes")
     srcs = [os.path.join(ROOT, "tests", "cpp", "draw_routes.cpp")] + [os.path.join(CSRC, n + ".cpp") for n in
                                                                      ("genome", "parsers", "registry", "snippet_hashes")]
-    subprocess.run(["g++", "-std=c++17", "-O1", "-DHOTTEST_OF_PLANE", "-I", os.path.join(ROOT, "include"), "-I", CSRC,
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "include"), "-I", CSRC,
                     "-I", "/usr/local/cuda/include"] + srcs + ["-o", exe], check=True)
     return exe
 
 
-@pytest.mark.parametrize("scene", ["failed_call"])
+@pytest.mark.parametrize("scene", ["failed_call", "own_points"])
 def test_routes(routes, scene):
     r = subprocess.run([routes, scene], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and "OK" in r.stdout, r.stdout + r.stderr
