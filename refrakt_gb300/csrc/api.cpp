@@ -362,25 +362,31 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
 // them in one bin: 1.63 ms with records, 1.80 with lists): the first call measures its points (not the caller's
 // plane, which may hold others), later ones take records above a share of 1 / kListHot in one bin or where an
 // eighth of the points found their list full.
-bool lists_suit(const rf_sim* s, uint32_t W, uint32_t H) {
-    if (!s->list_asked || s->list_wh[0] != W || s->list_wh[1] != H) return true;
-    const volatile unsigned long long* h = s->list_stats;
+// The verdict holds for the genome, the grid and the view that it was taken for, once its statistics have arrived.
+bool lists_suit(const rf_sim* s, const ListView& view) {
+    if (!s->list_asked || !(s->list_view == view)) return true;
+    const cudaError_t q = cudaEventQuery(s->list_ev);
+    if (q != cudaSuccess) {
+        if (q == cudaErrorNotReady && cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError();  // clear only this status
+        return true;
+    }
+    const unsigned long long* h = s->list_stats;
     return (double)h[0] * kListHot * s->list_launches < (double)h[1] + (h[1] == 0) && h[2] * 8 <= s->list_points;
 }
 
-// asks for the statistics of the call's launches (counters[4..6], launch_ranges), once per genome and grid (an
+// asks for the statistics of the call's launches (counters[4..6], launch_ranges), once per genome, grid and view (an
 // option: nothing fails for it)
-void measure_lists(rf_sim* s, uint32_t W, uint32_t H, uint32_t passes) {
-    if (s->list_asked && s->list_wh[0] == W && s->list_wh[1] == H) return;
-    if (!s->list_stats && cudaHostAlloc((void**)&s->list_stats, 24, cudaHostAllocDefault) != cudaSuccess) s->list_stats = nullptr;
+void measure_lists(rf_sim* s, const ListView& view, uint32_t passes) {
+    if (s->list_asked && s->list_view == view) return;
     s->list_asked = false;
-    if (s->list_stats) {
-        for (int k = 0; k < 3; k++) s->list_stats[k] = 0;
-        s->list_asked = cudaMemcpyAsync(s->list_stats, s->counters + 4, 24, cudaMemcpyDeviceToHost, s->stream) == cudaSuccess;
+    if ((s->list_ev || cudaEventCreateWithFlags(&s->list_ev, cudaEventDisableTiming) == cudaSuccess) &&
+        (s->list_stats || cudaHostAlloc((void**)&s->list_stats, 24, cudaHostAllocDefault) == cudaSuccess)) {
+        // (an earlier request's copy may still be on its way; the event is this one's from here on)
+        s->list_asked = cudaMemcpyAsync(s->list_stats, s->counters + 4, 24, cudaMemcpyDeviceToHost, s->stream) == cudaSuccess &&
+                        cudaEventRecord(s->list_ev, s->stream) == cudaSuccess;
         s->list_points = s->N * passes;
         s->list_launches = (double)passes / std::min(passes, s->L);
-        s->list_wh[0] = W;
-        s->list_wh[1] = H;
+        s->list_view = view;
     }
     if (!s->list_asked) cudaGetLastError();
 }
@@ -393,9 +399,7 @@ bool reserve_lists(rf_sim* s, size_t nb, uint32_t passes, ListShape& shape) {
     uint32_t bits = kMaxRangeBits;
     if ((s->N * std::min(passes, s->L) >> 23) << bits > nb && nb <= (uint64_t)kMaxRanges << (bits - 1)) bits--;
     const uint32_t ranges = (uint32_t)((nb + (1u << bits) - 1) >> bits);
-    // (a captured call takes records: a later call may move the lists)
-    if (s->splat != RF_SPLAT_AUTO || ranges > kMaxRanges || (s->spec && cluster_for_launch(s, true) > 1) || capturing(s->stream))
-        return false;
+    if (s->splat != RF_SPLAT_AUTO || ranges > kMaxRanges || (s->spec && cluster_for_launch(s, true) > 1)) return false;
     const uint64_t ctas = s->N / s->slots, points = (uint64_t)s->slots * std::min(passes, s->L);  // of a CTA
     const size_t head = kListScratch + ((ctas * ranges + 3) & ~(uint64_t)3) * 4;
     if (head >= kListBytes) return false;
@@ -429,10 +433,12 @@ int draw_passes(rf_sim* s, uint32_t passes, float4* bins, uint32_t* hits, uint32
     if (s->bin_layout == RF_BINS_AUTO) il = hits != nullptr && nb * 20 > kInterleaveMinBytes;
     if (!il) return launch_passes(s, passes, false, true, bins, hits, W, H, ss);
     ListShape lists;
-    if (s->bin_layout == RF_BINS_AUTO && nb >= kListMinBins && lists_suit(s, W, H) && reserve_lists(s, nb, passes, lists)) {
+    const ListView view{W, H, {ss[0], ss[1], ss[2], ss[3], ss[4], ss[5]}};
+    // (a captured call takes records: a later call may move the lists)
+    if (s->bin_layout == RF_BINS_AUTO && nb >= kListMinBins && !capturing(s->stream) && lists_suit(s, view) && reserve_lists(s, nb, passes, lists)) {
         RF_CUDA(cudaMemsetAsync(s->counters + 4, 0, 3 * sizeof(unsigned long long), s->stream));
         const int rc = launch_passes(s, passes, false, true, bins, hits, W, H, ss, &lists);
-        if (!rc && passes) measure_lists(s, W, H, passes);
+        if (!rc && passes) measure_lists(s, view, passes);
         return rc;
     }
     if (s->rec_n < nb) {
@@ -785,6 +791,7 @@ int rf_sim_destroy(rf_sim* s) {
     cudaSetDevice(s->device);
     cudaStreamSynchronize(s->stream);
     if (s->list_stats) cudaFreeHost(s->list_stats);
+    if (s->list_ev) cudaEventDestroy(s->list_ev);
     void* ptrs[] = {s->rec, s->lists, s->walk[0], s->walk[1], s->rng, s->table, s->base_prog, s->progs, s->palette, s->counters,
                     s->trace, s->r_bins, s->r_hits, s->r_de, s->r_img, s->r_stats, s->r_rad, s->r_dw};
     for (void* p : ptrs)

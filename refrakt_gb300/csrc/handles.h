@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <vector>
 
 #include "internal.h"
@@ -16,6 +17,13 @@ struct rf_flame {
     std::shared_ptr<const rfk::Registry> reg;
     uint64_t uid = 0;
     uint64_t version = 0;
+};
+
+// a bin grid and the screen affine that maps the plane to it
+struct ListView {
+    uint32_t w, h;
+    float ss[6];
+    bool operator==(const ListView& o) const { return w == o.w && h == o.h && std::equal(ss, ss + 6, o.ss); }
 };
 
 struct rf_sim {
@@ -73,13 +81,14 @@ struct rf_sim {
     // list per CTA and range
     unsigned char* lists = nullptr;
     size_t lists_bytes = 0, lists_refused = ~(size_t)0;  // refused: a size the device had no memory for
-    // after the first list call of a genome and grid (pinned, zero until they have arrived): the most points that a
-    // launch's lists held of one bin, the points in the call's lists, and those that found their list full; the call's
-    // points and launches (full ones)
+    // of the first list call of a genome, grid and view (pinned; there once list_ev has passed): the most points that
+    // a launch's lists held of one bin, the points in the call's lists, and those that found their list full; the
+    // call's points and launches (full ones)
     unsigned long long* list_stats = nullptr;
+    cudaEvent_t list_ev = nullptr;
     uint64_t list_points = 0;
     double list_launches = 1;
-    uint32_t list_wh[2] = {0, 0};
+    ListView list_view{};
     bool list_asked = false;
     // rf_render scratch
     float4* r_bins = nullptr;

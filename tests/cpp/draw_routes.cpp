@@ -24,8 +24,8 @@ static size_t live() {
     return n;
 }
 static void enqueue(std::function<void()> f) { g_queue.push_back(std::move(f)); g_queued++; }
-static void run_stream() {
-    while (!g_queue.empty()) {
+static void run_stream(size_t most = ~(size_t)0) {
+    for (; most && !g_queue.empty(); most--) {
         auto f = std::move(g_queue.front());
         g_queue.pop_front();
         f();
@@ -178,9 +178,43 @@ static int own_points() {
     return 0;
 }
 
+// a verdict is one grid's and one view's, and is not taken before its statistics have arrived
+static int own_view() {
+    Scene t(155648, 1024);
+    g_over = 0;
+    g_hottest = 1 << 19;
+    CHECK(t.draw(8192, 8192) == RF_OK && route() == kLists);
+    CHECK(t.draw(8192, 8192) == RF_OK && route() == kLists);  // nothing has arrived
+    cudaStreamSynchronize(nullptr);
+    CHECK(t.draw(8192, 8192) == RF_OK && route() == kRecords);
+    // another grid, asked for and drawn before the stream gets anywhere: the first grid's figures are not its own
+    g_hottest = 1;
+    CHECK(t.draw(8192, 4608) == RF_OK && route() == kLists);
+    cudaStreamSynchronize(nullptr);
+    CHECK(t.draw(8192, 4608) == RF_OK && route() == kLists);
+    // a view with a hot bin, after one without
+    const float center[2] = {0.1f, 0.2f};
+    g_hottest = 1 << 19;
+    CHECK(rf_flame_set_view(t.f, center, 5000.0f, 0.0f) == RF_OK);
+    CHECK(t.draw(8192, 4608) == RF_OK && route() == kLists);
+    cudaStreamSynchronize(nullptr);
+    CHECK(t.draw(8192, 4608) == RF_OK && route() == kRecords);
+    // and one without, after one with: the hot view's copy lands while the new view's is behind it
+    CHECK(rf_flame_set_view(t.f, center, 4000.0f, 0.0f) == RF_OK);
+    CHECK(t.draw(8192, 4608) == RF_OK && route() == kLists);  // hot, not arrived
+    g_hottest = 1;
+    CHECK(rf_flame_set_view(t.f, center, 3000.0f, 0.0f) == RF_OK);
+    CHECK(t.draw(8192, 4608) == RF_OK && route() == kLists);
+    run_stream(g_queue.size() - 1);  // all but the new view's copy
+    CHECK(t.draw(8192, 4608) == RF_OK && route() == kLists);
+    cudaStreamSynchronize(nullptr);
+    CHECK(t.draw(8192, 4608) == RF_OK && route() == kLists);
+    return 0;
+}
+
 int main(int argc, char** argv) {
     const std::string name = argc > 1 ? argv[1] : "";
-    const int rc = name == "failed_call" ? failed_call() : name == "own_points" ? own_points() : 2;
+    const int rc = name == "failed_call" ? failed_call() : name == "own_points" ? own_points() : name == "own_view" ? own_view() : 2;
     if (rc == 0) printf("OK\n");
     return rc;
 }
