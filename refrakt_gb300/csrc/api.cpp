@@ -223,6 +223,7 @@ int check_exchange(rf_sim* s) {
 // the geometry of a call's point lists in rf_sim.lists (reserve_lists)
 struct ListShape {
     uint32_t ranges = 0, range_bits = 0, cap = 0;
+    bool measure = false;  // with the statistics of measure_lists
 };
 
 // lists: the points go through them (splat 4); null: to the planes
@@ -334,7 +335,7 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
                 set[k].count = reinterpret_cast<uint32_t*>(s->lists + n * 64) + k * n;
             }
             RF_CUDA(launch_ranges(a, grid, set, reinterpret_cast<RangeState*>(s->lists + kListScratch) - kMaxRanges,
-                                  s->counters + 4, s->stream));
+                                  lists->measure ? s->counters + 4 : nullptr, s->stream));
         }
         s->cur ^= 1;
         s->pass += steps;
@@ -374,10 +375,8 @@ bool lists_suit(const rf_sim* s, const ListView& view) {
     return (double)h[0] * kListHot * s->list_launches < (double)h[1] + (h[1] == 0) && h[2] * 8 <= s->list_points;
 }
 
-// asks for the statistics of the call's launches (counters[4..6], launch_ranges), once per genome, grid and view (an
-// option: nothing fails for it)
+// asks for the statistics of the call's launches (counters[4..6], launch_ranges; an option: nothing fails for it)
 void measure_lists(rf_sim* s, const ListView& view, uint32_t passes) {
-    if (s->list_asked && s->list_view == view) return;
     s->list_asked = false;
     if ((s->list_ev || cudaEventCreateWithFlags(&s->list_ev, cudaEventDisableTiming) == cudaSuccess) &&
         (s->list_stats || cudaHostAlloc((void**)&s->list_stats, 24, cudaHostAllocDefault) == cudaSuccess)) {
@@ -420,7 +419,7 @@ bool reserve_lists(rf_sim* s, size_t nb, uint32_t passes, ListShape& shape) {
         }
         s->lists_bytes = bytes;
     }
-    shape = ListShape{ranges, bits, (uint32_t)cap};
+    shape = ListShape{ranges, bits, (uint32_t)cap, false};
     return true;
 }
 
@@ -436,9 +435,10 @@ int draw_passes(rf_sim* s, uint32_t passes, float4* bins, uint32_t* hits, uint32
     const ListView view{W, H, {ss[0], ss[1], ss[2], ss[3], ss[4], ss[5]}};
     // (a captured call takes records: a later call may move the lists)
     if (s->bin_layout == RF_BINS_AUTO && nb >= kListMinBins && !capturing(s->stream) && lists_suit(s, view) && reserve_lists(s, nb, passes, lists)) {
-        RF_CUDA(cudaMemsetAsync(s->counters + 4, 0, 3 * sizeof(unsigned long long), s->stream));
+        lists.measure = passes && !(s->list_asked && s->list_view == view);  // once per genome, grid and view
+        if (lists.measure) RF_CUDA(cudaMemsetAsync(s->counters + 4, 0, 3 * sizeof(unsigned long long), s->stream));
         const int rc = launch_passes(s, passes, false, true, bins, hits, W, H, ss, &lists);
-        if (!rc && passes) measure_lists(s, view, passes);
+        if (!rc && lists.measure) measure_lists(s, view, passes);
         return rc;
     }
     if (s->rec_n < nb) {

@@ -62,7 +62,7 @@ struct RangeArgs {
     RangeState* state;  // per range
     float4* bins;
     uint32_t* hits;
-    unsigned long long* stats;  // launch_ranges
+    unsigned long long* stats;  // launch_ranges (may be null)
 };
 constexpr uint32_t kRangeThreads = 512, kMergeCtas = 1024;
 
@@ -83,8 +83,8 @@ __global__ void __launch_bounds__(256) range_count_kernel(const uint32_t* __rest
     __syncthreads();
     if (threadIdx.x == 0) {
         state[blockIdx.x] = RangeState{s_sum[0] < (1u << 24) ? 1u : 0u, 0u};
-        atomicAdd(stats + 1, s_sum[0]);
-        if (s_sum[1]) atomicAdd(stats + 2, s_sum[1]);
+        if (stats) atomicAdd(stats + 1, s_sum[0]);
+        if (stats && s_sum[1]) atomicAdd(stats + 2, s_sum[1]);
     }
 }
 
@@ -181,6 +181,7 @@ __device__ __forceinline__ void range_merge(const RangeArgs& R, uint32_t cta) {
                 __stcs(R.hits + first + i0 + kStep * u, h[u] + c[u]);
             }
     }
+    if (!R.stats) return;
     most = __reduce_max_sync(0xffffffffu, most);
     if ((threadIdx.x & 31) == 0 && most > *(volatile unsigned long long*)R.stats) atomicMax(R.stats, (unsigned long long)most);
 }

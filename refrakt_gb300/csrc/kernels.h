@@ -31,7 +31,8 @@ struct RangeScratch {
 struct RangeState {
     uint32_t unit, mixed;  // fewer than 2^24 points in the range's lists; among them some of opacity other than 1
 };
-// the lists of a launch of `ctas` CTAs with splat 4 into its planes.  stats: [0] raised to the most points that
+// the lists of a launch of `ctas` CTAs with splat 4 into its planes.  stats (may be null; every step waits for
+// it some 0.4 us longer): [0] raised to the most points that
 // one bin got from them, [1] grows by the points in the lists, [2] by those that found their list full
 cudaError_t launch_ranges(const ChaosArgs& a, uint32_t ctas, const RangeScratch set[2], RangeState* state,
                           unsigned long long* stats, cudaStream_t st);

@@ -106,7 +106,7 @@ int spec_compile(const std::string&, std::vector<char>&) { return RF_ERR_UNSUPPO
 bool spec_available(std::string*) { return false; }
 cudaError_t launch_ranges(const ChaosArgs&, uint32_t, const RangeScratch[2], RangeState*, unsigned long long* stats, cudaStream_t) {
     const unsigned long long h = g_hottest, n = g_points, o = g_over;
-    enqueue([=] {
+    if (stats) enqueue([=] {
         stats[0] = std::max(stats[0], h);
         stats[1] += n;
         stats[2] += o;
@@ -153,7 +153,7 @@ static int failed_call() {
     Scene t(155648, 1024);
     CHECK(t.draw(8192, 8192) == RF_OK && route() == kLists);
     g_fail_memset = t.s->counters + 4;
-    CHECK(t.draw(8192, 8192) != RF_OK && !g_fail_memset);
+    CHECK(t.draw(8191, 8192) != RF_OK && !g_fail_memset);
     CHECK(rf_set_bin_layout(t.s, RF_BINS_DIRECT) == RF_OK);
     CHECK(t.draw(640, 360) == RF_OK && route() == kPlanes && g_last.ranges == 0);
     CHECK(rf_set_bin_layout(t.s, RF_BINS_AUTO) == RF_OK);
