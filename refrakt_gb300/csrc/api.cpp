@@ -58,6 +58,7 @@ namespace {
 constexpr size_t kListBytes = 16ull << 30;  // the lists' memory at most: 256 passes of 2.5 M walkers at three times an even spread
 constexpr size_t kListMinBins = 1u << 25;
 constexpr uint64_t kListHot = 1024;
+constexpr uint32_t kListTurns = 4;  // times that a genome's lists are released for records: each costs a wait and an allocation
 constexpr size_t kListScratch = ((size_t)72 << kMaxRangeBits) + kMaxRanges * sizeof(RangeState);  // two sets of scratch planes
 constexpr size_t kInterleaveMinBytes = 256ull << 20;  // bins + counts above ~2x L2: interleave
 
@@ -375,6 +376,12 @@ bool lists_suit(const rf_sim* s, const ListView& view) {
     return (double)h[0] * kListHot * s->list_launches < (double)h[1] + (h[1] == 0) && h[2] * 8 <= s->list_points;
 }
 
+void release_lists(rf_sim* s) {
+    cudaFree(s->lists);  // (waits for the launches that use them)
+    s->lists = nullptr;
+    s->lists_bytes = 0;
+}
+
 // asks for the statistics of the call's launches (counters[4..6], launch_ranges; an option: nothing fails for it)
 void measure_lists(rf_sim* s, const ListView& view, uint32_t passes) {
     s->list_asked = false;
@@ -390,37 +397,44 @@ void measure_lists(rf_sim* s, const ListView& view, uint32_t passes) {
     if (!s->list_asked) cudaGetLastError();
 }
 
-// the lists' memory for a call of `passes` passes, four times an even spread over the ranges where it fits, at
-// least 1.25 times; false: it does not, or the sim's domains are spread over clusters
-bool reserve_lists(rf_sim* s, size_t nb, uint32_t passes, ListShape& shape) {
+// the lists of a call of `passes` passes within `budget` bytes: four times an even spread over the ranges where it fits,
+// at least 1.25 times; 0 bytes: it does not, or the sim's domains are spread over clusters
+size_t list_shape(const rf_sim* s, size_t nb, uint32_t passes, size_t budget, ListShape& shape) {
     // ranges of 2^21 bins; of 2^20 where more than 2^23 points of a launch fall into one on average, so that
     // most stay below the 2^24 of a single reduction per point (637 M points on 8192 x 8192 bins: 13.9 -> 11.7 ms)
     uint32_t bits = kMaxRangeBits;
     if ((s->N * std::min(passes, s->L) >> 23) << bits > nb && nb <= (uint64_t)kMaxRanges << (bits - 1)) bits--;
     const uint32_t ranges = (uint32_t)((nb + (1u << bits) - 1) >> bits);
-    if (s->splat != RF_SPLAT_AUTO || ranges > kMaxRanges || (s->spec && cluster_for_launch(s, true) > 1)) return false;
+    if (s->splat != RF_SPLAT_AUTO || ranges > kMaxRanges || (s->spec && cluster_for_launch(s, true) > 1)) return 0;
     const uint64_t ctas = s->N / s->slots, points = (uint64_t)s->slots * std::min(passes, s->L);  // of a CTA
     const size_t head = kListScratch + ((ctas * ranges + 3) & ~(uint64_t)3) * 4;
-    if (head >= kListBytes) return false;
-    const uint64_t fit = (kListBytes - head) / (ctas * ranges * 8);
+    if (head >= budget) return 0;
+    const uint64_t fit = (budget - head) / (ctas * ranges * 8);
     const uint64_t cap = std::min<uint64_t>({points, std::max<uint64_t>(4 * points / ranges, 256), fit});
-    if (4 * cap * ranges < 5 * points || chaos_smem(s->slots, s->prog_words, s->L, 0, 1, ranges) > kMaxCtaSmem) return false;
-    const size_t bytes = head + ctas * ranges * cap * 8;
-    if (s->lists_bytes < bytes) {
-        if (bytes >= s->lists_refused) return false;
-        cudaFree(s->lists);
-        s->lists = nullptr;
-        s->lists_bytes = 0;
-        if (cudaMalloc((void**)&s->lists, bytes) != cudaSuccess ||
-            cudaMemsetAsync(s->lists, 0, kListScratch, s->stream) != cudaSuccess) {
-            cudaGetLastError();
-            s->lists_refused = bytes;
-            return false;
-        }
-        s->lists_bytes = bytes;
-    }
+    if (4 * cap * ranges < 5 * points || chaos_smem(s->slots, s->prog_words, s->L, 0, 1, ranges) > kMaxCtaSmem) return 0;
     shape = ListShape{ranges, bits, (uint32_t)cap, false};
-    return true;
+    return head + ctas * ranges * cap * 8;
+}
+
+// the lists' memory for a call, at most kListBytes, and no more than the records would take (32 bytes a bin) or an
+// eighth of what the device has free: the rest is left to the caller's later allocations.  false: records
+bool reserve_lists(rf_sim* s, size_t nb, uint32_t passes, ListShape& shape) {
+    const size_t want = list_shape(s, nb, passes, kListBytes, shape);
+    if (want > s->lists_bytes && want < s->lists_refused) {
+        size_t free = 0, total = 0;
+        if (cudaMemGetInfo(&free, &total) != cudaSuccess) { cudaGetLastError(); free = 0; }
+        const size_t get = list_shape(s, nb, passes, std::min(kListBytes, std::max(32 * nb, (free + s->lists_bytes) / 8)), shape);
+        if (get > s->lists_bytes) {
+            release_lists(s);
+            if (cudaMalloc((void**)&s->lists, get) == cudaSuccess &&
+                cudaMemsetAsync(s->lists, 0, kListScratch, s->stream) == cudaSuccess)
+                s->lists_bytes = get;
+            else
+                cudaGetLastError();
+        }
+        if (s->lists_bytes < want) s->lists_refused = want;
+    }
+    return list_shape(s, nb, passes, std::min(kListBytes, s->lists_bytes), shape) != 0;
 }
 
 // The drawing passes into the caller's planes, or — for histograms well above L2 with a count
@@ -434,7 +448,15 @@ int draw_passes(rf_sim* s, uint32_t passes, float4* bins, uint32_t* hits, uint32
     ListShape lists;
     const ListView view{W, H, {ss[0], ss[1], ss[2], ss[3], ss[4], ss[5]}};
     // (a captured call takes records: a later call may move the lists)
-    if (s->bin_layout == RF_BINS_AUTO && nb >= kListMinBins && !capturing(s->stream) && lists_suit(s, view) && reserve_lists(s, nb, passes, lists)) {
+    bool listed = s->bin_layout == RF_BINS_AUTO && nb >= kListMinBins && !capturing(s->stream);
+    if (listed && !lists_suit(s, view)) {
+        // records from here on; their memory comes in the place of the lists'
+        if (s->lists) s->list_turns++;
+        release_lists(s);
+        listed = false;
+    }
+    // (a program whose views turn and turn again stays with records: kListTurns)
+    if (listed && s->list_turns < kListTurns && reserve_lists(s, nb, passes, lists)) {
         lists.measure = passes && !(s->list_asked && s->list_view == view);  // once per genome, grid and view
         if (lists.measure) RF_CUDA(cudaMemsetAsync(s->counters + 4, 0, 3 * sizeof(unsigned long long), s->stream));
         const int rc = launch_passes(s, passes, false, true, bins, hits, W, H, ss, &lists);
@@ -850,6 +872,7 @@ int rf_warmup(rf_sim* s, rf_flame* f, uint32_t num_passes, float tss_width) {
         reset_exchange_tuning(s);
         s->auto_tile_state = 0;
         s->list_asked = false;
+        s->list_turns = 0;
     }
     if (s->d.specialize >= 0) {
         const void* k = nullptr;

@@ -80,7 +80,7 @@ struct rf_sim {
     // the list splat's memory: two sets of scratch planes of one range (all zero between calls), then a count and a
     // list per CTA and range
     unsigned char* lists = nullptr;
-    size_t lists_bytes = 0, lists_refused = ~(size_t)0;  // refused: a size the device had no memory for
+    size_t lists_bytes = 0, lists_refused = ~(size_t)0;  // refused: a size it had too little memory for
     // of the first list call of a genome, grid and view (pinned; there once list_ev has passed): the most points that
     // a launch's lists held of one bin, the points in the call's lists, and those that found their list full; the
     // call's points and launches (full ones)
@@ -90,6 +90,7 @@ struct rf_sim {
     double list_launches = 1;
     ListView list_view{};
     bool list_asked = false;
+    uint32_t list_turns = 0;  // times that the genome turned to records
     // rf_render scratch
     float4* r_bins = nullptr;
     uint32_t* r_hits = nullptr;

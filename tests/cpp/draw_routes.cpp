@@ -212,9 +212,43 @@ static int own_view() {
     return 0;
 }
 
+// the lists take what the records would or an eighth of the free memory, and nothing when records take over
+static int memory() {
+    const size_t gb = (size_t)1 << 30, records = (size_t)32 << 26;
+    g_over = 0;
+    g_hottest = 1;
+    for (size_t free : {3 * gb, 8 * gb, 30 * gb, 200 * gb}) {
+        g_device = (size_t)280 << 30;
+        Scene t(622592, 4096);
+        const size_t held = live();
+        g_device = held + free;
+        for (int k = 0; k < 4; k++) {  // 159 M points a launch: 5.1e9 bytes of lists at four times an even spread, 1.6 at 1.25
+            CHECK(t.draw(8192, 8192, 512) == RF_OK && route() == kLists);
+            CHECK(live() - held <= std::max(free / 8, records));
+        }
+        CHECK(free < 200 * gb || live() - held > (size_t)5100000000);
+    }
+    g_device = (size_t)280 << 30;
+    Scene t(155648, 1024);
+    const size_t before = live();
+    for (int turn = 0; turn < 7; turn++) {
+        const float center[2] = {0.01f * turn, 0.0f};
+        CHECK(rf_flame_set_view(t.f, center, 4000.0f, 0.0f) == RF_OK);
+        g_hottest = 1 << 19;
+        CHECK(t.draw(8192, 8192) == RF_OK);
+        CHECK(route() == (turn < 4 ? kLists : kRecords));  // views that turn and turn again stay with records
+        cudaStreamSynchronize(nullptr);
+        CHECK(t.draw(8192, 8192) == RF_OK && route() == kRecords);
+        CHECK(live() == before + records);
+    }
+    CHECK(rf_flame_set_xform_value(t.f, 0, "color", 0.7f) == RF_OK && rf_warmup(t.s, t.f, 3, 0.0f) == RF_OK);
+    CHECK(t.draw(8192, 8192) == RF_OK && route() == kLists);  // another genome
+    return 0;
+}
+
 int main(int argc, char** argv) {
     const std::string name = argc > 1 ? argv[1] : "";
-    const int rc = name == "failed_call" ? failed_call() : name == "own_points" ? own_points() : name == "own_view" ? own_view() : 2;
+    const int rc = name == "failed_call" ? failed_call() : name == "own_points" ? own_points() : name == "own_view" ? own_view() : name == "memory" ? memory() : 2;
     if (rc == 0) printf("OK\n");
     return rc;
 }
