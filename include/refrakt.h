@@ -294,6 +294,11 @@ RF_API int  rf_sim_counters(rf_sim* s, uint64_t out[3]);
  * shaders/tonemap.glsl).  All pointers are device pointers.
  * ---------------------------------------------------------------------------------------- */
 
+/* The image passes' scratch comes from a memory pool of the library, which keeps up to 64 MB per device between
+   calls and gives them back when a simulation, batch or denoiser is destroyed; this call gives the
+   current device's unused scratch back at any other time. */
+RF_API int rf_release_scratch(void);
+
 /* Adaptive density estimation: out (float4 per bin) = every bin with a > 0 spread over a disc
    of radius max(min, min(R, int(R / a^curve))), kernel (1 - d^2) * (2/pi) / r^2 with
    d = |offset| / (r + 0.5); r = 0 copies the bin.  R <= 100 (main.cpp:502).  A bin whose colour is
@@ -327,7 +332,7 @@ RF_API int rf_tonemap_filter(const float* rgba, uint32_t width, uint32_t height,
    to 12 and ss dividing 8 the estimator's output stays in on-chip memory (each 32 x 8 tile is
    tonemapped where it is estimated) and the density sum comes from the radius pass, so the FP32
    output plane is never written; otherwise the passes run one after another.  Scratch comes from
-   cudaMallocAsync on `stream`. */
+   the library's pool (rf_release_scratch), in the order of `stream`. */
 RF_API int rf_density_tonemap(const float* bins_rgba, uint32_t width, uint32_t height, int radius, int min_radius,
                               float curve, uint32_t ss, float gamma, float brightness, float vibrancy, float k2,
                               float* out_f32, uint8_t* out_rgba8, void* stream);

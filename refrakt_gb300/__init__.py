@@ -13,7 +13,7 @@ import ctypes
 import json
 import os
 
-__all__ = ["RefraktError", "FlameCompiler", "Flame", "Sim", "library", "build", "density_estimate",
+__all__ = ["RefraktError", "FlameCompiler", "Flame", "Sim", "library", "build", "release_scratch", "density_estimate",
            "tonemap", "hist_stats", "shuffle_generate", "probe_xform", "write_png", "render",
            "SYNTH_SMALL", "SYNTH_RANDOM", "SYNTH_CONTRACT", "SYNTH_SPACEFILL",
            "SPLAT_AUTO", "SPLAT_GLOBAL", "SPLAT_WARP", "BINS_AUTO", "BINS_DIRECT", "BINS_INTERLEAVED", "Batch", "Denoiser", "denoiser_features", "gemm_bf16",
@@ -155,6 +155,7 @@ _SIGS = {
     "rf_set_splat_tile": ([ctypes.c_void_p] + [ctypes.c_uint32] * 4, ctypes.c_int),
     "rf_set_bin_layout": ([ctypes.c_void_p, ctypes.c_int], ctypes.c_int),
     "rf_sim_counters": ([ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint64)], ctypes.c_int),
+    "rf_release_scratch": ([], ctypes.c_int),
     "rf_density_estimate": ([ctypes.c_void_p, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_int, ctypes.c_int,
                              ctypes.c_float, ctypes.c_void_p, ctypes.c_void_p], ctypes.c_int),
     "rf_tonemap_filter": ([ctypes.c_void_p, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_uint32, ctypes.c_float,
@@ -624,6 +625,11 @@ class Batch:
 
 def render(sim, flame, *a, **k):
     return sim.render(flame, *a, **k)
+
+
+def release_scratch():
+    """Gives the image passes' unused device scratch back (rf_release_scratch)."""
+    _check(library().rf_release_scratch())
 
 
 def density_estimate(bins_rgba, width, height, radius, min_radius, curve, out, stream=None):

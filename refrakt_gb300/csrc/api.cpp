@@ -1106,6 +1106,11 @@ int rf_density_tonemap(const float* in, uint32_t w, uint32_t h, int radius, int 
     return RF_OK;
 }
 
+int rf_release_scratch(void) {
+    RF_CUDA(scratch_trim());
+    return RF_OK;
+}
+
 int rf_hist_stats(const float* rgba, uint32_t w, uint32_t h, double* out3, void* stream) {
     if (!rgba || !out3) return fail(RF_ERR_INVALID_ARG, "rf_hist_stats: null argument");
     cudaStream_t st = (cudaStream_t)stream;

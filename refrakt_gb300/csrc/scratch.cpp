@@ -5,7 +5,7 @@
 // each image pays for mapping its scratch again in every call: density_tonemap of 640 x 360 bins took
 // 243 us after a synchronisation and 84 us without one.  This pool keeps up to kScratchKeep bytes --
 // the radius plane of a 67-million-bin grid -- and gives them back when a simulation, batch or denoiser
-// is destroyed.  Pools order their memory by stream, so calls on several streams and threads share it
+// is destroyed, or at rf_release_scratch.  Pools order their memory by stream, so calls on several streams and threads share it
 // safely.  During stream capture the allocation becomes a node of the graph, as before, from the
 // default pool.
 #include "scratch.h"
@@ -53,8 +53,9 @@ cudaError_t scratch_alloc(void** p, size_t bytes, cudaStream_t st) {
     return mp ? cudaMallocFromPoolAsync(p, bytes, mp, st) : cudaMallocAsync(p, bytes, st);
 }
 
-void scratch_trim() {
-    if (cudaMemPool_t mp = pool(false)) cudaMemPoolTrimTo(mp, 0);
+cudaError_t scratch_trim() {
+    cudaMemPool_t mp = pool(false);
+    return mp ? cudaMemPoolTrimTo(mp, 0) : cudaSuccess;
 }
 
 }  // namespace rfk

@@ -13,6 +13,6 @@ cudaError_t scratch_alloc(T** p, size_t count, cudaStream_t st) {
     return scratch_alloc((void**)p, count * sizeof(T), st);
 }
 // gives the current device's unused scratch back
-void scratch_trim();
+cudaError_t scratch_trim();
 
 }  // namespace rfk

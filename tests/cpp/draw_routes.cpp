@@ -99,7 +99,7 @@ int filter_taps(uint32_t, float, int, float*) { return 1; }
 cudaError_t launch_tonemap_filter(const float4*, uint32_t, uint32_t, uint32_t, float, int, float, float, float, float, const double*, float4*, uchar4*, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_density_tonemap(const float4*, uint32_t, uint32_t, int, int, float, uint32_t, float, float, float, float, float4*, uchar4*, uint8_t*, const float*, double*, float4*, cudaStream_t) { return cudaSuccess; }
 cudaError_t scratch_alloc(void** p, size_t n, cudaStream_t) { return cudaMalloc(p, n); }
-void scratch_trim() {}
+cudaError_t scratch_trim() { return cudaSuccess; }
 int spec_kernel(const std::vector<uint32_t>&, int, int, int, const void**, SpecKind, int, int, int, int) { return RF_ERR_UNSUPPORTED; }
 std::string spec_source(const std::vector<uint32_t>&, int, int, SpecKind, int, int, int, int) { return ""; }
 int spec_compile(const std::string&, std::vector<char>&) { return RF_ERR_UNSUPPORTED; }

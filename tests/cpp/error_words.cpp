@@ -57,7 +57,7 @@ cudaError_t launch_adam(float*, const float*, float*, float*, const AdamLayers&,
 cudaError_t launch_stats(const float4*, uint32_t, uint32_t, double*, cudaStream_t) { return cudaSuccess; }
 cudaError_t launch_features(const float4*, uint64_t, float, const double*, const float4*, float, __nv_bfloat16*, cudaStream_t) { return cudaSuccess; }
 cudaError_t scratch_alloc(void** p, size_t n, cudaStream_t) { return cudaMalloc(p, n); }
-void scratch_trim() {}
+cudaError_t scratch_trim() { return cudaSuccess; }
 }  // namespace rfk
 
 #define CHECK(x) do { if (!(x)) { printf("line %d: %s (%s)\n", __LINE__, #x, g_message.c_str()); return 1; } } while (0)
