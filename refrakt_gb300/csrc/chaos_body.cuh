@@ -150,9 +150,9 @@ __device__ __forceinline__ float4 cluster_load(const float4* local, uint32_t ran
 //
 // CLUSTER = K > 1 spreads a mixing domain over the K CTAs of a cluster (SLOTS = its slots / K), for
 // simulations whose domains are fewer than the SMs: with one CTA per domain the others idle.  The
-// arrival on the pass's cluster barrier comes right after the walker's store, the wait before the next
-// pass's first read, so the splat and the group's xform draw (as PIPE draws it) pass under it.  What is
-// left is one warp's chain per pass: 65,536 walkers of the three-xform genome in 2048-slot domains take
+// arrival on the pass's cluster barrier comes after the last walker's store and the group's xform draw (as
+// PIPE draws it: the next pass reads both behind the barrier), the wait before the next pass's first
+// read, so the splat alone passes under it.  What is left is one warp's chain per pass: 65,536 walkers of the three-xform genome in 2048-slot domains take
 // 3.9 us per pass on 32 CTAs and 2.7 us on 128 (16.6 -> 24.0 Gpoints/s), in 4096-slot ones 6.3 us on 16
 // and 4.4 us on 128.
 template <int THREADS, int SPT, class Eval, int SPLAT = -1, int RESET = -1, int PIPE = 0, int CLUSTER = 1>

@@ -621,7 +621,7 @@ struct WgradArgs {
     WgradLayer layer[kMaxWgradLayers];
     uint32_t layers, bars;
     int* error;
-    // the head's bias gradient, by the last CTAs of the grid
+    // the head's bias gradient, by the grid's first bias_first CTAs
     uint32_t bias_first;
     const __nv_bfloat16* bias_dz;
     float* bias_out;

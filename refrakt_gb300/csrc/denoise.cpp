@@ -441,9 +441,6 @@ int rf_denoiser_train_step(rf_denoiser* D, const void* feats, const float* targe
     if (!D || !feats || !target_rgb) return fail(RF_ERR_INVALID_ARG, "rf_denoiser_train_step: null argument");
     if (int rc = check_shape(D, n, h, w)) return rc;
     cudaSetDevice(D->device);
-    // the weight-gradient products run over whole blocks of 8 pixels at every level
-    if ((uint64_t)n * (h / 8) * (w / 8) % 8)
-        return fail(RF_ERR_CUDA, "rf_denoiser_train_step: batch x height / 8 x width / 8 must be a multiple of 8");
     if (int rc = train(D, static_cast<const __nv_bfloat16*>(feats), target_rgb, lr)) return rc;
     if (loss) {
         double l = 0;
