@@ -236,10 +236,13 @@ enum rf_splat { RF_SPLAT_AUTO = 0, RF_SPLAT_GLOBAL = 1, RF_SPLAT_WARP = 2, RF_SP
    records {RGBA, count} in a library buffer merged into the caller's planes at the end of each
    draw call (INTERLEAVED: one DRAM sector per point instead of two; pays for itself when the bins
    exceed L2).  AUTO: INTERLEAVED when a count plane is given and the planes exceed 256 MB; from
-   2^25 bins on DIRECT through lists of points per bin range (library memory of about 32 bytes a
-   point of one launch, at most 16 GB and the records' 32 bytes a bin or an eighth of the free device
-   memory) that are added range by range in L2, but where those do not fit, a bin takes more than 1/1024 of the points (the lists are
-   freed then), or the call is captured. */
+   2^25 bins on that or DIRECT through lists of points per bin range, added range by range in L2,
+   whichever is faster: for a genome, grid and view one call of each form is timed with CUDA events (of
+   equal passes, without a host wait; a choice stands for 16 calls while genomes or views change).  The
+   records take 32 bytes a bin of library memory, the lists about 32 bytes a point of one launch, at
+   most 16 GB and the records' memory or an eighth of the free device memory, one in the other's place;
+   where there is no memory for one form the other serves.  A captured call takes records that an
+   earlier call has left, else the planes directly. */
 enum rf_bin_layout { RF_BINS_AUTO = 0, RF_BINS_DIRECT = 1, RF_BINS_INTERLEAVED = 2 };
 RF_API int  rf_set_bin_layout(rf_sim* s, int layout);
 RF_API int  rf_draw_to_bins(rf_sim* s, rf_flame* f, float* bins_rgba, uint32_t* bins_hits,

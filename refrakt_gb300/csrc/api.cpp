@@ -57,8 +57,8 @@ namespace {
 
 constexpr size_t kListBytes = 16ull << 30;  // the lists' memory at most: 256 passes of 2.5 M walkers at three times an even spread
 constexpr size_t kListMinBins = 1u << 25;
-constexpr uint64_t kListHot = 1024;
-constexpr uint32_t kListTurns = 4;  // times that a genome's lists are released for records: each costs a wait and an allocation
+constexpr uint32_t kListStands = 16;  // calls for which one genome's and view's choice stands for the next: a change of form costs
+                                      // an allocation (8192 x 8192 bins: 3 ms)
 constexpr size_t kListScratch = ((size_t)72 << kMaxRangeBits) + kMaxRanges * sizeof(RangeState);  // two sets of scratch planes
 constexpr size_t kInterleaveMinBytes = 256ull << 20;  // bins + counts above ~2x L2: interleave
 
@@ -224,12 +224,18 @@ int check_exchange(rf_sim* s) {
 // the geometry of a call's point lists in rf_sim.lists (reserve_lists)
 struct ListShape {
     uint32_t ranges = 0, range_bits = 0, cap = 0;
-    bool measure = false;  // with the statistics of measure_lists
 };
 
-// lists: the points go through them (splat 4); null: to the planes
+// the way of a drawing call's points
+struct DrawWay {
+    const ListShape* lists = nullptr;  // through them (splat 4); null: to the planes
+    bool tune = true;                  // RF_EXCHANGE_AUTO may time launches
+    cudaEvent_t begin = nullptr;       // recorded before the first launch
+};
+
 int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4* bins, uint32_t* hits,
-                  uint32_t W, uint32_t H, const float ss[6], const ListShape* lists = nullptr) {
+                  uint32_t W, uint32_t H, const float ss[6], const DrawWay& way = {}) {
+    const ListShape* lists = way.lists;
     uint32_t done = 0;
     while (done < passes) {
         const uint32_t steps = std::min(s->L, passes - done);
@@ -296,7 +302,7 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
         // (RF_SPLAT_AUTO's tile is timed first, in the pipelined form; the exchange after it)
         const bool tile_busy = tile_warmup || tile_timed >= 0 || (s->splat == RF_SPLAT_AUTO && s->auto_tile_state >= 2);
         const bool timed = s->spec && cluster_for_launch(s, false) == 1;  // else the cluster form, untimed
-        const int want = timed ? exchange_for_launch(s, a.draw, steps, !tile_busy && !a.ranges, &measure) : 0;
+        const int want = timed ? exchange_for_launch(s, a.draw, steps, !tile_busy && !a.ranges && way.tune, &measure) : 0;
         const int pipe = want && s->spec && use_pipe(s, tile_bins) ? 1 : 0;
         // one CTA per mixing domain, or a cluster of `cl`
         const int cl = cluster_for_launch(s, !want);
@@ -318,6 +324,7 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
             return fail(RF_ERR_CAPACITY, "splat tile of " + std::to_string(tile_bins) +
                                          " bins exceeds the shared memory beside " + std::to_string(s->slots) +
                                          " walker slots");
+        if (way.begin && done == 0 && cudaEventRecord(way.begin, s->stream) != cudaSuccess) cudaGetLastError();
         if (measure >= 0 && cudaEventRecord(s->tune_ev[2 * measure], s->stream) != cudaSuccess) measure = -1;
         if (tile_timed >= 0 && cudaEventRecord(s->tile_ev[2 * tile_timed], s->stream) != cudaSuccess) tile_timed = -1;
         cudaError_t e = s->spec ? launch_spec(s->spec, (int)threads, (int)local, a, grid,
@@ -335,8 +342,7 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
                 set[k].rgba2 = set[k].rgba + n;
                 set[k].count = reinterpret_cast<uint32_t*>(s->lists + n * 64) + k * n;
             }
-            RF_CUDA(launch_ranges(a, grid, set, reinterpret_cast<RangeState*>(s->lists + kListScratch) - kMaxRanges,
-                                  lists->measure ? s->counters + 4 : nullptr, s->stream));
+            RF_CUDA(launch_ranges(a, grid, set, reinterpret_cast<RangeState*>(s->lists + kListScratch) - kMaxRanges, s->stream));
         }
         s->cur ^= 1;
         s->pass += steps;
@@ -356,45 +362,74 @@ int launch_passes(rf_sim* s, uint32_t passes, bool first_run, bool draw, float4*
     return RF_OK;
 }
 
-// Point lists (splat 4) for the drawing launches of a call on a grid far above L2, instead of interleaved
-// records.  80 M points of the space-filling genome, of the 1080p genome, ms with records and with lists: 8192 x
-// 8192 bins 3.94, 1.84 and 3.49, 2.47 (637 M points 24.9, 11.7); 8192 x 4608 3.26, 1.65 and 2.50, 2.28; 6000 x
-// 4000 2.58, 1.56 and 1.88, 2.28; 4099 x 3301 1.68, 1.49 and 1.69, 2.29: from kListMinBins bins on.  Not for hot bins, whose points the lists' second step adds one after another while the
-// records' reductions pass under the chaos game (62 M points of the 5-xform genome on 5000 x 4001 bins, 0.3 % of
-// them in one bin: 1.63 ms with records, 1.80 with lists): the first call measures its points (not the caller's
-// plane, which may hold others), later ones take records above a share of 1 / kListHot in one bin or where an
-// eighth of the points found their list full.
-// The verdict holds for the genome, the grid and the view that it was taken for, once its statistics have arrived.
-bool lists_suit(const rf_sim* s, const ListView& view) {
-    if (!s->list_asked || !(s->list_view == view)) return true;
-    const cudaError_t q = cudaEventQuery(s->list_ev);
-    if (q != cudaSuccess) {
-        if (q == cudaErrorNotReady && cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError();  // clear only this status
-        return true;
+// Point lists (splat 4) for the drawing launches of a call on a grid far above L2, instead of interleaved records.
+// Which form is the faster one depends on how the genome's points spread over bins and ranges: records gain where L2
+// holds the bins that most points fall into, lists lose to hot bins, full lists and ranges of 2^24 points and more.
+// Calls of 2.5 M walkers x 32 and x 256 passes, ms with records and with lists, of the space-filling genome, the 1080p
+// genome and two others of the batch workload's kind: 8192 x 8192 bins 3.95, 1.80 and 25.3, 11.6; 3.20, 2.49 and
+// 19.6, 17.9; 2.57, 3.06 and 15.1, 25.2; 2.66, 2.70 and 15.4, 19.4; 8192 x 4608 bins 3.25, 1.58 and 22.1, 13.8;
+// 2.14, 2.68 and 13.1, 18.0; (the third: hot bins); 2.09, 2.77 and 12.6, 20.2.  So a call of each form is timed with
+// CUDA events, on one genome, grid and view and with equal passes, and the faster form taken from then on.  The first
+// form is the last decision's; without one, lists up to 1.25 points of a launch per bin and records above (lists over
+// records, mean of the genomes without hot bins: 0.77 of 12 on 8192 x 8192 bins at 1.2 points; 0.92 and 1.10 of 7 on
+// 8192 x 4608 at 1.05 and 4.2).
+// While calls change from one genome or view to another, a decision stands for kListStands calls.
+// 1: lists, 0: records; *timed: 0 / 1 when the call is the first / second one timed, else -1.  (No host wait.)
+int lists_for_call(rf_sim* s, const ListView& view, uint32_t passes, int* timed) {
+    *timed = -1;
+    s->list_calls++;
+    if (s->list_step == 2) {
+        const cudaError_t q = cudaEventQuery(s->list_ev[3]);
+        if (q == cudaErrorNotReady) {
+            if (cudaPeekAtLastError() == cudaErrorNotReady) cudaGetLastError();  // clear only this status
+        } else {
+            float t0 = 0.0f, t1 = 0.0f;
+            const bool ok = q == cudaSuccess && cudaEventElapsedTime(&t0, s->list_ev[0], s->list_ev[1]) == cudaSuccess &&
+                            cudaEventElapsedTime(&t1, s->list_ev[2], s->list_ev[3]) == cudaSuccess;
+            if (!ok) cudaGetLastError();
+            s->list_form = ok ? (t1 < t0) != (s->list_first != 0) : 0;
+            s->list_step = 3;
+            s->list_calls = 0;
+        }
     }
-    const unsigned long long* h = s->list_stats;
-    return (double)h[0] * kListHot * s->list_launches < (double)h[1] + (h[1] == 0) && h[2] * 8 <= s->list_points;
+    const bool same = s->list_view == view;
+    if (s->list_step == 3 && !same && s->list_calls >= kListStands) s->list_step = 0;
+    if (s->list_step == 1 && same && passes == s->list_passes) {
+        *timed = 1;
+        return !s->list_first;
+    }
+    if (s->list_step < 2) {
+        const uint64_t points = s->N * std::min(passes, s->L), bins = (uint64_t)view.w * view.h;
+        if (s->list_form >= 0) s->list_first = s->list_form;
+        else if (s->list_step == 0 || !same) s->list_first = 4 * points <= 5 * bins;
+        s->list_view = view;
+        s->list_passes = passes;
+        *timed = 0;
+    }
+    return s->list_step < 3 ? s->list_first : s->list_form;
 }
 
 void release_lists(rf_sim* s) {
     cudaFree(s->lists);  // (waits for the launches that use them)
     s->lists = nullptr;
     s->lists_bytes = 0;
+    s->lists_refused = ~(size_t)0;
 }
-
-// asks for the statistics of the call's launches (counters[4..6], launch_ranges; an option: nothing fails for it)
-void measure_lists(rf_sim* s, const ListView& view, uint32_t passes) {
-    s->list_asked = false;
-    if ((s->list_ev || cudaEventCreateWithFlags(&s->list_ev, cudaEventDisableTiming) == cudaSuccess) &&
-        (s->list_stats || cudaHostAlloc((void**)&s->list_stats, 24, cudaHostAllocDefault) == cudaSuccess)) {
-        // (an earlier request's copy may still be on its way; the event is this one's from here on)
-        s->list_asked = cudaMemcpyAsync(s->list_stats, s->counters + 4, 24, cudaMemcpyDeviceToHost, s->stream) == cudaSuccess &&
-                        cudaEventRecord(s->list_ev, s->stream) == cudaSuccess;
-        s->list_points = s->N * passes;
-        s->list_launches = (double)passes / std::min(passes, s->L);
-        s->list_view = view;
-    }
-    if (!s->list_asked) cudaGetLastError();
+void release_records(rf_sim* s) {
+    if (s->rec_captured) return;
+    cudaFree(s->rec);
+    s->rec = nullptr;
+    s->rec_n = 0;
+}
+cudaError_t reserve_records(rf_sim* s, size_t nb) {
+    if (s->rec_n >= nb) return cudaSuccess;
+    cudaFree(s->rec);
+    s->rec = nullptr;
+    s->rec_n = 0;
+    cudaError_t e = cudaMalloc((void**)&s->rec, nb * 32);
+    if (e == cudaSuccess) e = cudaMemsetAsync(s->rec, 0, nb * 32, s->stream);
+    if (e == cudaSuccess) s->rec_n = nb;
+    return e;
 }
 
 // the lists of a call of `passes` passes within `budget` bytes: four times an even spread over the ranges where it fits,
@@ -412,7 +447,7 @@ size_t list_shape(const rf_sim* s, size_t nb, uint32_t passes, size_t budget, Li
     const uint64_t fit = (budget - head) / (ctas * ranges * 8);
     const uint64_t cap = std::min<uint64_t>({points, std::max<uint64_t>(4 * points / ranges, 256), fit});
     if (4 * cap * ranges < 5 * points || chaos_smem(s->slots, s->prog_words, s->L, 0, 1, ranges) > kMaxCtaSmem) return 0;
-    shape = ListShape{ranges, bits, (uint32_t)cap, false};
+    shape = ListShape{ranges, bits, (uint32_t)cap};
     return head + ctas * ranges * cap * 8;
 }
 
@@ -444,41 +479,60 @@ int draw_passes(rf_sim* s, uint32_t passes, float4* bins, uint32_t* hits, uint32
     const size_t nb = (size_t)W * H;
     bool il = s->bin_layout == RF_BINS_INTERLEAVED;
     if (s->bin_layout == RF_BINS_AUTO) il = hits != nullptr && nb * 20 > kInterleaveMinBytes;
-    if (!il) return launch_passes(s, passes, false, true, bins, hits, W, H, ss);
-    ListShape lists;
-    const ListView view{W, H, {ss[0], ss[1], ss[2], ss[3], ss[4], ss[5]}};
-    // (a captured call takes records: a later call may move the lists)
-    bool listed = s->bin_layout == RF_BINS_AUTO && nb >= kListMinBins && !capturing(s->stream);
-    if (listed && !lists_suit(s, view)) {
-        // records from here on; their memory comes in the place of the lists'
-        if (s->lists) s->list_turns++;
+    if (!il || !passes) return launch_passes(s, passes, false, true, bins, hits, W, H, ss);
+    const bool captured = capturing(s->stream);
+    // (a captured call takes records that are there: later calls may move the lists, and nothing can be allocated)
+    if (captured && s->rec_n < nb) return launch_passes(s, passes, false, true, bins, hits, W, H, ss);
+    if (captured) s->rec_captured = true;
+    DrawWay way;
+    ListShape shape;
+    int timed = -1;
+    const bool choose = s->bin_layout == RF_BINS_AUTO && nb >= kListMinBins && !captured &&
+                        list_shape(s, nb, passes, kListBytes, shape) != 0;
+    bool listed = choose && lists_for_call(s, ListView{s->list_genome, W, H, {ss[0], ss[1], ss[2], ss[3], ss[4], ss[5]}}, passes, &timed);
+    // one form's memory comes in the place of the other's; where there is none for a form, the other serves and stays
+    const bool wanted = listed;
+    if (listed) {
+        release_records(s);
+        listed = reserve_lists(s, nb, passes, shape);
+    } else if (choose) {
         release_lists(s);
-        listed = false;
     }
-    // (a program whose views turn and turn again stays with records: kListTurns)
-    if (listed && s->list_turns < kListTurns && reserve_lists(s, nb, passes, lists)) {
-        lists.measure = passes && !(s->list_asked && s->list_view == view);  // once per genome, grid and view
-        if (lists.measure) RF_CUDA(cudaMemsetAsync(s->counters + 4, 0, 3 * sizeof(unsigned long long), s->stream));
-        const int rc = launch_passes(s, passes, false, true, bins, hits, W, H, ss, &lists);
-        if (!rc && lists.measure) measure_lists(s, view, passes);
+    if (!listed) {
+        const cudaError_t e = reserve_records(s, nb);
+        if (e != cudaSuccess && choose) listed = reserve_lists(s, nb, passes, shape);
+        if (e != cudaSuccess && !listed) return cuda_fail(e, "bin records");
+        if (e != cudaSuccess) cudaGetLastError();
+    }
+    if (listed != wanted) {
+        s->list_step = 3;
+        s->list_form = listed;
+        s->list_calls = 0;
+        timed = -1;
+    }
+    if (timed >= 0 && load_draw_kernels() != cudaSuccess) { cudaGetLastError(); timed = -1; }
+    if (timed >= 0) way.begin = s->list_ev[2 * timed];
+    way.tune = !choose || s->list_step == 3;
+    const auto time_end = [&] {
+        if (timed < 0) return;
+        if (cudaEventRecord(s->list_ev[2 * timed + 1], s->stream) == cudaSuccess) s->list_step = timed + 1;
+        else cudaGetLastError();
+    };
+    if (listed) {
+        way.lists = &shape;
+        const int rc = launch_passes(s, passes, false, true, bins, hits, W, H, ss, way);
+        if (rc == RF_OK) time_end();
         return rc;
-    }
-    if (s->rec_n < nb) {
-        cudaFree(s->rec);
-        s->rec = nullptr;
-        s->rec_n = 0;
-        RF_CUDA(cudaMalloc((void**)&s->rec, nb * 32));
-        RF_CUDA(cudaMemsetAsync(s->rec, 0, nb * 32, s->stream));
-        s->rec_n = nb;
     }
     s->rgba_shift = 1;
     s->count_shift = 3;
     const int rc = launch_passes(s, passes, false, true, s->rec, hits ? reinterpret_cast<uint32_t*>(s->rec) + 4 : nullptr,
-                                 W, H, ss);
+                                 W, H, ss, way);
     s->rgba_shift = 0;
     s->count_shift = 0;
     if (rc) return rc;
     RF_CUDA(launch_merge_records(s->rec, nb, bins, hits, s->stream));
+    time_end();
     return RF_OK;
 }
 
@@ -803,6 +857,8 @@ int rf_sim_create(const rf_sim_desc* d, rf_sim** out) {
         if ((e = cudaEventCreate(&ev)) != cudaSuccess) return cleanup(cuda_fail(e, "event"));
     for (auto& ev : s->tile_ev)
         if ((e = cudaEventCreate(&ev)) != cudaSuccess) return cleanup(cuda_fail(e, "event"));
+    for (auto& ev : s->list_ev)
+        if ((e = cudaEventCreate(&ev)) != cudaSuccess) return cleanup(cuda_fail(e, "event"));
     if ((e = cudaStreamSynchronize(s->stream)) != cudaSuccess) return cleanup(cuda_fail(e, "sim init"));
     *out = s;
     return RF_OK;
@@ -812,8 +868,6 @@ int rf_sim_destroy(rf_sim* s) {
     if (!s) return RF_OK;
     cudaSetDevice(s->device);
     cudaStreamSynchronize(s->stream);
-    if (s->list_stats) cudaFreeHost(s->list_stats);
-    if (s->list_ev) cudaEventDestroy(s->list_ev);
     void* ptrs[] = {s->rec, s->lists, s->walk[0], s->walk[1], s->rng, s->table, s->base_prog, s->progs, s->palette, s->counters,
                     s->trace, s->r_bins, s->r_hits, s->r_de, s->r_img, s->r_stats, s->r_rad, s->r_dw};
     for (void* p : ptrs)
@@ -821,6 +875,8 @@ int rf_sim_destroy(rf_sim* s) {
     for (auto ev : s->tune_ev)
         if (ev) cudaEventDestroy(ev);
     for (auto ev : s->tile_ev)
+        if (ev) cudaEventDestroy(ev);
+    for (auto ev : s->list_ev)
         if (ev) cudaEventDestroy(ev);
     scratch_trim();
     delete s;
@@ -871,8 +927,7 @@ int rf_warmup(rf_sim* s, rf_flame* f, uint32_t num_passes, float tss_width) {
     if (prog != s->spec_prog) {
         reset_exchange_tuning(s);
         s->auto_tile_state = 0;
-        s->list_asked = false;
-        s->list_turns = 0;
+        s->list_genome++;
     }
     if (s->d.specialize >= 0) {
         const void* k = nullptr;

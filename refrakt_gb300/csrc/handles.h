@@ -19,11 +19,15 @@ struct rf_flame {
     uint64_t version = 0;
 };
 
-// a bin grid and the screen affine that maps the plane to it
+// what a choice between records and point lists is made for: a warmed genome, a bin grid and the screen affine that
+// maps the plane to it
 struct ListView {
+    uint64_t genome;
     uint32_t w, h;
     float ss[6];
-    bool operator==(const ListView& o) const { return w == o.w && h == o.h && std::equal(ss, ss + 6, o.ss); }
+    bool operator==(const ListView& o) const {
+        return genome == o.genome && w == o.w && h == o.h && std::equal(ss, ss + 6, o.ss);
+    }
 };
 
 struct rf_sim {
@@ -81,16 +85,17 @@ struct rf_sim {
     // list per CTA and range
     unsigned char* lists = nullptr;
     size_t lists_bytes = 0, lists_refused = ~(size_t)0;  // refused: a size it had too little memory for
-    // of the first list call of a genome, grid and view (pinned; there once list_ev has passed): the most points that
-    // a launch's lists held of one bin, the points in the call's lists, and those that found their list full; the
-    // call's points and launches (full ones)
-    unsigned long long* list_stats = nullptr;
-    cudaEvent_t list_ev = nullptr;
-    uint64_t list_points = 0;
-    double list_launches = 1;
+    // RF_BINS_AUTO's choice between records and lists (lists_for_call): 0 -- nothing timed; 1 -- one call of list_view
+    // timed; 2 -- one of each form, deciding when the second has finished; 3 -- decided
+    int list_step = 0;
     ListView list_view{};
-    bool list_asked = false;
-    uint32_t list_turns = 0;  // times that the genome turned to records
+    uint64_t list_genome = 0;         // of the warmed flame
+    uint32_t list_passes = 0;         // of the first timed call (the second must match)
+    int list_first = 0;               // the form timed first (1: lists)
+    int list_form = -1;               // the last decision; -1: none yet
+    uint32_t list_calls = 0;          // since then
+    cudaEvent_t list_ev[4] = {nullptr, nullptr, nullptr, nullptr};
+    bool rec_captured = false;        // a captured call's graph holds the records
     // rf_render scratch
     float4* r_bins = nullptr;
     uint32_t* r_hits = nullptr;

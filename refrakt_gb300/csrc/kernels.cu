@@ -62,30 +62,20 @@ struct RangeArgs {
     RangeState* state;  // per range
     float4* bins;
     uint32_t* hits;
-    unsigned long long* stats;  // launch_ranges (may be null)
 };
 constexpr uint32_t kRangeThreads = 512, kMergeCtas = 1024;
 
-// a CTA per range: the points in its lists, and those that found their list full
+// a CTA per range: whether its lists hold fewer than 2^24 points
 __global__ void __launch_bounds__(256) range_count_kernel(const uint32_t* __restrict__ list_n, uint32_t ctas, uint32_t ranges,
-                                                          uint32_t cap, RangeState* state, unsigned long long* stats) {
-    __shared__ unsigned long long s_sum[2];
-    if (threadIdx.x < 2) s_sum[threadIdx.x] = 0;
+                                                          uint32_t cap, RangeState* state) {
+    __shared__ unsigned long long s_sum;
+    if (threadIdx.x == 0) s_sum = 0;
     __syncthreads();
-    unsigned long long in = 0, out = 0;
-    for (uint32_t c = threadIdx.x; c < ctas; c += 256) {
-        const uint32_t n = list_n[(size_t)c * ranges + blockIdx.x];
-        in += min(n, cap);
-        out += n - min(n, cap);
-    }
-    atomicAdd(&s_sum[0], in);
-    atomicAdd(&s_sum[1], out);
+    unsigned long long in = 0;
+    for (uint32_t c = threadIdx.x; c < ctas; c += 256) in += min(list_n[(size_t)c * ranges + blockIdx.x], cap);
+    atomicAdd(&s_sum, in);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        state[blockIdx.x] = RangeState{s_sum[0] < (1u << 24) ? 1u : 0u, 0u};
-        if (stats) atomicAdd(stats + 1, s_sum[0]);
-        if (stats && s_sum[1]) atomicAdd(stats + 2, s_sum[1]);
-    }
+    if (threadIdx.x == 0) state[blockIdx.x] = RangeState{s_sum < (1u << 24) ? 1u : 0u, 0u};
 }
 
 template <bool UNIT>
@@ -133,7 +123,6 @@ __device__ __forceinline__ void range_merge(const RangeArgs& R, uint32_t cta) {
     const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     constexpr uint32_t kStep = kMergeCtas * kRangeThreads;
     constexpr int U = 2;
-    uint32_t most = 0;
     for (uint32_t i0 = cta * kRangeThreads + threadIdx.x; i0 < n; i0 += kStep * U) {
         float4 v[U], b[U];
         uint32_t c[U], h[U];
@@ -166,8 +155,6 @@ __device__ __forceinline__ void range_merge(const RangeArgs& R, uint32_t cta) {
             }
         }
 #pragma unroll
-        for (int u = 0; u < U; u++) most = max(most, c[u]);
-#pragma unroll
         for (int u = 0; u < U; u++)
             if (c[u]) {
                 b[u] = __ldcs(R.bins + first + i0 + kStep * u);
@@ -181,9 +168,6 @@ __device__ __forceinline__ void range_merge(const RangeArgs& R, uint32_t cta) {
                 __stcs(R.hits + first + i0 + kStep * u, h[u] + c[u]);
             }
     }
-    if (!R.stats) return;
-    most = __reduce_max_sync(0xffffffffu, most);
-    if ((threadIdx.x & 31) == 0 && most > *(volatile unsigned long long*)R.stats) atomicMax(R.stats, (unsigned long long)most);
 }
 
 __global__ void __launch_bounds__(kRangeThreads, 3) range_step_kernel(const __grid_constant__ RangeArgs R) {
@@ -202,11 +186,16 @@ __global__ void __launch_bounds__(kRangeThreads, 3) range_step_kernel(const __gr
     }
 }
 
-cudaError_t launch_ranges(const ChaosArgs& a, uint32_t ctas, const RangeScratch set[2], RangeState* state,
-                          unsigned long long* stats, cudaStream_t st) {
-    RangeArgs R{a.list, a.list_n, a.list_cap, a.ranges, a.range_bits, ctas, 0, a.W * a.H, a.palette, {set[0], set[1]}, state, a.bins, a.hits,
-                stats};
-    range_count_kernel<<<a.ranges, 256, 0, st>>>(a.list_n, ctas, a.ranges, a.list_cap, state, stats);
+cudaError_t load_draw_kernels() {
+    cudaFuncAttributes f;
+    for (const void* k : {(const void*)range_count_kernel, (const void*)range_step_kernel, (const void*)merge_records_kernel})
+        if (const cudaError_t e = cudaFuncGetAttributes(&f, k)) return e;
+    return cudaSuccess;
+}
+
+cudaError_t launch_ranges(const ChaosArgs& a, uint32_t ctas, const RangeScratch set[2], RangeState* state, cudaStream_t st) {
+    RangeArgs R{a.list, a.list_n, a.list_cap, a.ranges, a.range_bits, ctas, 0, a.W * a.H, a.palette, {set[0], set[1]}, state, a.bins, a.hits};
+    range_count_kernel<<<a.ranges, 256, 0, st>>>(a.list_n, ctas, a.ranges, a.list_cap, state);
     cudaError_t e = cudaGetLastError();
     for (; R.range <= a.ranges && e == cudaSuccess; R.range++) {
         const uint32_t grid = (R.range < a.ranges ? ctas : 0u) + (R.range > 0 ? kMergeCtas : 0u);

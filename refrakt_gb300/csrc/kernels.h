@@ -31,11 +31,10 @@ struct RangeScratch {
 struct RangeState {
     uint32_t unit, mixed;  // fewer than 2^24 points in the range's lists; among them some of opacity other than 1
 };
-// the lists of a launch of `ctas` CTAs with splat 4 into its planes.  stats (may be null; every step waits for
-// it some 0.4 us longer): [0] raised to the most points that
-// one bin got from them, [1] grows by the points in the lists, [2] by those that found their list full
-cudaError_t launch_ranges(const ChaosArgs& a, uint32_t ctas, const RangeScratch set[2], RangeState* state,
-                          unsigned long long* stats, cudaStream_t st);
+// the lists of a launch of `ctas` CTAs with splat 4 into its planes
+cudaError_t launch_ranges(const ChaosArgs& a, uint32_t ctas, const RangeScratch set[2], RangeState* state, cudaStream_t st);
+// loads the kernels of launch_ranges and launch_merge_records (before a call that is timed)
+cudaError_t load_draw_kernels();
 cudaError_t launch_merge_records(float4* rec, size_t n, float4* bins, uint32_t* hits, cudaStream_t st);
 cudaError_t launch_init_rng(uint4* rng, uint64_t n, uint64_t seed, cudaStream_t st);
 cudaError_t launch_shuffle_table(uint16_t* out, uint32_t n, uint32_t count, uint64_t seed, cudaStream_t st,

@@ -20,7 +20,7 @@ def routes(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scene", ["failed_call", "own_points", "own_view", "memory"])
+@pytest.mark.parametrize("scene", ["failed_call", "faster_form", "own_view", "memory", "captured"])
 def test_routes(routes, scene):
     r = subprocess.run([routes, scene], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and "OK" in r.stdout, r.stdout + r.stderr
