@@ -56,6 +56,9 @@ int splat_code(int splat) {
 namespace {
 
 constexpr size_t kListBytes = 16ull << 30;  // the lists' memory at most: 256 passes of 2.5 M walkers at three times an even spread
+// (7680 x 4320 bins, which take records, calls of 32 and 256 passes, ms with records and with lists: the space-filling
+// genome 3.10, 1.56 and 21.0, 13.7, the 1080p genome 1.96, 2.69 and 11.9, 18.2; 6144 x 4608 2.83, 1.54 and 19.1, 13.6,
+// 1.90, 2.72 and 11.3, 18.2)
 constexpr size_t kListMinBins = 1u << 25;
 constexpr uint32_t kListStands = 16;  // calls for which one genome's and view's choice stands for the next: a change of form costs
                                       // an allocation (8192 x 8192 bins: 3 ms)

@@ -686,10 +686,13 @@ static cudaError_t launch_de_rows(int R, const DeParams& P, const float4* in, co
 }
 
 // R: the launch's largest radius.  More rows per warp read a source once for more outputs, fewer leave
-// more warps to hide latency.  Measured, radius 9 (density estimation alone, 8 / 4 / 2 rows, before the
-// staging was asynchronous): 3840 x 2160
-// 642 / 737 / 872 us, 1920 x 1080 242 / 236 / 274, 960 x 540 116 / 96 / 107, 512 x 512 95 / 73 / 82, 640 x 360
-// 93 / 70 / 64, 320 x 180 88 / 58 / 47: 8 rows from 12 CTAs for each of the 152 SMs, 4 from about 1.6.
+// more warps to hide latency.  Measured, radius 9, 250 points per bin, us at 8 / 4 / 2 rows, density estimation
+// alone and with the tonemap on chip: 3840 x 2160 (4,080 CTAs of 8 rows) 640 / 736 / 890 and 694 / 835 / 959;
+// 2560 x 1440 (1,800) 342 / 376 / 437 and 370 / 422 / 468; 1920 x 1080 (1,020) 235 / 242 / 273 and 252 / 270 / 293;
+// 1600 x 900 (725) 183 / 186 / 208 and 195 / 208 / 221; 1440 x 810 (598) 163 / 167 / 179 and 175 / 183 / 192;
+// 1280 x 720 (460) 153 / 144 / 152 and 157 / 161 / 161; 960 x 540 114 / 99 / 108 and 120 / 110 / 115; 512 x 512 (256
+// CTAs of 4 rows) 90 / 77 / 77 and 97 / 85 / 81; 640 x 360 (230) 89 / 73 / 65 and 97 / 81 / 67; 320 x 180
+// 83 / 63 / 48 and 89 / 69 / 50: 8 rows from 4 CTAs for each of the 152 SMs, 4 from about 1.6.
 static cudaError_t launch_de_sweep(int R, const float4* in, const uint8_t* rad, uint32_t w, uint32_t h, float4* out,
                                    cudaStream_t st, const TmArgs* tm = nullptr) {
     cudaError_t e = density_prepare();
@@ -697,7 +700,7 @@ static cudaError_t launch_de_sweep(int R, const float4* in, const uint8_t* rad, 
     DeParams P{};
     de_weight_params(R, P);
     const auto ctas = [&](uint32_t rows) { return (uint64_t)((w + kCtaW - 1) / kCtaW) * ((h + 4 * rows - 1) / (4 * rows)); };
-    if (ctas(8) >= 12 * 152) return launch_de_rows<8>(R, P, in, rad, w, h, out, st, tm);
+    if (ctas(8) >= 4 * 152) return launch_de_rows<8>(R, P, in, rad, w, h, out, st, tm);
     if (ctas(4) >= 240) return launch_de_rows<4>(R, P, in, rad, w, h, out, st, tm);
     return launch_de_rows<2>(R, P, in, rad, w, h, out, st, tm);
 }
