@@ -270,7 +270,7 @@ __device__ __forceinline__ uchar4 to_rgba8(float4 o) {
 // not finite are taken again from the covering sources alone (de_row_covered): looking at the sums costs a
 // hundredth of the instructions (3840 x 2160 bins 641 -> 629 us, 960 x 540 at radius 20 329 -> 331).
 //
-// Bound: instruction issue (62 % of the slots at 24 warps per SM; about 70 instructions per source and
+// Bound: instruction issue (67 % of the slots at 23 warps per SM; about 70 instructions per source and
 // 8 outputs).  Density estimation of 3840 x 2160 bins at 1000 points per bin: 990 us as one output per
 // thread over the box of the tile's largest radius, 598 here; 960 x 540 at radius 20 1,090 us as a gather
 // from global memory, 330 here.
