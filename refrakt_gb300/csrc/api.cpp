@@ -413,13 +413,14 @@ int lists_for_call(rf_sim* s, const ListView& view, uint32_t passes, int* timed)
 }
 
 void release_lists(rf_sim* s) {
+    s->lists_refused = ~(size_t)0;
+    if (!s->lists) return;
     cudaFree(s->lists);  // (waits for the launches that use them)
     s->lists = nullptr;
     s->lists_bytes = 0;
-    s->lists_refused = ~(size_t)0;
 }
 void release_records(rf_sim* s) {
-    if (s->rec_captured) return;
+    if (!s->rec || s->rec_captured) return;
     cudaFree(s->rec);
     s->rec = nullptr;
     s->rec_n = 0;
